@@ -15,6 +15,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cstdint>
+
 #include "cell_walk.cuh"
 #include "kernels.h"
 
@@ -50,7 +52,7 @@ __device__ __forceinline__ void st<__half> (__half *p, size_t i, float v)
 
 __device__ __forceinline__ size_t flin (const GeomDev &g, int x, int y, int z)
 {
-  return ((size_t) x * g.n[1] + y) * g.n[2] + z;
+  return ((size_t) x * g.n[1] + y) * g.pz + z;
 }
 
 // incident value in FP64 (1-D grid is FP64 in every form)
@@ -255,30 +257,106 @@ __global__ void fast_point_source_kernel (T *f, size_t index, const double *src,
     st (f, index, (float) src[src_index] * scale);
 }
 
-template <typename T>
-__global__ void convert_in_kernel (T *dst, const double *src, size_t n, double scale)
+// FP64 arrays <-> stored fields, dst = src * scale.  A copy is bound by DRAM
+// (8 + sizeof (T) bytes per cell), so the flat form (rows without padding,
+// both pointers on 16-byte boundaries) moves four cells per thread in 16-byte
+// accesses; the row form takes rows of nz cells, pz stored, one warp each.
+__device__ __forceinline__ void ld4 (const double *p, size_t q, double v[4])
 {
-  for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x)
-    st (dst, i, (float) (src[i] * scale));
+  const double2 a = reinterpret_cast<const double2 *> (p)[2 * q], b = reinterpret_cast<const double2 *> (p)[2 * q + 1];
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = b.x;
+  v[3] = b.y;
+}
+__device__ __forceinline__ void ld4 (const float *p, size_t q, double v[4])
+{
+  const float4 a = reinterpret_cast<const float4 *> (p)[q];
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = a.z;
+  v[3] = a.w;
+}
+__device__ __forceinline__ void ld4 (const __half *p, size_t q, double v[4])
+{
+  const uint2 t = reinterpret_cast<const uint2 *> (p)[q];
+  const float2 a = __half22float2 (*reinterpret_cast<const __half2 *> (&t.x));
+  const float2 b = __half22float2 (*reinterpret_cast<const __half2 *> (&t.y));
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = b.x;
+  v[3] = b.y;
+}
+__device__ __forceinline__ void st4 (double *p, size_t q, const double v[4])
+{
+  __stcs (reinterpret_cast<double2 *> (p) + 2 * q, make_double2 (v[0], v[1]));
+  __stcs (reinterpret_cast<double2 *> (p) + 2 * q + 1, make_double2 (v[2], v[3]));
+}
+__device__ __forceinline__ void st4 (float *p, size_t q, const double v[4])
+{
+  reinterpret_cast<float4 *> (p)[q] = make_float4 ((float) v[0], (float) v[1], (float) v[2], (float) v[3]);
+}
+__device__ __forceinline__ void st4 (__half *p, size_t q, const double v[4])
+{
+  __half2 a = __floats2half2_rn ((float) v[0], (float) v[1]), b = __floats2half2_rn ((float) v[2], (float) v[3]);
+  uint2 t;
+  t.x = *reinterpret_cast<unsigned *> (&a);
+  t.y = *reinterpret_cast<unsigned *> (&b);
+  reinterpret_cast<uint2 *> (p)[q] = t;
 }
 
-__global__ void convert_in_double_kernel (double *dst, const double *src, size_t n, double scale)
+__device__ __forceinline__ double get (const double *p, size_t i)
 {
-  for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x)
-    dst[i] = src[i] * scale;
+  return p[i];
+}
+__device__ __forceinline__ double get (const float *p, size_t i)
+{
+  return (double) p[i];
+}
+__device__ __forceinline__ double get (const __half *p, size_t i)
+{
+  return (double) __half2float (p[i]);
+}
+__device__ __forceinline__ void put (double *p, size_t i, double v)
+{
+  p[i] = v;
+}
+__device__ __forceinline__ void put (float *p, size_t i, double v)
+{
+  p[i] = (float) v;
+}
+__device__ __forceinline__ void put (__half *p, size_t i, double v)
+{
+  p[i] = __float2half_rn ((float) v);
 }
 
-template <typename T>
-__global__ void convert_out_kernel (double *dst, const T *src, size_t n, double scale)
+template <typename D, typename S, bool VEC>
+__global__ void __launch_bounds__ (256) convert_flat_kernel (D *dst, const S *src, size_t n, double scale)
 {
-  for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x)
-    dst[i] = (double) ld (src, i) * scale;
+  const size_t t = (size_t) blockIdx.x * blockDim.x + threadIdx.x, step = (size_t) gridDim.x * blockDim.x;
+  const size_t n4 = VEC ? n / 4 : 0;
+  for (size_t q = t; q < n4; q += step)
+  {
+    double v[4];
+    ld4 (src, q, v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v[j] *= scale;
+    st4 (dst, q, v);
+  }
+  for (size_t i = 4 * n4 + t; i < n; i += step)
+    put (dst, i, get (src, i) * scale);
 }
 
-__global__ void convert_out_double_kernel (double *dst, const double *src, size_t n, double scale)
+template <typename D, typename S>
+__global__ void __launch_bounds__ (256) convert_rows_kernel (D *dst, const S *src, size_t rows, int nz, int dpitch,
+                                                             int spitch, double scale)
 {
-  for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x)
-    dst[i] = src[i] * scale;
+  const int lane = threadIdx.x & 31;
+  for (size_t r = ((size_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows;
+       r += ((size_t) gridDim.x * blockDim.x) >> 5)
+    for (int z = lane; z < nz; z += 32)
+      put (dst, r * dpitch + z, get (src, r * spitch + z) * scale);
 }
 
 // Neumaier (compensated) accumulation in FP64
@@ -391,16 +469,35 @@ int launch_fast_point_source (void *f, int fp16, size_t index, const double *src
   return 1;
 }
 
-int launch_convert_in (void *dst, int dst_kind, const double *src, size_t n, double scale, cudaStream_t s)
+namespace {
+
+template <typename D, typename S>
+int launch_convert (D *dst, const S *src, size_t rows, int nz, int dpitch, int spitch, double scale, cudaStream_t s)
 {
-  int blocks = grid_for (n, 148);
-  if (dst_kind == 0)
-    convert_in_double_kernel<<<blocks, 256, 0, s>>> ((double *) dst, src, n, scale);
-  else if (dst_kind == 1)
-    convert_in_kernel<float><<<blocks, 256, 0, s>>> ((float *) dst, src, n, scale);
+  if (nz == dpitch && nz == spitch)
+  {
+    const size_t n = rows * (size_t) nz;
+    const bool vec = (((uintptr_t) dst | (uintptr_t) src) & 15u) == 0;
+    if (vec)
+      convert_flat_kernel<D, S, true><<<grid_for ((n + 3) / 4, 148), 256, 0, s>>> (dst, src, n, scale);
+    else
+      convert_flat_kernel<D, S, false><<<grid_for (n, 148), 256, 0, s>>> (dst, src, n, scale);
+  }
   else
-    convert_in_kernel<__half><<<blocks, 256, 0, s>>> ((__half *) dst, src, n, scale);
+    convert_rows_kernel<D, S><<<grid_for (rows * 32, 148), 256, 0, s>>> (dst, src, rows, nz, dpitch, spitch, scale);
   return 1;
+}
+
+}  // namespace
+
+int launch_convert_in (void *dst, int dst_kind, const double *src, size_t rows, int nz, int pz, double scale,
+                       cudaStream_t s)
+{
+  if (dst_kind == 0)
+    return launch_convert ((double *) dst, src, rows, nz, pz, nz, scale, s);
+  if (dst_kind == 1)
+    return launch_convert ((float *) dst, src, rows, nz, pz, nz, scale, s);
+  return launch_convert ((__half *) dst, src, rows, nz, pz, nz, scale, s);
 }
 
 namespace {
@@ -421,16 +518,14 @@ int launch_find_nonfinite (const double *src, size_t n, unsigned long long *firs
   return 1;
 }
 
-int launch_convert_out (double *dst, const void *src, int src_kind, size_t n, double scale, cudaStream_t s)
+int launch_convert_out (double *dst, const void *src, int src_kind, size_t rows, int nz, int pz, double scale,
+                        cudaStream_t s)
 {
-  int blocks = grid_for (n, 148);
   if (src_kind == 0)
-    convert_out_double_kernel<<<blocks, 256, 0, s>>> (dst, (const double *) src, n, scale);
-  else if (src_kind == 1)
-    convert_out_kernel<float><<<blocks, 256, 0, s>>> (dst, (const float *) src, n, scale);
-  else
-    convert_out_kernel<__half><<<blocks, 256, 0, s>>> (dst, (const __half *) src, n, scale);
-  return 1;
+    return launch_convert (dst, (const double *) src, rows, nz, nz, pz, scale, s);
+  if (src_kind == 1)
+    return launch_convert (dst, (const float *) src, rows, nz, nz, pz, scale, s);
+  return launch_convert (dst, (const __half *) src, rows, nz, nz, pz, scale, s);
 }
 
 int launch_reduce_sq (const void *src, int kind, size_t n, const void *weight, int wkind, double scale,
@@ -520,7 +615,7 @@ __device__ __forceinline__ void neumaier (double *s, double *c, double v)
 // in FP64 with Neumaier compensation (acc: re, re compensation, im, im
 // compensation per cell and frequency).
 template <typename T>
-__global__ void dft_kernel (const T *src, int axis, int index, int n0, int n1, int n2, double scale,
+__global__ void dft_kernel (const T *src, int axis, int index, int n0, int n1, int n2, int pz, double scale,
                             const double *phase, int nf, double *acc)
 {
   const int ma = axis == 0 ? n1 : n0;             // plane extents (first, second remaining axis)
@@ -534,11 +629,11 @@ __global__ void dft_kernel (const T *src, int axis, int index, int n0, int n1, i
     const int a = (int) (c / mb), b = (int) (c % mb);
     long long id;
     if (axis == 0)
-      id = ((long long) index * n1 + a) * n2 + b;
+      id = ((long long) index * n1 + a) * pz + b;
     else if (axis == 1)
-      id = ((long long) a * n1 + index) * n2 + b;
+      id = ((long long) a * n1 + index) * pz + b;
     else
-      id = ((long long) a * n1 + b) * n2 + index;
+      id = ((long long) a * n1 + b) * pz + index;
     const double v = ldd (src, (size_t) id) * scale;
     double *r = acc + q * 4;
     neumaier (r + 0, r + 1, v * phase[2 * j]);
@@ -548,21 +643,21 @@ __global__ void dft_kernel (const T *src, int axis, int index, int n0, int n1, i
 
 }  // namespace
 
-int launch_dft (const void *src, int kind, int axis, int index, const int n[3], double scale, const double *phase,
-                int nf, double *acc, int sm_count, cudaStream_t s)
+int launch_dft (const void *src, int kind, int axis, int index, const int n[3], int pz, double scale,
+                const double *phase, int nf, double *acc, int sm_count, cudaStream_t s)
 {
   const long long cells = (long long) (axis == 0 ? n[1] : n[0]) * (axis == 2 ? n[1] : n[2]) * nf;
   long long blocks = (cells + 255) / 256;
   if (blocks > (long long) sm_count * 16)
     blocks = (long long) sm_count * 16;
   if (kind == 0)
-    dft_kernel<double><<<(unsigned) blocks, 256, 0, s>>> ((const double *) src, axis, index, n[0], n[1], n[2], scale,
+    dft_kernel<double><<<(unsigned) blocks, 256, 0, s>>> ((const double *) src, axis, index, n[0], n[1], n[2], pz, scale,
                                                           phase, nf, acc);
   else if (kind == 1)
-    dft_kernel<float><<<(unsigned) blocks, 256, 0, s>>> ((const float *) src, axis, index, n[0], n[1], n[2], scale,
+    dft_kernel<float><<<(unsigned) blocks, 256, 0, s>>> ((const float *) src, axis, index, n[0], n[1], n[2], pz, scale,
                                                          phase, nf, acc);
   else
-    dft_kernel<__half><<<(unsigned) blocks, 256, 0, s>>> ((const __half *) src, axis, index, n[0], n[1], n[2], scale,
+    dft_kernel<__half><<<(unsigned) blocks, 256, 0, s>>> ((const __half *) src, axis, index, n[0], n[1], n[2], pz, scale,
                                                           phase, nf, acc);
   return 1;
 }

@@ -66,6 +66,8 @@ struct fdtd_ctx
   cudaStream_t stream = nullptr;
   int prec = 0;
   int kind = 0;
+  int pz = 0;             // stored cells per z row (row_pitch)
+  size_t scells = 0;      // stored cells per array: nx * ny * pz
   int64_t launches = 0;
   int *d_err = nullptr;
   double eta0 = 1.0;
@@ -243,12 +245,30 @@ int dalloc (fdtd_ctx *ctx, void **p, size_t bytes, bool zero = true)
       return r_;                                                                                   \
   } while (0)
 
-GeomDev make_geom_dev (const Geometry &g)
+// Stored cells per z row.  The TMA kernels of the 3-D FP32 / FP16 forms need
+// rows of whole 16-byte units, so their grids store rows of nz rounded up to
+// one (the added cells hold zeros and are never updated): 203 x 181 x 165
+// cells, PML and TF/SF, FP32: 187 us per step against 326 us in the
+// register-blocked kernel.  Rows shorter than a warp keep nz, and with it
+// the register-blocked kernel when nz is no whole unit (thin grids bound by
+// their launches in either kernel).
+constexpr int kPadRow = 32;
+int row_pitch (const Geometry &g, int kind)
+{
+  const int nz = g.n[2];
+  if (kind == 0 || g.drop != 0 || g.cfg.layout != 0 || g.dmp || nz < kPadRow)
+    return nz;
+  const int unit = kind == 2 ? 8 : 4;
+  return (nz + unit - 1) / unit * unit;
+}
+
+GeomDev make_geom_dev (const Geometry &g, int pz)
 {
   GeomDev d;
   std::memset (&d, 0, sizeof (d));
   for (int a = 0; a < 3; ++a)
     d.n[a] = g.n[a];
+  d.pz = pz;
   d.drop = g.drop;
   for (int j = 0; j < 2; ++j)
   {
@@ -511,7 +531,7 @@ int upload_fine_material (fdtd_ctx *ctx, int which, const double *src, cudaMemcp
 int alloc_fast (fdtd_ctx *ctx)
 {
   const Geometry &g = ctx->g;
-  size_t n = (size_t) g.cells;
+  const size_t n = ctx->scells;
   // the one-sweep 3-D kernels (register-blocked and TMA) are written for the
   // E_CENTERED stencil on cell-centred materials; H_CENTERED, double material
   // precision and the 2-D / 1-D modes run the per-cell kernels on one buffer set
@@ -582,7 +602,7 @@ int alloc_fast (fdtd_ctx *ctx)
   {
     FastHalf &p = h ? ctx->fast_h : ctx->fast_e;
     std::memset (&p, 0, sizeof (p));
-    p.g = make_geom_dev (g);
+    p.g = make_geom_dev (g, ctx->pz);
     p.is_h = h;
     p.use_pml = g.cfg.use_pml;
     p.use_tfsf = g.cfg.use_tfsf;
@@ -662,7 +682,7 @@ void init_fused (fdtd_ctx *ctx)
   const Geometry &g = ctx->g;
   FusedParams &f = ctx->fused;
   std::memset (&f, 0, sizeof (f));
-  f.g = make_geom_dev (g);
+  f.g = make_geom_dev (g, ctx->pz);
   f.use_pml = g.cfg.use_pml;
   f.use_tfsf = g.cfg.use_tfsf;
   f.fp16 = ctx->kind == 2;
@@ -810,7 +830,7 @@ std::string plan_shell (fdtd_ctx *ctx, void *const e[2][3], void *const h[2][3],
     return "the PML shell leaves no core";
   // set T (fields as the step stores them, PML auxiliaries), starting as a
   // copy of the current set (its never-updated faces must hold the fields)
-  const size_t n = (size_t) g.cells;
+  const size_t n = ctx->scells;
   for (int k = 0; k < 6; ++k)
   {
     if (!ctx->tfb[k])
@@ -1053,7 +1073,7 @@ int plan_sweep (fdtd_ctx *ctx)
   {
     if (!ctx->drude_box_dev)
       DALLOC (ctx->drude_box_dev, 6 * sizeof (int));
-    ctx->launches += launch_drude_box (ctx->dflag, g.n[0], g.n[1], g.n[2], ctx->drude_box_dev, ctx->stream);
+    ctx->launches += launch_drude_box (ctx->dflag, g.n[0], g.n[1], ctx->pz, ctx->drude_box_dev, ctx->stream);
     int hb[6];
     CK (cudaMemcpyAsync (hb, ctx->drude_box_dev, sizeof (hb), cudaMemcpyDeviceToHost, ctx->stream));
     CK (cudaStreamSynchronize (ctx->stream));
@@ -1197,6 +1217,8 @@ int create_impl (const fdtd_config *cfg, int device, fdtd_ctx *ctx)
         ctx->cs_mask[k / 3] |= 1 << (k % 3);
   }
   ctx->kind = kind_of (cfg->precision);
+  ctx->pz = row_pitch (ctx->g, ctx->kind);
+  ctx->scells = (size_t) ctx->g.n[0] * ctx->g.n[1] * ctx->pz;
   ctx->eta0 = ctx->kind == 0 ? 1.0 : kEta0;
   CK (cudaSetDevice (device));
   CK (cudaDeviceGetAttribute (&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
@@ -1281,12 +1303,7 @@ void release (fdtd_ctx *ctx)
   delete ctx;
 }
 
-size_t cell_index (const Geometry &g, int x, int y, int z)
-{
-  return ((size_t) x * g.n[1] + y) * g.n[2] + z;
-}
-
-bool point_source_index (const Geometry &g, size_t *idx)
+bool point_source_index (const Geometry &g, int pz, size_t *idx)
 {
   int p[3];
   for (int a = 0; a < 3; ++a)
@@ -1295,7 +1312,7 @@ bool point_source_index (const Geometry &g, size_t *idx)
     if (p[a] < 0 || p[a] >= g.n[a])
       return false;
   }
-  *idx = cell_index (g, p[0], p[1], p[2]);
+  *idx = ((size_t) p[0] * g.n[1] + p[1]) * pz + p[2];
   return true;
 }
 
@@ -1314,7 +1331,7 @@ PlainHalf plain_half (fdtd_ctx *ctx, int h)
   const Geometry &g = ctx->g;
   PlainHalf p;
   std::memset (&p, 0, sizeof (p));
-  p.g = make_geom_dev (g);
+  p.g = make_geom_dev (g, ctx->pz);
   p.is_h = h;
   p.use_pml = g.cfg.use_pml;
   p.use_tfsf = g.cfg.use_tfsf;
@@ -1430,7 +1447,7 @@ void dft_step (fdtd_ctx *ctx, uint32_t i)
   const int k = ctx->dft_comp;
   const void *src = ctx->kind == 0 ? (const void *) ctx->f[k][1] : (const void *) ctx->ff[k];
   const double scale = k >= 3 ? 1.0 / ctx->eta0 : 1.0;
-  ctx->launches += launch_dft (src, ctx->kind, ctx->dft_axis, ctx->dft_index, ctx->g.n, scale,
+  ctx->launches += launch_dft (src, ctx->kind, ctx->dft_axis, ctx->dft_index, ctx->g.n, ctx->pz, scale,
                                ctx->dft_phase + (size_t) i * ctx->dft_nf * 2, ctx->dft_nf, ctx->dft_acc,
                                ctx->sm_count, ctx->stream);
 }
@@ -1459,7 +1476,7 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
   if (n > 1 || t_start > 0)
     ctx->stepped = true;
   size_t ps_idx = 0;
-  bool ps_ok = g.cfg.point_source_mask && point_source_index (g, &ps_idx);
+  bool ps_ok = g.cfg.point_source_mask && point_source_index (g, ctx->pz, &ps_idx);
   cudaStream_t s = ctx->stream;
   // a current source runs with the one-sweep kernels as a fix-up after each
   // step (launch_current_fix) when its cell and the cells around it update
@@ -1705,7 +1722,7 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
           {
             for (int ci = 0; ci < 3; ++ci)
               if (g.comp[3 + ci].exists)
-                CK (cudaMemcpyAsync (ctx->hprev[ci], ctx->ff[3 + ci], (size_t) g.cells * elem_size (ctx->kind),
+                CK (cudaMemcpyAsync (ctx->hprev[ci], ctx->ff[3 + ci], ctx->scells * elem_size (ctx->kind),
                                      cudaMemcpyDeviceToDevice, s));
             ctx->prev_src = 2;
           }
@@ -1817,6 +1834,8 @@ int fdtd_upload_material_device (fdtd_ctx *ctx, int which, const double *dev)
   if (r != FDTD_OK)
     return r;
   size_t n = (size_t) ctx->g.cells;
+  const int nz = ctx->g.n[2];
+  const size_t rows = n / nz;
   if (ctx->g.dmp && which < 2)
     return upload_fine_material (ctx, which, dev, cudaMemcpyDeviceToDevice);
   if (ctx->kind == 0)
@@ -1835,17 +1854,17 @@ int fdtd_upload_material_device (fdtd_ctx *ctx, int which, const double *dev)
     if (!ctx->dflag)
       return fail (ctx, FDTD_ERR_UNSUPPORTED, "Drude grids need use_metamaterials");
     // FDTD_MAT_OMEGAPE..GAMMAM = 2..5 -> omegape, omegapm, gammae, gammam
-    ctx->launches += launch_convert_in (ctx->drude32[which - 2], 1, dev, n, 1.0, ctx->stream);
+    ctx->launches += launch_convert_in (ctx->drude32[which - 2], 1, dev, rows, nz, ctx->pz, 1.0, ctx->stream);
     ctx->launches += launch_drude_flags (ctx->dflag, ctx->drude32[0], ctx->drude32[2], ctx->drude32[1],
-                                         ctx->drude32[3], ctx->g.n[0], ctx->g.n[1], ctx->g.n[2], ctx->stream);
+                                         ctx->drude32[3], ctx->g.n[0], ctx->g.n[1], nz, ctx->pz, ctx->stream);
     CK (cudaGetLastError ());
     if (ctx->sweep_state != 0)
       ctx->sweep_state = 0;   // the Drude cells changed: plan again at the next step
     return FDTD_OK;
   }
   if (!ctx->mat32[which])
-    DALLOC (ctx->mat32[which], n * sizeof (float));
-  ctx->launches += launch_convert_in (ctx->mat32[which], 1, dev, n, 1.0, ctx->stream);
+    DALLOC (ctx->mat32[which], ctx->scells * sizeof (float));
+  ctx->launches += launch_convert_in (ctx->mat32[which], 1, dev, rows, nz, ctx->pz, 1.0, ctx->stream);
   CK (cudaGetLastError ());
   return FDTD_OK;
 }
@@ -1873,8 +1892,8 @@ int fdtd_upload_field (fdtd_ctx *ctx, int component, const double *host)
     {
       void *dst = b < 2 ? ctx->ffb[b][component] : ctx->tfb[component];
       if (dst)
-        ctx->launches += launch_convert_in (dst, ctx->kind, ctx->staging, n, component >= 3 ? kEta0 : 1.0,
-                                            ctx->stream);
+        ctx->launches += launch_convert_in (dst, ctx->kind, ctx->staging, n / ctx->g.n[2], ctx->g.n[2], ctx->pz,
+                                            component >= 3 ? kEta0 : 1.0, ctx->stream);
     }
   }
   CK (cudaStreamSynchronize (ctx->stream));
@@ -1948,7 +1967,7 @@ int fdtd_download_field_device (fdtd_ctx *ctx, int component, double *dev)
   }
   else
   {
-    ctx->launches += launch_convert_out (dev, ctx->ff[component], ctx->kind, n,
+    ctx->launches += launch_convert_out (dev, ctx->ff[component], ctx->kind, n / ctx->g.n[2], ctx->g.n[2], ctx->pz,
                                          component >= 3 ? 1.0 / kEta0 : 1.0, ctx->stream);
     CK (cudaGetLastError ());
   }
@@ -2043,7 +2062,7 @@ int fdtd_download_field_scattered (fdtd_ctx *ctx, int component, double *host)
     right[a] = (double) (g.n[a] - g.cfg.tfsf_right[a]);
   }
   const double *inc = component >= 3 ? ctx->hinc[ctx->hcur] : ctx->einc[ctx->ecur];
-  ctx->launches += launch_scattered (ctx->staging, make_geom_dev (g), component, inc, g.inc_len, left, right,
+  ctx->launches += launch_scattered (ctx->staging, make_geom_dev (g, g.n[2]), component, inc, g.inc_len, left, right,
                                      ctx->d_err, ctx->sm_count, ctx->stream);
   CK (cudaGetLastError ());
   const size_t n = (size_t) g.cells;
@@ -2083,7 +2102,7 @@ int fdtd_reduce (fdtd_ctx *ctx, int what, double *out)
   int r = set_device (ctx);
   if (r != FDTD_OK)
     return r;
-  size_t n = (size_t) ctx->g.cells;
+  const size_t n = ctx->scells;   // (padding cells hold zeros)
   for (int k = 0; k < 6; ++k)
   {
     if (!ctx->g.comp[k].exists)
@@ -2296,6 +2315,7 @@ int fdtd_ntff (fdtd_ctx *re, fdtd_ctx *im, const int left[3], const int right[3]
     len[a] = right[a] - left[a];
   }
   p.points = 2 * (len[1] * len[2] + len[0] * len[2] + len[0] * len[1]);
+  p.pz = re->pz;   // (the same form and grid: the same rows)
   p.dx = g.cfg.dx;
   p.k = 2 * kPi / g.cfg.wavelength;
   p.teta = teta;
@@ -2375,7 +2395,7 @@ int fdtd_keep_previous_level (fdtd_ctx *ctx, int on)
     return r;
   if (on && !ctx->hprev[0])
     for (int ci = 0; ci < 3; ++ci)
-      if ((r = dalloc (ctx, &ctx->hprev[ci], (size_t) ctx->g.cells * elem_size (ctx->kind))) != FDTD_OK)
+      if ((r = dalloc (ctx, &ctx->hprev[ci], ctx->scells * elem_size (ctx->kind))) != FDTD_OK)
         return r;
   ctx->keep_prev = on != 0;
   ctx->prev_src = 0;

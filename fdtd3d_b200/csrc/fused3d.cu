@@ -88,9 +88,9 @@ __device__ __forceinline__ void tfsf_apply (const FusedParams &p, int k, const d
 // getMetaMaterial does (two points for E, the plain mean of four for H).
 __device__ __forceinline__ void drude_coeffs (const FusedParams &p, int k, int x, int y, int z, float c[5])
 {
-  const int ny = p.g.n[1], nz = p.g.n[2];
-  const size_t stride[3] = {(size_t) ny * nz, (size_t) nz, 1};
-  const size_t id = ((size_t) x * ny + y) * nz + z;
+  const int ny = p.g.n[1], pz = p.g.pz;
+  const size_t stride[3] = {(size_t) ny * pz, (size_t) pz, 1};
+  const size_t id = ((size_t) x * ny + y) * pz + z;
   const int side = k >= 3 ? 1 : 0;
   const float *om = p.omega[side];
   const float *ga = p.gamma[side];
@@ -227,7 +227,7 @@ __device__ __forceinline__ float update_any (const FusedParams &p, unsigned fl, 
 template <typename T, int R, int W, bool META>
 __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *err)
 {
-  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2];
+  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2], pz = p.g.pz;
   const int lane = threadIdx.x;
   const int w = threadIdx.y;
   const int z0 = 1 + blockIdx.x * 31;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *e
   const bool zinner = z <= nz - 2;
   const bool zown = lane < 31 && zinner;
   const unsigned FULL = 0xffffffffu;
-  const size_t sx = (size_t) ny * nz;
+  const size_t sx = (size_t) ny * pz;
 
   __shared__ float sHb[2][W + 1][2][32];   // [parity][warp + 1][Hz, Hx][lane]: row above each warp
   __shared__ float sEb[2][W][2][32];       // [parity][warp][Ex, Ez][lane]: E_new of each warp's first row
@@ -271,11 +271,11 @@ __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *e
   float hp[3][R], ep[3][R], epsc[R];
   unsigned char flp[R];
   {
-    const size_t b0 = (size_t) (xa - 1) * sx + (size_t) yw * nz + z;
+    const size_t b0 = (size_t) (xa - 1) * sx + (size_t) yw * pz + z;
 #pragma unroll
     for (int r = 0; r < R; ++r)
     {
-      const size_t id = b0 + (size_t) r * nz;
+      const size_t id = b0 + (size_t) r * pz;
       hp[0][r] = rvalid[r] ? ldf (Ho0, id) : 0.f;
       hp[1][r] = rvalid[r] ? ldf (Ho1, id) : 0.f;
       hp[2][r] = rvalid[r] ? ldf (Ho2, id) : 0.f;
@@ -288,14 +288,14 @@ __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *e
   for (int x = xa; x <= xb + 1; ++x)
   {
     const int par = x & 1;
-    const size_t b = (size_t) x * sx + (size_t) yw * nz + z;
+    const size_t b = (size_t) x * sx + (size_t) yw * pz + z;
     // ---- loads of plane x (independent, all in flight together)
     float h[3][R], e[3][R], epsn[R];
     unsigned char fl[R];
 #pragma unroll
     for (int r = 0; r < R; ++r)
     {
-      const size_t id = b + (size_t) r * nz;
+      const size_t id = b + (size_t) r * pz;
       h[0][r] = rvalid[r] ? ldf (Ho0, id) : 0.f;
       h[1][r] = rvalid[r] ? ldf (Ho1, id) : 0.f;
       h[2][r] = rvalid[r] ? ldf (Ho2, id) : 0.f;
@@ -309,17 +309,17 @@ __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *e
 #pragma unroll
     for (int r = 0; r < R; ++r)
     {
-      const size_t id = b + (size_t) r * nz;
+      const size_t id = b + (size_t) r * pz;
       const bool rv = yw + r <= ny - 1;
       hzl_x[r] = (lane == 0 && rv) ? ldf (Ho0, id - 1) : 0.f;
       hzl_y[r] = (lane == 0 && rv) ? ldf (Ho1, id - 1) : 0.f;
       epz[r] = (eps && lane == 31 && rv && z + 1 <= nz - 1) ? __ldg (eps + id + 1) : 1.f;
     }
-    const float epsy = (eps && zvalid && yw + R <= ny - 1) ? __ldg (eps + b + (size_t) R * nz) : 1.f;
+    const float epsy = (eps && zvalid && yw + R <= ny - 1) ? __ldg (eps + b + (size_t) R * pz) : 1.f;
     if (w == 0)
     {
-      sHb[par][0][0][lane] = zvalid ? ldf (Ho2, b - nz) : 0.f;
-      sHb[par][0][1][lane] = zvalid ? ldf (Ho0, b - nz) : 0.f;
+      sHb[par][0][0][lane] = zvalid ? ldf (Ho2, b - pz) : 0.f;
+      sHb[par][0][1][lane] = zvalid ? ldf (Ho0, b - pz) : 0.f;
     }
     sHb[par][w + 1][0][lane] = h[2][R - 1];
     sHb[par][w + 1][1][lane] = h[0][R - 1];
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *e
       if (rinner[r] && xin)
       {
         const int y = yw + r;
-        const size_t id = b + (size_t) r * nz;
+        const size_t id = b + (size_t) r * pz;
         float i0 = 1.f, i1 = 1.f, i2 = 1.f;
         if (eps)
         {
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *e
         if (rown[r])
         {
           const int y = yw + r;
-          const size_t hid = b - sx + (size_t) r * nz;
+          const size_t hid = b - sx + (size_t) r * pz;
           const float ez_yp = r < R - 1 ? ep[2][r + 1] : sEb[par ^ 1][w + 1 < W ? w + 1 : w][1][lane];
           const float ex_yp = r < R - 1 ? ep[0][r + 1] : sEb[par ^ 1][w + 1 < W ? w + 1 : w][0][lane];
           float a0 = ep[1][r], a1 = ey_zp, a2 = ep[2][r], a3 = ez_yp;
@@ -467,14 +467,14 @@ __global__ void __launch_bounds__ (32 * W) fused3d_kernel (FusedParams p, int *e
 // bit k of flags[cell]: component k averages a non-zero plasma frequency or
 // collision rate (the averaging stencils of getMetaMaterial)
 __global__ void drude_flags_kernel (unsigned char *flags, const float *ome, const float *gae, const float *omm,
-                                    const float *gam, int nx, int ny, int nz)
+                                    const float *gam, int nx, int ny, int nz, int pz)
 {
-  const size_t n = (size_t) nx * ny * nz;
-  const size_t stride[3] = {(size_t) ny * nz, (size_t) nz, 1};
+  const size_t n = (size_t) nx * ny * pz;   // (cells past nz hold zeros and get no flag)
+  const size_t stride[3] = {(size_t) ny * pz, (size_t) pz, 1};
   for (size_t id = (size_t) blockIdx.x * blockDim.x + threadIdx.x; id < n; id += (size_t) gridDim.x * blockDim.x)
   {
-    const int z = (int) (id % nz);
-    const int y = (int) ((id / nz) % ny);
+    const int z = (int) (id % pz);
+    const int y = (int) ((id / pz) % ny);
     const int x = (int) (id / stride[0]);
     const int pos[3] = {x, y, z};
     const int lim[3] = {nx, ny, nz};
@@ -569,15 +569,15 @@ namespace {
 
 // Bounding box of the cells with any Drude flag: box[0..2] = lowest x, y, z
 // (atomicMin from INT_MAX), box[3..5] = highest (atomicMax from -1).
-__global__ void drude_box_kernel (const unsigned char *flags, int nx, int ny, int nz, int *box)
+__global__ void drude_box_kernel (const unsigned char *flags, int nx, int ny, int pz, int *box)
 {
-  const size_t n = (size_t) nx * ny * nz;
+  const size_t n = (size_t) nx * ny * pz;
   int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1};
   for (size_t id = (size_t) blockIdx.x * blockDim.x + threadIdx.x; id < n; id += (size_t) gridDim.x * blockDim.x)
   {
     if (!flags[id])
       continue;
-    const int pos[3] = {(int) (id / ((size_t) ny * nz)), (int) ((id / nz) % ny), (int) (id % nz)};
+    const int pos[3] = {(int) (id / ((size_t) ny * pz)), (int) ((id / pz) % ny), (int) (id % pz)};
     for (int a = 0; a < 3; ++a)
     {
       lo[a] = min (lo[a], pos[a]);
@@ -610,8 +610,8 @@ __global__ void drude_box_kernel (const unsigned char *flags, int nx, int ny, in
 template <typename T>
 __global__ void __launch_bounds__ (256) drude_fix_e_kernel (const __grid_constant__ FusedParams p, DrudeBox b)
 {
-  const int ny = p.g.n[1], nz = p.g.n[2];
-  const size_t sx = (size_t) ny * nz;
+  const int ny = p.g.n[1], pz = p.g.pz;
+  const size_t sx = (size_t) ny * pz;
   const int ez = b.hi[2] - b.lo[2], ey = b.hi[1] - b.lo[1];
   const long long total = (long long) (b.hi[0] - b.lo[0]) * ey * ez;
   const T *Ho0 = (const T *) p.h_old[0], *Ho1 = (const T *) p.h_old[1], *Ho2 = (const T *) p.h_old[2];
@@ -621,13 +621,13 @@ __global__ void __launch_bounds__ (256) drude_fix_e_kernel (const __grid_constan
     const int z = b.lo[2] + (int) (t % ez);
     const int y = b.lo[1] + (int) ((t / ez) % ey);
     const int x = b.lo[0] + (int) (t / ((long long) ez * ey));
-    const size_t id = (size_t) x * sx + (size_t) y * nz + z;
+    const size_t id = (size_t) x * sx + (size_t) y * pz + z;
     const unsigned fl = p.dflag[id];
     if (!(fl & 7u))
       continue;
     if (fl & 1u)
     {
-      const float c = (ldf (Ho2, id) - ldf (Ho2, id - nz)) - (ldf (Ho1, id) - ldf (Ho1, id - 1));
+      const float c = (ldf (Ho2, id) - ldf (Ho2, id - pz)) - (ldf (Ho1, id) - ldf (Ho1, id - 1));
       stf ((T *) p.e_new[0], id, update_drude (p, 0, ldf ((const T *) p.e_old[0], id), c, x, y, z, id, true));
     }
     if (fl & 2u)
@@ -637,7 +637,7 @@ __global__ void __launch_bounds__ (256) drude_fix_e_kernel (const __grid_constan
     }
     if (fl & 4u)
     {
-      const float c = (ldf (Ho1, id) - ldf (Ho1, id - sx)) - (ldf (Ho0, id) - ldf (Ho0, id - nz));
+      const float c = (ldf (Ho1, id) - ldf (Ho1, id - sx)) - (ldf (Ho0, id) - ldf (Ho0, id - pz));
       stf ((T *) p.e_new[2], id, update_drude (p, 2, ldf ((const T *) p.e_old[2], id), c, x, y, z, id, true));
     }
   }
@@ -661,8 +661,8 @@ __device__ __forceinline__ float ld_new<__half> (const __half *p, size_t i)
 template <typename T>
 __global__ void __launch_bounds__ (256) drude_fix_h_kernel (const __grid_constant__ FusedParams p, DrudeBox b)
 {
-  const int ny = p.g.n[1], nz = p.g.n[2];
-  const size_t sx = (size_t) ny * nz;
+  const int ny = p.g.n[1], pz = p.g.pz;
+  const size_t sx = (size_t) ny * pz;
   const int ez = b.hi[2] - b.lo[2], ey = b.hi[1] - b.lo[1];
   const long long total = (long long) (b.hi[0] - b.lo[0]) * ey * ez;
   const T *E0 = (const T *) p.e_new[0], *E1 = (const T *) p.e_new[1], *E2 = (const T *) p.e_new[2];
@@ -672,12 +672,12 @@ __global__ void __launch_bounds__ (256) drude_fix_h_kernel (const __grid_constan
     const int z = b.lo[2] + (int) (t % ez);
     const int y = b.lo[1] + (int) ((t / ez) % ey);
     const int x = b.lo[0] + (int) (t / ((long long) ez * ey));
-    const size_t id = (size_t) x * sx + (size_t) y * nz + z;
+    const size_t id = (size_t) x * sx + (size_t) y * pz + z;
     const unsigned fl = p.dflag[id];
     const float ex = ld_new (E0, id), ey_ = ld_new (E1, id), ez_ = ld_new (E2, id);
-    const float a = (ld_new (E1, id + 1) - ey_) - (ld_new (E2, id + nz) - ez_);
+    const float a = (ld_new (E1, id + 1) - ey_) - (ld_new (E2, id + pz) - ez_);
     const float bb = (ld_new (E2, id + sx) - ez_) - (ld_new (E0, id + 1) - ex);
-    const float c = (ld_new (E0, id + nz) - ex) - (ld_new (E1, id + sx) - ey_);
+    const float c = (ld_new (E0, id + pz) - ex) - (ld_new (E1, id + sx) - ey_);
     auto inside = [&] (int k) {
       return x >= p.ilo[k][0] && x < p.ihi[k][0] && y >= p.ilo[k][1] && y < p.ihi[k][1] && z >= p.ilo[k][2] &&
              z < p.ihi[k][2];
@@ -696,16 +696,16 @@ __global__ void __launch_bounds__ (256) drude_fix_h_kernel (const __grid_constan
 
 }  // namespace
 
-int launch_drude_box (const unsigned char *flags, int nx, int ny, int nz, int *box, cudaStream_t s)
+int launch_drude_box (const unsigned char *flags, int nx, int ny, int pz, int *box, cudaStream_t s)
 {
   const int init[6] = {INT_MAX, INT_MAX, INT_MAX, -1, -1, -1};
   if (cudaMemcpyAsync (box, init, sizeof (init), cudaMemcpyHostToDevice, s) != cudaSuccess)
     return 0;
-  size_t n = (size_t) nx * ny * nz;
+  size_t n = (size_t) nx * ny * pz;
   size_t blocks = (n + 255) / 256;
   if (blocks > 148 * 16)
     blocks = 148 * 16;
-  drude_box_kernel<<<(unsigned) blocks, 256, 0, s>>> (flags, nx, ny, nz, box);
+  drude_box_kernel<<<(unsigned) blocks, 256, 0, s>>> (flags, nx, ny, pz, box);
   return 1;
 }
 
@@ -737,8 +737,8 @@ __global__ void current_fix_kernel (FusedParams p, CurrentFix cf, const double *
 {
   if (threadIdx.x != 0 || blockIdx.x != 0)
     return;
-  const int ny = p.g.n[1], nz = p.g.n[2];
-  const size_t st[3] = {(size_t) ny * nz, (size_t) nz, 1};
+  const int ny = p.g.n[1], pz = p.g.pz;
+  const size_t st[3] = {(size_t) ny * pz, (size_t) pz, 1};
   const size_t c = (size_t) cf.pos[0] * st[0] + (size_t) cf.pos[1] * st[1] + cf.pos[2];
   const float S = p.courant;
   auto rmw = [&] (void *f, size_t id, float d) {
@@ -793,13 +793,13 @@ int launch_current_fix (const FusedParams &p, const CurrentFix &cf, const double
 }
 
 int launch_drude_flags (unsigned char *flags, const float *ome, const float *gae, const float *omm, const float *gam,
-                        int nx, int ny, int nz, cudaStream_t s)
+                        int nx, int ny, int nz, int pz, cudaStream_t s)
 {
-  size_t n = (size_t) nx * ny * nz;
+  size_t n = (size_t) nx * ny * pz;
   size_t blocks = (n + 255) / 256;
   if (blocks > 148 * 32)
     blocks = 148 * 32;
-  drude_flags_kernel<<<(unsigned) blocks, 256, 0, s>>> (flags, ome, gae, omm, gam, nx, ny, nz);
+  drude_flags_kernel<<<(unsigned) blocks, 256, 0, s>>> (flags, ome, gae, omm, gam, nx, ny, nz, pz);
   return 1;
 }
 

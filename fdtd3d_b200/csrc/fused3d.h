@@ -65,8 +65,9 @@ struct DrudeBox
 };
 
 // Bounding box of the cells with a Drude flag into box[6] (device ints:
-// lowest x, y, z, then highest; INT_MAX / -1 when no cell has one).
-int launch_drude_box (const unsigned char *flags, int nx, int ny, int nz, int *box, cudaStream_t s);
+// lowest x, y, z, then highest; INT_MAX / -1 when no cell has one); rows of
+// pz stored cells.
+int launch_drude_box (const unsigned char *flags, int nx, int ny, int pz, int *box, cudaStream_t s);
 
 // Drude fix-up of a TMA sweep step over the Drude cells of `box` (two
 // launches; returns how many).
@@ -92,6 +93,6 @@ int launch_current_fix (const FusedParams &p, const CurrentFix &cf, const double
 
 // Recomputes the per-cell Drude bitmask from the four material arrays.
 int launch_drude_flags (unsigned char *flags, const float *ome, const float *gae, const float *omm, const float *gam,
-                        int nx, int ny, int nz, cudaStream_t s);
+                        int nx, int ny, int nz, int pz, cudaStream_t s);
 
 }  // namespace fdtdb

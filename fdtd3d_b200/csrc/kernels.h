@@ -94,8 +94,11 @@ int launch_fast_point_source (void *f, int fp16, size_t index, const double *src
                               cudaStream_t s);
 
 // conversions between host-order FP64 arrays and the stored forms
-int launch_convert_in (void *dst, int dst_kind, const double *src, size_t n, double scale, cudaStream_t s);
-int launch_convert_out (double *dst, const void *src, int src_kind, size_t n, double scale, cudaStream_t s);
+// (rows of nz cells, pz stored cells per row on the library's side)
+int launch_convert_in (void *dst, int dst_kind, const double *src, size_t rows, int nz, int pz, double scale,
+                       cudaStream_t s);
+int launch_convert_out (double *dst, const void *src, int src_kind, size_t rows, int nz, int pz, double scale,
+                        cudaStream_t s);
 // kinds: 0 = double, 1 = float, 2 = __half
 // *first = min(*first, index of every NaN / Inf among src[0 .. n))
 int launch_find_nonfinite (const double *src, size_t n, unsigned long long *first, cudaStream_t s);
@@ -108,8 +111,8 @@ int launch_fill (double *dst, size_t n, double value, cudaStream_t s);
 // one step of the running DFT of a stored field (kind 0 double, 1 float,
 // 2 half) on the plane x_axis = index; phase: (cos, sin) per frequency;
 // acc: (re, re comp., im, im comp.) per frequency and plane cell
-int launch_dft (const void *src, int kind, int axis, int index, const int n[3], double scale, const double *phase,
-                int nf, double *acc, int sm_count, cudaStream_t s);
+int launch_dft (const void *src, int kind, int axis, int index, const int n[3], int pz, double scale,
+                const double *phase, int nf, double *acc, int sm_count, cudaStream_t s);
 int launch_reduce_final (const double *partials, int nblocks, double *out, cudaStream_t s);
 // the two reduction launches with their own launch status (cudaLaunchKernel)
 cudaError_t launch_reduce_sq_checked (const void *src, int kind, size_t n, const void *weight, int wkind,

@@ -54,7 +54,7 @@ __device__ __forceinline__ int64_t cell (const NtffParams &p, const double q[3])
 #pragma unroll
   for (int a = 0; a < 3; ++a)
     i[a] = min (max ((int) q[a], 0), p.n[a] - 1);
-  return ((int64_t) i[0] * p.n[1] + i[1]) * p.n[2] + i[2];
+  return ((int64_t) i[0] * p.n[1] + i[1]) * p.pz + i[2];
 }
 
 // A stored field value in physical units (FP64 as stored; FP32 / FP16

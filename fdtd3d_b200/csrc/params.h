@@ -45,6 +45,7 @@ struct CompDev
 struct GeomDev
 {
   int n[3];
+  int pz;                     // stored cells per z row: n[2], or n[2] rounded up (FP32 / FP16 rows of 16-byte units)
   int drop;                   // bit a: axis a has size 1 (2-D / 1-D modes)
   int inc_ax[2];              // 2-D / 1-D: incident distance u k0 + v k1 along these axes
   double inc_k[2];

@@ -223,8 +223,8 @@ __global__ void __launch_bounds__ (32 * NW, 1)
 
   const int lane = threadIdx.x, w = threadIdx.y;
   const bool leader = w == 0 && lane == 0;
-  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2];
-  const size_t sx = (size_t) ny * nz;
+  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2], pz = p.g.pz;
+  const size_t sx = (size_t) ny * pz;
   const uint32_t raw = tma::smem_addr (smem_raw);
   const uint32_t sbase = (raw + 127u) & ~127u;
   unsigned char *const smem = smem_raw + (sbase - raw);
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__ (32 * NW, 1)
           cupd |= 1u << j;
     }
     const bool own = w >= 1 && w <= kTb2Yown && r < wk.yend && lane >= L::OLO && lane <= L::OHI && zc >= 0 && zc < nz;
-    const size_t rowoff = (size_t) r * nz + zc;
+    const size_t rowoff = (size_t) r * pz + zc;
     // y / z membership of this lane's cells in each component's sigma = 0
     // box: bit 2k + j (k = 0 .. 5, cell j) of yz_in
     unsigned yz_in = 0;
@@ -737,12 +737,12 @@ std::string plan_t (Sweep2Plan &pl, const FusedParams &p, void *const e[2][3], v
   {
     Sweep2Maps &m = pl.maps[b];
     for (int c = 0; c < 3; ++c)
-      if (!make_map (m.h[c], h[b][c], half, p.g.n, L::HW, L::HR) ||
-          !make_map (m.e[c], e[b][c], half, p.g.n, L::EW, L::ER))
+      if (!make_map (m.h[c], h[b][c], half, p.g, L::HW, L::HR) ||
+          !make_map (m.e[c], e[b][c], half, p.g, L::EW, L::ER))
         return "tensor map encoding failed";
     if (eps)
     {
-      if (!make_map (m.eps, eps, false, p.g.n, L::PW, L::PR))
+      if (!make_map (m.eps, eps, false, p.g, L::PW, L::PR))
         return "tensor map encoding failed";
     }
     else
@@ -751,7 +751,7 @@ std::string plan_t (Sweep2Plan &pl, const FusedParams &p, void *const e[2][3], v
     {
       if (p.use_pml && aux && aux[b][k])
       {
-        if (!make_map (m.aux[k], aux[b][k], false, p.g.n, ZW, NW))
+        if (!make_map (m.aux[k], aux[b][k], false, p.g, ZW, NW))
           return "tensor map encoding failed";
       }
       else
@@ -834,8 +834,8 @@ std::string sweep2_plan (Sweep2Plan &plan, const FusedParams &p, void *const e[2
   if (p.use_meta)
     return "metamaterials";
   const int unit = p.fp16 ? 8 : 4;
-  if (n[2] % unit != 0)
-    return "nz is not a multiple of one 16-byte unit";
+  if (p.g.pz % unit != 0)
+    return "the stored rows are not a multiple of one 16-byte unit";
   if (n[0] < 3 || n[1] < 3 || n[2] < 3)
     return "grid too small";
   if (x1 < 0)

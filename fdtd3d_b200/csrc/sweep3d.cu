@@ -404,8 +404,8 @@ __global__ void __launch_bounds__ (32 * WY, 1)
   const int lane = threadIdx.x, w = threadIdx.y;
   const int tid = w * 32 + lane;
   const bool leader = tid == 0;
-  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2];
-  const size_t sx = (size_t) ny * nz;
+  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2], pz = p.g.pz;
+  const size_t sx = (size_t) ny * pz;
   // 128-byte aligned base of the dynamic shared memory (TMA destinations)
   const uint32_t raw = smem_addr (smem_raw);
   const uint32_t sbase = (raw + 127u) & ~127u;
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__ (32 * WY, 1)
     const int y = y0 + w;
     const bool yupd = y <= ny - 2;
     const bool own_row = w < WY - 1 && yupd;
-    const size_t rowoff = (size_t) y * nz + zc;
+    const size_t rowoff = (size_t) y * pz + zc;
     unsigned zupd = 0, zface = 0, zin = 0, yin = 0;   // zin bit 4k + j, yin bit k
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -1088,8 +1088,8 @@ __global__ void __launch_bounds__ (256) tfsf_post_kernel (const __grid_constant_
   int x, y, z;
   if (!band_cell (b, bk.y, x, y, z))
     return;
-  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2];
-  const size_t sx = (size_t) ny * nz;
+  const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2], pz = p.g.pz;
+  const size_t sx = (size_t) ny * pz;
   const float S = p.courant;
   // correction of E component k at (cx, cy, cz) from its terms in mask m:
   // zero where the step does not update the cell and on the point source
@@ -1105,14 +1105,14 @@ __global__ void __launch_bounds__ (256) tfsf_post_kernel (const __grid_constant_
     float im = 1.f;
     if (p.eps)
     {
-      const size_t c = (size_t) cx * sx + (size_t) cy * nz + cz;
-      const size_t st = k == 0 ? sx : (k == 1 ? (size_t) nz : 1);
+      const size_t c = (size_t) cx * sx + (size_t) cy * pz + cz;
+      const size_t st = k == 0 ? sx : (k == 1 ? (size_t) pz : 1);
       im = __fdividef (2.f, p.eps[c] + p.eps[c + st]);
     }
     return (S * im) * d;
   };
   auto em = [] (unsigned mask, int k) { return (mask >> (4 * k)) & 15u; };
-  const size_t id = (size_t) x * sx + (size_t) y * nz + z;
+  const size_t id = (size_t) x * sx + (size_t) y * pz + z;
   const float d0 = de (0, em (b.mask, 0), x, y, z), d1 = de (1, em (b.mask, 1), x, y, z),
               d2 = de (2, em (b.mask, 2), x, y, z);
   const float dd[3] = {d0, d1, d2};
@@ -1163,8 +1163,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn ()
 
 }  // namespace
 
-// 3-D map over an (nx, ny, nz) array, z fastest, box bw x bh x 1
-bool make_map (CUtensorMap &m, const void *base, bool half, const int n[3], int bw, int bh)
+// 3-D map over the stored (nx, ny, pz) array, z fastest, box bw x bh x 1
+bool make_map (CUtensorMap &m, const void *base, bool half, const GeomDev &g, int bw, int bh)
 {
   // L2 fetch granularity of the copies: 64 bytes measured best at 512^3
   // with the concurrent class launches (1.673 ms per step against 1.681 for
@@ -1174,8 +1174,8 @@ bool make_map (CUtensorMap &m, const void *base, bool half, const int n[3], int 
   if (!fn)
     return false;
   const cuuint64_t es = half ? 2 : 4;
-  cuuint64_t dims[3] = {(cuuint64_t) n[2], (cuuint64_t) n[1], (cuuint64_t) n[0]};
-  cuuint64_t strides[2] = {(cuuint64_t) n[2] * es, (cuuint64_t) n[2] * (cuuint64_t) n[1] * es};
+  cuuint64_t dims[3] = {(cuuint64_t) g.pz, (cuuint64_t) g.n[1], (cuuint64_t) g.n[0]};
+  cuuint64_t strides[2] = {(cuuint64_t) g.pz * es, (cuuint64_t) g.pz * (cuuint64_t) g.n[1] * es};
   cuuint32_t box[3] = {(cuuint32_t) bw, (cuuint32_t) bh, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn (&m, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
@@ -1196,13 +1196,13 @@ std::string plan_t (SweepPlan &pl, const FusedParams &p, void *const e[2][3], vo
   {
     SweepMaps &m = pl.maps[b];
     for (int c = 0; c < 3; ++c)
-      if (!make_map (m.h[c], h[b][c], half, p.g.n, L::HW, WY + 1) ||
-          !make_map (m.e[c], e[b][c], half, p.g.n, L::EW, WY))
+      if (!make_map (m.h[c], h[b][c], half, p.g, L::HW, WY + 1) ||
+          !make_map (m.e[c], e[b][c], half, p.g, L::EW, WY))
         return "tensor map encoding failed";
     // descriptors the kernel never uses are copies of a valid one
     if (eps)
     {
-      if (!make_map (m.eps, eps, false, p.g.n, PW, WY))
+      if (!make_map (m.eps, eps, false, p.g, PW, WY))
         return "tensor map encoding failed";
     }
     else
@@ -1211,8 +1211,8 @@ std::string plan_t (SweepPlan &pl, const FusedParams &p, void *const e[2][3], vo
     {
       if (p.use_pml)
       {
-        if (!aux[b][k] || !make_map (m.aux[k], aux[b][k], false, p.g.n, PW, WY) ||
-            !make_map (m.auxn[k], aux[b][k], false, p.g.n, L::AN, WY))
+        if (!aux[b][k] || !make_map (m.aux[k], aux[b][k], false, p.g, PW, WY) ||
+            !make_map (m.auxn[k], aux[b][k], false, p.g, L::AN, WY))
           return "tensor map encoding failed";
       }
       else
@@ -1345,8 +1345,8 @@ std::string sweep3d_plan (SweepPlan &plan, const FusedParams &p, void *const e[2
   if (p.g.drop != 0)
     return "2-D grid";
   const int unit = p.fp16 ? 8 : 4;
-  if (n[2] % unit != 0)
-    return "nz is not a multiple of one 16-byte unit";
+  if (p.g.pz % unit != 0)
+    return "the stored rows are not a multiple of one 16-byte unit";
   if (n[0] < 3 || n[1] < 3 || n[2] < 3)
     return "grid too small";
   if (wy != 8)

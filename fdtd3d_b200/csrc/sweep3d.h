@@ -1,6 +1,6 @@
 // sweep3d.h - TMA-pipelined one-sweep E+H step for the 3-D FP32 and
-// FP16-storage forms (uniform mu, no metamaterials, nz a multiple of one
-// 16-byte unit).
+// FP16-storage forms (uniform mu, no metamaterials, stored rows a multiple of
+// one 16-byte unit).
 #pragma once
 
 #include <cuda.h>
@@ -25,9 +25,9 @@ struct SweepMaps
   CUtensorMap auxn[6];         // narrow (32-cell) boxes for planes whose PML cells are all at a z edge
 };
 
-// Tiled 3-D tensor map over an (n[0], n[1], n[2]) array (z fastest, FP32 or
-// FP16), box bw (z) x bh (y) x 1 (x), 64-byte L2 promotion, zero fill.
-bool make_map (CUtensorMap &m, const void *base, bool half, const int n[3], int bw, int bh);
+// Tiled 3-D tensor map over a stored (n[0], n[1], pz) array (z fastest, FP32
+// or FP16), box bw (z) x bh (y) x 1 (x), 64-byte L2 promotion, zero fill.
+bool make_map (CUtensorMap &m, const void *base, bool half, const GeomDev &g, int bw, int bh);
 
 constexpr int kMaxChunks = 256;   // x chunks per step (the chunk grows for larger grids)
 

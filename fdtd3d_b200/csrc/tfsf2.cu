@@ -144,7 +144,7 @@ __global__ void __launch_bounds__ (256, 4) tfsf2_fused (const __grid_constant__ 
   float *const sH = sE + 3 * nE;
   float *const sP = sH + 3 * nH;
   const int nx = p.g.n[0], ny = p.g.n[1], nz = p.g.n[2];
-  const size_t sx = (size_t) ny * nz, sy = nz;
+  const size_t sx = (size_t) ny * p.g.pz, sy = p.g.pz;
   const float S = p.courant;
   const int o[3] = {t.lo[0] - 1, t.lo[1] - 1, t.lo[2] - 1};   // origin of every domain
   const bool has_eps = p.eps != nullptr;

@@ -1,0 +1,54 @@
+"""FP32 / FP16-storage 3-D grids whose rows are no whole number of 16-byte
+units: they store padded rows, so that the TMA kernels serve them.  Fields,
+uploads, the energy and the DFT are checked against the FP64 plain form (its
+rows are never padded)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+COMPS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
+ETA0 = 376.730313461770655
+
+
+def _family(got, ref, fam):
+    g = np.concatenate([got[c].ravel() for c in COMPS if c[0] == fam])
+    r = np.concatenate([ref[c].ravel() for c in COMPS if c[0] == fam])
+    return np.linalg.norm(g - r) / np.linalg.norm(r)
+
+
+# nz = 31: the last length that keeps its rows; 32, 56: whole units of both
+# types; 127 .. 133: around one 128-cell tile; 33 .. 36, 63: every remainder
+@pytest.mark.parametrize("nz", [31, 32, 33, 34, 35, 36, 56, 63, 127, 129, 133])
+@pytest.mark.parametrize("prec,tol", [(1, 1e-5), (2, 2e-2)])
+def test_padded_rows_match_fp64(fdtd, nz, prec, tol):
+    shape = (40, 37, nz)
+    rng = np.random.default_rng(nz)
+    # noise resumed at t = 30, with values FP16 storage holds exactly
+    fields = {c: np.zeros(shape) for c in COMPS}
+    for c in COMPS:
+        v = rng.standard_normal(tuple(n - 2 for n in shape)).astype(np.float16).astype(np.float64)
+        fields[c][1:-1, 1:-1, 1:-1] = v / (1.0 if c[0] == "E" else ETA0)
+    eps = 1.0 + np.kron(rng.uniform(0, 3, (7, 7, nz // 6 + 1)), np.ones((6, 6, 6)))[:40, :37, :nz].astype(np.float32)
+    kw = dict(mode=3, size=shape, use_pml=True, pml=4, use_tfsf=True, tfsf_left=13, tfsf_right=13, teta=30, phi=45,
+              psi=20)
+    out, spectrum, energy = {}, {}, {}
+    for p in (0, prec):
+        with fdtd.Simulation(materials={"eps": eps}, precision=p, **kw) as sim:
+            for c, v in fields.items():
+                sim.set_field(c, v)
+                if p == 1:
+                    np.testing.assert_allclose(sim.field(c), v, rtol=1e-6, atol=0)
+            sim.step(12, t_start=30)
+            sim.dft_setup("Ey", 1, 17, [15e9, 9e9])
+            sim.step(3)
+            out[p] = {c: sim.field(c) for c in COMPS}
+            spectrum[p], energy[p] = sim.dft(), sim.reduce()[0]
+            if p:
+                unit = 8 if p == 2 else 4
+                want = "fused3d_regblock" if nz < 32 and nz % unit else "sweep3d_tma"
+                assert sim.step_kernel == want, sim.step_kernel
+    for fam in "EH":
+        assert _family(out[prec], out[0], fam) <= tol, (nz, fam, _family(out[prec], out[0], fam))
+    assert np.linalg.norm(spectrum[prec] - spectrum[0]) <= tol * np.linalg.norm(spectrum[0])
+    assert abs(energy[prec] / energy[0] - 1) <= tol
