@@ -76,6 +76,7 @@ struct fdtd_ctx
   double *einc[2] = {nullptr, nullptr};
   double *hinc[2] = {nullptr, nullptr};
   int ecur = 0, hcur = 0;
+  int64_t inc_steps = 0;   // incident E steps taken: cells from that index on still hold 0 at both levels
 
   // per-step source table: [incident, point source E, point source H]
   double *d_src = nullptr;
@@ -88,6 +89,7 @@ struct fdtd_ctx
   double *dd[6][3] = {};
   double *d1[6][3] = {};
   double *mat64[6] = {};
+  bool mat_set[2] = {false, false};   // eps / mu uploaded (else uniform 1)
   double *sig64[3] = {};
   double *ptab[6][6] = {};   // FP64 plain form: PML coefficient tables per component (PlainTabs)
   // double material precision: eps / mu per component averaged from the fine
@@ -1452,6 +1454,37 @@ void dft_step (fdtd_ctx *ctx, uint32_t i)
                                ctx->sm_count, ctx->stream);
 }
 
+// Incident-grid steps.  The wave enters at cell 0 and moves one cell per
+// step, so after k E steps only cells 0 .. k - 1 hold anything but 0: the
+// updates stop there (the grid is 500 times the first axis long, 40 000 cells
+// at 80^3).
+IncidentJob incident_e_job (fdtd_ctx *ctx, uint32_t i)
+{
+  ++ctx->inc_steps;
+  IncidentJob j;
+  j.now = ctx->einc[1 - ctx->ecur];
+  j.old = ctx->einc[ctx->ecur];
+  j.other = ctx->hinc[ctx->hcur];
+  j.cells = (int) std::min<int64_t> (ctx->g.inc_len, ctx->inc_steps + 1);
+  j.modifier = ctx->g.mod_e;
+  j.src = ctx->d_src + kSrcStride * i;
+  ctx->ecur ^= 1;
+  return j;
+}
+
+IncidentJob incident_h_job (fdtd_ctx *ctx)
+{
+  IncidentJob j;
+  j.now = ctx->hinc[1 - ctx->hcur];
+  j.old = ctx->hinc[ctx->hcur];
+  j.other = ctx->einc[ctx->ecur];
+  j.cells = (int) std::min<int64_t> (ctx->g.inc_len - 1, ctx->inc_steps + 1);
+  j.modifier = ctx->g.mod_h;
+  j.src = nullptr;
+  ctx->hcur ^= 1;
+  return j;
+}
+
 int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
 {
   const Geometry &g = ctx->g;
@@ -1549,12 +1582,8 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
       }
       if (g.cfg.use_tfsf)
       {
-        ctx->launches += launch_incident_e (ctx->einc[1 - ctx->ecur], ctx->einc[ctx->ecur], ctx->hinc[ctx->hcur],
-                                            g.inc_len, g.mod_e, ctx->d_src, kSrcStride * i, si);
-        ctx->ecur ^= 1;
-        ctx->launches += launch_incident_h (ctx->hinc[1 - ctx->hcur], ctx->hinc[ctx->hcur], ctx->einc[ctx->ecur],
-                                            g.inc_len, g.mod_h, si);
-        ctx->hcur ^= 1;
+        ctx->launches += launch_incident_e (incident_e_job (ctx, i), si);
+        ctx->launches += launch_incident_h (incident_h_job (ctx), si);
       }
       f.inc_h = ctx->hinc[hprev];
       f.inc_e = ctx->einc[ctx->ecur];
@@ -1573,13 +1602,9 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
           inc_h1 = ctx->hinc_keep;
           inc_e1 = ctx->einc[ctx->ecur];
           inc_h2 = ctx->hinc[ctx->hcur];
-          ctx->launches += launch_incident_e (ctx->einc[1 - ctx->ecur], ctx->einc[ctx->ecur], ctx->hinc[ctx->hcur],
-                                              g.inc_len, g.mod_e, ctx->d_src, kSrcStride * (i + 1), si);
-          ctx->ecur ^= 1;
+          ctx->launches += launch_incident_e (incident_e_job (ctx, i + 1), si);
           inc_e2 = ctx->einc[ctx->ecur];
-          ctx->launches += launch_incident_h (ctx->hinc[1 - ctx->hcur], ctx->hinc[ctx->hcur], ctx->einc[ctx->ecur],
-                                              g.inc_len, g.mod_h, si);
-          ctx->hcur ^= 1;
+          ctx->launches += launch_incident_h (incident_h_job (ctx), si);
           if (inc_side)
             CK (cudaEventRecord (ctx->inc_done, si));
         }
@@ -1656,37 +1681,39 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
     }
     for (int h = 0; h < 2; ++h)
     {
+      // the FP64 3-D form takes the incident step in its half-step's launch:
+      // the E half reads HInc before its update, the H half EInc after its
+      const bool march = ctx->kind == 0 && t > 0 && g.drop == 0 && !g.cfg.use_metamaterials && ctx->cs_mask[h] == 0;
+      const double *inc_read = h ? ctx->einc[ctx->ecur] : ctx->hinc[ctx->hcur];
+      IncidentJob job{};
       if (g.cfg.use_tfsf)
       {
-        if (!h)
-        {
-          ctx->launches += launch_incident_e (ctx->einc[1 - ctx->ecur], ctx->einc[ctx->ecur],
-                                              ctx->hinc[ctx->hcur], g.inc_len, g.mod_e, ctx->d_src, kSrcStride * i, s);
-          ctx->ecur ^= 1;
-        }
-        else
-        {
-          ctx->launches += launch_incident_h (ctx->hinc[1 - ctx->hcur], ctx->hinc[ctx->hcur],
-                                              ctx->einc[ctx->ecur], g.inc_len, g.mod_h, s);
-          ctx->hcur ^= 1;
-        }
+        job = h ? incident_h_job (ctx) : incident_e_job (ctx, i);
+        if (!march)
+          ctx->launches += h ? launch_incident_h (job, s) : launch_incident_e (job, s);
       }
       if (ctx->kind == 0)
       {
         if (t > 0)
         {
           PlainHalf p = plain_half (ctx, h);
+          p.inc = inc_read;
           p.cs_val = ctx->d_src + kSrcStride * i + 3 + h;
           cudaEvent_t pe;
           if ((r = prof_begin (ctx, &pe)) != FDTD_OK)
             return r;
-          if (p.cs_mask == 0 && (!g.cfg.use_pml || ctx->ptab[3 * h][0] || ctx->ptab[3 * h + 1][0] ||
-                                 ctx->ptab[3 * h + 2][0]))
+          PlainTabs tb;
+          for (int ci = 0; ci < 3; ++ci)
+            for (int j = 0; j < 6; ++j)
+              tb.t[ci][j] = ctx->ptab[ci + 3 * h][j];
+          if (march)
           {
-            PlainTabs tb;
-            for (int ci = 0; ci < 3; ++ci)
-              for (int j = 0; j < 6; ++j)
-                tb.t[ci][j] = ctx->ptab[ci + 3 * h][j];
+            const bool uniform = g.dmp ? !ctx->matc64[3 * h] : !ctx->mat_set[h];
+            ctx->launches += launch_plain_march (p, tb, job, uniform, g.inc_len, ctx->d_err, ctx->sm_count, s);
+          }
+          else if (p.cs_mask == 0 && (!g.cfg.use_pml || ctx->ptab[3 * h][0] || ctx->ptab[3 * h + 1][0] ||
+                                      ctx->ptab[3 * h + 2][0]))
+          {
             ctx->launches += launch_plain_fast (p, tb, g.inc_len, ctx->d_err, ctx->sm_count, s);
           }
           else
@@ -1842,6 +1869,8 @@ int fdtd_upload_material_device (fdtd_ctx *ctx, int which, const double *dev)
   {
     if (!ctx->mat64[which])
       return fail (ctx, FDTD_ERR_UNSUPPORTED, "Drude grids need use_metamaterials");
+    if (which < 2)
+      ctx->mat_set[which] = true;
     CK (cudaMemcpyAsync (ctx->mat64[which], dev, n * sizeof (double), cudaMemcpyDeviceToDevice, ctx->stream));
     return FDTD_OK;
   }

@@ -69,10 +69,23 @@ int launch_plain_tables (const PlainHalf &p, double *const out[3][6], cudaStream
 // Returns the launches.
 int launch_plain_fast (const PlainHalf &p, const PlainTabs &t, int inc_len, int *err, int sm_count,
                        cudaStream_t s);
-int launch_incident_e (double *e_new, const double *e_old, const double *h_old, int len, double modifier,
-                       const double *src, int src_index, cudaStream_t s);
-int launch_incident_h (double *h_new, const double *h_old, const double *e_new, int len, double modifier,
-                       cudaStream_t s);
+// 3-D, no metamaterials, no current source: one half-step of the FP64 plain
+// form by columns (plain_march_kernel), with the half-step's update of the
+// 1-D incident grid in the same launch (inc.cells > 0).  mat_uniform: the
+// family's material was never uploaded (1 everywhere).
+struct IncidentJob
+{
+  double *now;                 // level written
+  const double *old;           // the same family's previous level
+  const double *other;         // E: HInc before its update; H: EInc after its update
+  int cells;                   // cells 0 .. cells - 1 are updated (0: nothing to do)
+  double modifier;
+  const double *src;           // E: value of cell 0
+};
+int launch_plain_march (const PlainHalf &p, const PlainTabs &t, const IncidentJob &inc, bool mat_uniform, int inc_len,
+                        int *err, int sm_count, cudaStream_t s);
+int launch_incident_e (const IncidentJob &j, cudaStream_t s);
+int launch_incident_h (const IncidentJob &j, cudaStream_t s);
 int launch_point_source (double *f, size_t index, const double *src, int src_index, cudaStream_t s);
 
 // Double material precision: per coarse cell, the average of the fine cells

@@ -15,6 +15,9 @@
 //   (YeeGridLayout.h:866-1030, Approximation.cpp:34-54), once per upload.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "cell_walk.cuh"
 #include "kernels.h"
 #include "plain_cell.cuh"
@@ -45,23 +48,21 @@ __global__ void __launch_bounds__ (256) plain_half_kernel (PlainHalf p, int inc_
   }
 }
 
-__global__ void incident_e_kernel (double *e_new, const double *e_old, const double *h_old, int len,
-                                   double modifier, const double *src, int src_index)
+__global__ void incident_e_kernel (IncidentJob j)
 {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x)
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < j.cells; i += gridDim.x * blockDim.x)
   {
     if (i == 0)
-      e_new[0] = src[src_index];
+      j.now[0] = *j.src;
     else
-      e_new[i] = e_old[i] + (h_old[i - 1] - h_old[i]) * modifier;
+      j.now[i] = j.old[i] + (j.other[i - 1] - j.other[i]) * j.modifier;
   }
 }
 
-__global__ void incident_h_kernel (double *h_new, const double *h_old, const double *e_new, int len,
-                                   double modifier)
+__global__ void incident_h_kernel (IncidentJob j)
 {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len - 1; i += gridDim.x * blockDim.x)
-    h_new[i] = h_old[i] + (e_new[i] - e_new[i + 1]) * modifier;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < j.cells; i += gridDim.x * blockDim.x)
+    j.now[i] = j.old[i] + (j.other[i] - j.other[i + 1]) * j.modifier;
 }
 
 __global__ void point_source_kernel (double *f, size_t index, const double *src, int src_index)
@@ -271,6 +272,314 @@ __global__ void __launch_bounds__ (256) plain_fast_kernel (const __grid_constant
   }
 }
 
+// ------------------------------------------------- 3-D half-step by columns
+
+// Incident value for the TF/SF slow path of plain_march_kernel (out of line:
+// only the columns and planes on the faces take it).
+__device__ __noinline__ double march_incident (const PlainHalf *p, int inc_len, int *err, int k, int x, int y, int z)
+{
+  return incident_value (p->g, p->inc, inc_len, err, k, x, y, z);
+}
+
+// E-from-D's two coefficients of a cell (out of line: the divisions are taken
+// only where the material or a coefficient changes).
+__device__ __noinline__ double2 march_coeffs (double plus, double minus, double modifier, double dd)
+{
+  const double p = (plus / modifier) / dd;
+  return make_double2 (p, minus == plus ? p : (minus / modifier) / dd);
+}
+
+constexpr int kMarchBlock = 128;
+constexpr int kMarchMax = 64;   // largest x chunk (per-plane TF/SF masks in shared memory)
+
+// One half-step (all three components) of the FP64 plain form, 3-D: a thread
+// owns one (y, z) column of a chunk of x planes and marches along x, the
+// arithmetic of plain_component in its order.
+//
+// What bounds it: at one component per thread and cell (plain_fast_kernel)
+// the half-step is bound by instructions, 410 per component and cell, most
+// of them the four IEEE divisions of E-from-D, the index arithmetic and the
+// reloads of the opposite family.  A column keeps all of that in registers:
+//  * the y and z coefficients are constants of the thread, the x ones
+//    uniform loads;
+//  * E-from-D's coefficients are recomputed only when the averaged material
+//    or an x coefficient changes from one plane to the next (two divisions,
+//    four where sigma along the component's own axis differs from 0), so
+//    uniform regions divide once per column;
+//  * the x neighbours are the previous plane's values.
+// Columns are numbered flat over y and z, so no lane idles on odd sizes; the
+// next plane's material and coefficients are worked out after the stores,
+// where few values are live (96 registers, 20 warps per SM).  What is left is
+// memory latency (3.9 TB/s of DRAM, 30 % issue active).
+// 203 x 181 x 165, PML 12, TF/SF: 370 -> 210 us per half-step (a step 735 ->
+// 429 us); a step at 80^3, PML 10: 82 -> 55 us.
+// IS_H: the family, which orders the two differences of a curl.  LO: the lower
+// cell of a difference (-1: E in E_CENTERED, H in H_CENTERED; 0 the other way
+// round).  MK: material points a component averages (0: uniform 1, 1:
+// per-component arrays of double material precision, 2 with LO = -1, 4 with
+// LO = 0).
+template <bool IS_H, int LO, bool PML, int MK>
+__global__ void __launch_bounds__ (kMarchBlock, 5)
+    plain_march_kernel (const __grid_constant__ PlainHalf p, const __grid_constant__ PlainTabs tb,
+                        const __grid_constant__ IncidentJob inc, int inc_blocks, int col_blocks, int chunk, int inc_len,
+                        int *err)
+{
+  if ((int) blockIdx.x < inc_blocks)
+  {
+    for (int i = blockIdx.x * kMarchBlock + threadIdx.x; i < inc.cells; i += inc_blocks * kMarchBlock)
+    {
+      if (p.is_h)
+        inc.now[i] = inc.old[i] + (inc.other[i] - inc.other[i + 1]) * inc.modifier;
+      else if (i == 0)
+        inc.now[0] = *inc.src;
+      else
+        inc.now[i] = inc.old[i] + (inc.other[i - 1] - inc.other[i]) * inc.modifier;
+    }
+    return;
+  }
+  const GeomDev &g = p.g;
+  const int b = (int) blockIdx.x - inc_blocks;
+  const int wz = g.n[2] - 2, cols = (g.n[1] - 2) * wz;
+  const int col = (b % col_blocks) * kMarchBlock + threadIdx.x;
+  const int xa = 1 + (b / col_blocks) * chunk, xe = min (xa + chunk, g.n[0] - 1);
+
+  // TF/SF terms (bit 4 ci + t) whose x range holds plane xa + i
+  __shared__ unsigned s_terms[kMarchMax];
+  if (p.use_tfsf)
+  {
+    for (int i = threadIdx.x; i < xe - xa; i += kMarchBlock)
+    {
+      unsigned m = 0;
+      for (int ci = 0; ci < 3; ++ci)
+        for (int t = 0; t < p.comp[ci].nterms; ++t)
+          if (xa + i >= p.comp[ci].term[t].lo[0] && xa + i < p.comp[ci].term[t].hi[0])
+            m |= 1u << (4 * ci + t);
+      s_terms[i] = m;
+    }
+    __syncthreads ();
+  }
+  if (col >= cols)
+    return;
+  const int y = 1 + col / wz, z = 1 + col % wz;
+  const int64_t sy = g.n[2], sx = (int64_t) g.n[1] * g.n[2];
+  int64_t id = xa * sx + y * sy + z;
+  unsigned terms = 0;   // terms whose y and z ranges hold the column
+  if (p.use_tfsf)
+    for (int ci = 0; ci < 3; ++ci)
+      for (int t = 0; t < p.comp[ci].nterms; ++t)
+      {
+        const TermDev &tm = p.comp[ci].term[t];
+        if (y >= tm.lo[1] && y < tm.hi[1] && z >= tm.lo[2] && z < tm.hi[2])
+          terms |= 1u << (4 * ci + t);
+      }
+
+  const double dt = g.dt, dx = g.dx, mm = p.mat_modifier;
+  // PML coefficients: component 0 has ca, cb along y, the denominator along
+  // z, the numerators along x; 1 and 2 are its rotations
+  // (the ones only march_coeffs takes are read there again)
+  double ca0 = 1, cb0 = 0, e0 = 1, ca1 = 1, cb1 = 0, e2 = 1;
+  if (PML)
+  {
+    ca0 = tb.t[0][0][y];
+    cb0 = tb.t[0][1][y];
+    e0 = tb.t[0][2][z];
+    ca1 = tb.t[1][0][z];
+    cb1 = tb.t[1][1][z];
+    e2 = tb.t[2][2][y];
+  }
+  // what the current E-from-D coefficients (without PML: cb) were made from
+  double m_of[3] = {-1, -1, -1}, np0 = 0, nm0 = 0, dd1 = 0;
+  double cp[3] = {0, 0, 0}, cm[3] = {0, 0, 0};
+  // x coefficients of the plane: component 2's ca, cb and component 1's ca2
+  double cax = 1, cbx = 0, e1 = 1;
+  auto coeffs = [&] (const double m[3], int x) __attribute__ ((always_inline)) {
+    if (PML)
+    {
+      cax = tb.t[2][0][x];
+      cbx = tb.t[2][1][x];
+      e1 = tb.t[1][2][x];
+      const double d = tb.t[1][3][x], a = tb.t[0][4][x], s = tb.t[0][5][x];
+      if (m[0] != m_of[0] || a != np0 || s != nm0)
+      {
+        m_of[0] = m[0];
+        np0 = a;
+        nm0 = s;
+        const double2 c = march_coeffs (a, s, m[0] * mm, tb.t[0][3][z]);
+        cp[0] = c.x;
+        cm[0] = c.y;
+      }
+      if (m[1] != m_of[1] || d != dd1)
+      {
+        m_of[1] = m[1];
+        dd1 = d;
+        const double2 c = march_coeffs (tb.t[1][4][y], tb.t[1][5][y], m[1] * mm, d);
+        cp[1] = c.x;
+        cm[1] = c.y;
+      }
+      if (m[2] != m_of[2])
+      {
+        m_of[2] = m[2];
+        const double2 c = march_coeffs (tb.t[2][4][z], tb.t[2][5][z], m[2] * mm, tb.t[2][3][y]);
+        cp[2] = c.x;
+        cm[2] = c.y;
+      }
+    }
+    else
+    {
+#pragma unroll
+      for (int ci = 0; ci < 3; ++ci)
+        if (m[ci] != m_of[ci])
+        {
+          m_of[ci] = m[ci];
+          cp[ci] = dt / (m[ci] * mm * dx);
+        }
+    }
+  };
+  // material points of the plane at `id`, and those of the plane after it at
+  // (0, 0), (y + 1), (z + 1) where the averages span x
+  double mc = 1, my = 1, mz = 1, myz = 1, mx = 1, mxy = 1, mxz = 1;
+  auto material = [&] (int64_t at) __attribute__ ((always_inline)) {
+    if (MK == 1)
+    {
+      mc = p.matc[0][at];
+      my = p.matc[1][at];
+      mz = p.matc[2][at];
+    }
+    else if (MK == 2)
+    {
+      my = p.mat[at + sy];
+      mz = p.mat[at + 1];
+      mx = p.mat[at + sx];
+    }
+    else if (MK == 4)
+    {
+      myz = p.mat[at + sy + 1];
+      mx = p.mat[at + sx];
+      mxy = p.mat[at + sx + sy];
+      mxz = p.mat[at + sx + 1];
+    }
+  };
+  // their averages, then the plane's centre moves on
+  auto averages = [&] (double m[3]) __attribute__ ((always_inline)) {
+    m[0] = m[1] = m[2] = 1;
+    if (MK == 1)
+    {
+      m[0] = mc;
+      m[1] = my;
+      m[2] = mz;
+    }
+    else if (MK == 2)
+    {
+      m[0] = (mc + mx) / 2.0;
+      m[1] = (mc + my) / 2.0;
+      m[2] = (mc + mz) / 2.0;
+      mc = mx;
+    }
+    else if (MK == 4)
+    {
+      m[0] = ((mc + mz) / 2.0 + (my + myz) / 2.0) / 2.0;
+      m[1] = ((mc + mz) / 2.0 + (mx + mxz) / 2.0) / 2.0;
+      m[2] = ((mc + my) / 2.0 + (mx + mxy) / 2.0) / 2.0;
+      mc = mx;
+      my = mxy;
+      mz = mxz;
+    }
+  };
+
+  const double *O0 = p.opp[0], *O1 = p.opp[1], *O2 = p.opp[2];
+  // carried along x: LO = -1 the previous plane's values (the x neighbours),
+  // LO = 0 the centre's (read a plane ahead as its x neighbours)
+  double c1 = O1[LO ? id - sx : id], c2 = O2[LO ? id - sx : id];
+  if (MK == 2 || MK == 4)
+    mc = p.mat[id];
+  if (MK == 4)
+  {
+    my = p.mat[id + sy];
+    mz = p.mat[id + 1];
+  }
+  {
+    double m[3];
+    material (id);
+    averages (m);
+    coeffs (m, xa);
+  }
+  for (int x = xa; x < xe; ++x, id += sx)
+  {
+    const int64_t oy = LO ? id - sy : id + sy, oz = LO ? id - 1 : id + 1;
+    const double o0 = O0[id];
+    const double n1 = O1[LO ? id : id + sx], n2 = O2[LO ? id : id + sx];
+    const double o2y = O2[oy], o1z = O1[oz], o0z = O0[oz], o0y = O0[oy];
+    double old[3], fld[3] = {0, 0, 0};
+#pragma unroll
+    for (int ci = 0; ci < 3; ++ci)
+    {
+      old[ci] = PML ? p.dd[ci][1][id] : p.f[ci][1][id];
+      if (PML)
+        fld[ci] = p.f[ci][1][id];
+    }
+    // (the next plane's material and coefficients follow the stores, where
+    // no field value is live; its loads are in flight with the fields')
+    if (x + 1 < xe)
+      material (id + sx);
+    // neighbours of the curls, v[ci] = {11, 12, 21, 22}: the difference of the
+    // family's component ci + 2 along ci + 1 and of ci + 1 along ci + 2, in
+    // this order for E, in the other for H
+    double v[3][4];
+    auto pair = [&] (int ci, int q, double near, double far) {
+      const int at = (q == 0) != IS_H ? 0 : 2;
+      v[ci][at] = LO ? far : near;
+      v[ci][at + 1] = LO ? near : far;
+    };
+    const double x1 = LO ? c1 : n1, x2 = LO ? c2 : n2, o1 = LO ? n1 : c1, o2 = LO ? n2 : c2;
+    pair (0, 0, o2, o2y);
+    pair (0, 1, o1, o1z);
+    pair (1, 0, o0, o0z);
+    pair (1, 1, o2, x2);
+    pair (2, 0, o1, x1);
+    pair (2, 1, o0, o0y);
+    c1 = n1;
+    c2 = n2;
+    if (p.use_tfsf)
+    {
+      const unsigned on = terms & s_terms[x - xa];
+      for (unsigned left = on; left; left &= left - 1)
+      {
+        const int bit = __ffs ((int) left) - 1, ci = bit >> 2;
+        const TermDev &tm = p.comp[ci].term[bit & 3];
+        double diff = march_incident (&p, inc_len, err, tm.inc_comp, x + tm.aux[0], y + tm.aux[1], z + tm.aux[2]);
+        if (tm.negate < 0)
+          diff *= -1.0;
+        const int at = 4 * ci + tm.slot;
+#pragma unroll
+        for (int q = 0; q < 12; ++q)
+          if (at == q)
+            v[q / 4][q % 4] -= diff;
+      }
+    }
+    const double ca[3] = {ca0, ca1, cax}, cb[3] = {PML ? cb0 : cp[0], PML ? cb1 : cp[1], PML ? cbx : cp[2]};
+    const double e[3] = {e0, e1, e2};
+#pragma unroll
+    for (int ci = 0; ci < 3; ++ci)
+    {
+      const double tmp = v[ci][1] - v[ci][0] - v[ci][3] + v[ci][2];
+      const double nv = old[ci] * ca[ci] + tmp * cb[ci];
+      if (PML)
+      {
+        p.dd[ci][0][id] = nv;
+        p.f[ci][0][id] = fld[ci] * e[ci] + nv * cp[ci] - old[ci] * cm[ci];
+      }
+      else
+        p.f[ci][0][id] = nv;
+    }
+    if (x + 1 < xe)
+    {
+      double m[3];
+      averages (m);
+      coeffs (m, x + 1);
+    }
+  }
+}
+
 int launch_plain_tables (const PlainHalf &p, double *const out[3][6], cudaStream_t s)
 {
   PlainTabOut o;
@@ -308,6 +617,50 @@ int launch_plain_fast (const PlainHalf &p, const PlainTabs &t, int inc_len, int 
   return 1;
 }
 
+int launch_plain_march (const PlainHalf &p, const PlainTabs &t, const IncidentJob &inc, bool mat_uniform, int inc_len,
+                        int *err, int sm_count, cudaStream_t s)
+{
+  const int cols = (p.g.n[1] - 2) * (p.g.n[2] - 2), planes = p.g.n[0] - 2;
+  const int col_blocks = (cols + kMarchBlock - 1) / kMarchBlock;
+  const int inc_blocks = inc.cells > 0 ? std::min (64, (inc.cells + kMarchBlock - 1) / kMarchBlock) : 0;
+  const int mk = mat_uniform ? 0 : (p.dmp ? 1 : p.comp[0].nmat);
+  using Kernel = void (*) (const PlainHalf, const PlainTabs, const IncidentJob, int, int, int, int, int *);
+#define FDTDB_MARCH(H, LO, PML)                                                                                        \
+  (mk == 0 ? plain_march_kernel<H, LO, PML, 0> : mk == 1 ? plain_march_kernel<H, LO, PML, 1>                           \
+                                                         : plain_march_kernel<H, LO, PML, (LO ? 2 : 4)>)
+  const bool low = p.comp[0].d11[1] < 0 || p.comp[0].d11[2] < 0;   // (E differs along y first, H along z)
+  Kernel kern = nullptr;
+  if (p.is_h)
+    kern = low ? (p.use_pml ? FDTDB_MARCH (true, -1, true) : FDTDB_MARCH (true, -1, false))
+               : (p.use_pml ? FDTDB_MARCH (true, 0, true) : FDTDB_MARCH (true, 0, false));
+  else
+    kern = low ? (p.use_pml ? FDTDB_MARCH (false, -1, true) : FDTDB_MARCH (false, -1, false))
+               : (p.use_pml ? FDTDB_MARCH (false, 0, true) : FDTDB_MARCH (false, 0, false));
+#undef FDTDB_MARCH
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, kern, kMarchBlock, 0) != cudaSuccess || per_sm < 1)
+    per_sm = 4;
+  // x chunk: the blocks run in waves of sm_count * per_sm, each as long as
+  // its planes and the start of a column (about three planes' time)
+  int chunk = 4;
+  double best = 1e300;
+  for (int c : {2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
+  {
+    const int m = (planes + c - 1) / c, even = (planes + m - 1) / m;
+    const double waves = std::max (1.0, (double) col_blocks * m / ((double) sm_count * per_sm));
+    const double cost = (waves < 8 ? std::ceil (waves) : waves + 0.5) * (even + 3);
+    if (cost < best * 0.999)
+    {
+      best = cost;
+      chunk = even;
+    }
+  }
+  const int chunks = (planes + chunk - 1) / chunk;
+  kern<<<(unsigned) (inc_blocks + col_blocks * chunks), kMarchBlock, 0, s>>> (p, t, inc, inc_blocks, col_blocks, chunk,
+                                                                              inc_len, err);
+  return 1;
+}
+
 int launch_plain_half (const PlainHalf &p, int inc_len, int *err, int sm_count, cudaStream_t s)
 {
   const int ix = (p.g.drop & 1) ? 1 : p.g.n[0] - 2;
@@ -334,19 +687,15 @@ int launch_plain_half (const PlainHalf &p, int inc_len, int *err, int sm_count, 
   return 1;
 }
 
-int launch_incident_e (double *e_new, const double *e_old, const double *h_old, int len, double modifier,
-                       const double *src, int src_index, cudaStream_t s)
+int launch_incident_e (const IncidentJob &j, cudaStream_t s)
 {
-  int blocks = (len + 255) / 256;
-  incident_e_kernel<<<blocks, 256, 0, s>>> (e_new, e_old, h_old, len, modifier, src, src_index);
+  incident_e_kernel<<<(j.cells + 255) / 256, 256, 0, s>>> (j);
   return 1;
 }
 
-int launch_incident_h (double *h_new, const double *h_old, const double *e_new, int len, double modifier,
-                       cudaStream_t s)
+int launch_incident_h (const IncidentJob &j, cudaStream_t s)
 {
-  int blocks = (len + 255) / 256;
-  incident_h_kernel<<<blocks, 256, 0, s>>> (h_new, h_old, e_new, len, modifier);
+  incident_h_kernel<<<(j.cells + 255) / 256, 256, 0, s>>> (j);
   return 1;
 }
 
