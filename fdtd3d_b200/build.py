@@ -9,6 +9,8 @@ Translation units and flags:
   csrc/fused3d.cu         nvcc                          3-D single-sweep E+H kernel (register-blocked)
   csrc/sweep3d.cu         nvcc                          3-D single-sweep E+H kernel (TMA-pipelined)
   csrc/sweep2.cu          nvcc                          3-D two-step (temporally blocked) sweep
+  csrc/tile2d_fp64.cu     nvcc --fmad=false            2-D modes, several steps per launch (FP64 plain form)
+  csrc/tile2d_fast.cu     nvcc                          the same, FP32 / FP16 storage
   csrc/fdtd_api.cu        nvcc                          C ABI, context, launch sequence
   csrc/cli.cpp            g++ -> fdtd3d-b200            command-line drop-in over the C ABI
 """
@@ -43,6 +45,8 @@ def _units():
     units = [
         ("setup.cpp", ["g++", "-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-I", CSRC]),
         ("plain_kernels.cu", [nvcc] + common + ["--fmad=false"]),
+        ("tile2d_fp64.cu", [nvcc] + common + ["--fmad=false"]),
+        ("tile2d_fast.cu", [nvcc] + common),
         ("fast_kernels.cu", [nvcc] + common),
         ("fdtd_api.cu", [nvcc] + common),
     ]

@@ -26,6 +26,7 @@
 #include "fused3d.h"
 #include "sweep2.h"
 #include "tfsf2.h"
+#include "tile2d.h"
 #include "sweep3d.h"
 #include "kernels.h"
 #include "ntff.h"
@@ -530,6 +531,12 @@ int upload_fine_material (fdtd_ctx *ctx, int which, const double *src, cudaMemcp
   return FDTD_OK;
 }
 
+// 2-D modes without metamaterials advance several steps per launch (tile2d).
+bool tile2d_mode (const Geometry &g)
+{
+  return (g.drop == 1 || g.drop == 2 || g.drop == 4) && !g.cfg.use_metamaterials;
+}
+
 int alloc_fast (fdtd_ctx *ctx)
 {
   const Geometry &g = ctx->g;
@@ -538,7 +545,8 @@ int alloc_fast (fdtd_ctx *ctx)
   // E_CENTERED stencil on cell-centred materials; H_CENTERED, double material
   // precision and the 2-D / 1-D modes run the per-cell kernels on one buffer set
   ctx->has_second = g.drop == 0 && g.cfg.layout == 0 && !g.dmp;
-  for (int b = 0; b < (ctx->has_second ? 2 : 1); ++b)
+  // (the 2-D modes' several-step launches write a second set as well)
+  for (int b = 0; b < (ctx->has_second || tile2d_mode (g) ? 2 : 1); ++b)
   {
     for (int k = 0; k < 6; ++k)
     {
@@ -1485,6 +1493,156 @@ IncidentJob incident_h_job (fdtd_ctx *ctx)
   return j;
 }
 
+// Whether this call's steps may take the 2-D several-step launches: nothing
+// reads the fields between the steps (DFT, kept levels), no J / M current,
+// and a point source on an updated cell.
+bool tile2d_ready (const fdtd_ctx *ctx)
+{
+  const Geometry &g = ctx->g;
+  if (!tile2d_mode (g) || ctx->cs_mask[0] || ctx->cs_mask[1] || ctx->dft_comp >= 0 || (ctx->kind && ctx->keep_prev))
+    return false;
+  if (g.cfg.point_source_mask)
+    for (int a = 0; a < 3; ++a)
+      if (!((g.drop >> a) & 1) && (g.cfg.point_source[a] < 1 || g.cfg.point_source[a] > g.n[a] - 2))
+        return false;
+  return true;
+}
+
+// Steps i .. i + steps - 1 of the call in one launch (t > 0).
+int tile2d_run (fdtd_ctx *ctx, uint32_t i, int steps)
+{
+  const Geometry &g = ctx->g;
+  const int ua = g.drop == 1 ? 1 : 0, va = g.drop == 4 ? 1 : 2;
+  const bool f64 = ctx->kind == 0;
+  Tile2D p;
+  std::memset (&p, 0, sizeof (p));
+  p.nu = g.n[ua];
+  p.nv = g.n[va];
+  p.use_pml = g.cfg.use_pml;
+  p.steps = steps;
+  p.mm[0] = kEps0;
+  p.mm[1] = kMu0;
+  p.dt = g.dt;
+  p.dx = g.dx;
+  p.scale[0] = 1.f;
+  p.scale[1] = (float) kEta0;
+  p.pu = g.cfg.point_source[ua];
+  p.pv = g.cfg.point_source[va];
+  p.src = ctx->d_src + kSrcStride * i;
+  p.err = ctx->d_err;
+  int slot[6], ns = 0;
+  for (int k = 0; k < 6; ++k)
+    slot[k] = g.comp[k].exists ? ns++ : -1;
+  const int to = 1 - ctx->fcur;
+  for (int k = 0; k < 6; ++k)
+  {
+    if (slot[k] < 0)
+      continue;
+    TileComp &c = p.comp[slot[k]];
+    const CompDev l = make_comp_dev (g, k);
+    const int h = k >= 3, base = h ? 0 : 3;
+    c.is_h = h;
+    c.opp[0] = slot[base + l.opp1];
+    c.opp[1] = slot[base + l.opp2];
+    const int *d[4] = {l.d11, l.d12, l.d21, l.d22};
+    for (int q = 0; q < 4; ++q)
+    {
+      c.d[q][0] = d[q][ua];
+      c.d[q][1] = d[q][va];
+      c.m[q][0] = l.m[q][ua];
+      c.m[q][1] = l.m[q][va];
+    }
+    c.nmat = l.nmat;
+    auto axis = [&] (int a) { return a == ua ? 0 : (a == va ? 1 : 2); };
+    c.ax1 = axis (l.sig_cacb);
+    c.ax5 = axis (l.sig5);
+    c.ax4 = axis (l.sig4);
+    if (f64)
+    {
+      c.in = ctx->f[k][1];
+      c.out = ctx->f[k][0];
+      c.aux_in = ctx->dd[k][1];
+      c.aux_out = ctx->dd[k][0];
+      c.mat = g.dmp ? ctx->matc64[k] : (ctx->mat_set[h] ? ctx->mat64[h] : nullptr);
+      for (int j = 0; j < 6; ++j)
+        c.tab[j] = ctx->ptab[k][j];
+    }
+    else
+    {
+      const FastHalf &fh = h ? ctx->fast_h : ctx->fast_e;
+      p.courant = fh.courant;
+      c.in = ctx->ffb[ctx->fcur][k];
+      c.out = ctx->ffb[to][k];
+      c.aux_in = ctx->auxb[ctx->fcur][k];
+      c.aux_out = ctx->auxb[to][k];
+      c.mat = ctx->matc32[k] ? ctx->matc32[k] : ctx->mat32[h];
+      for (int j = 0; j < 6; ++j)
+        c.tab[j] = fh.tab[k % 3][j];
+      c.ilo[0] = fh.ilo[k % 3][ua];
+      c.ihi[0] = fh.ihi[k % 3][ua];
+      c.ilo[1] = fh.ilo[k % 3][va];
+      c.ihi[1] = fh.ihi[k % 3][va];
+    }
+    c.source = (g.cfg.point_source_mask >> k) & 1;
+    c.nterms = l.nterms;
+    for (int t = 0; t < l.nterms; ++t)
+    {
+      c.term[t] = l.term[t];
+      c.term[t].lo[0] = l.term[t].lo[ua];
+      c.term[t].hi[0] = l.term[t].hi[ua];
+      c.term[t].aux[0] = l.term[t].aux[ua];
+      c.term[t].lo[1] = l.term[t].lo[va];
+      c.term[t].hi[1] = l.term[t].hi[va];
+      c.term[t].aux[1] = l.term[t].aux[va];
+    }
+    p.pos[k][0] = g.comp[k].min_fp[ua];
+    p.pos[k][1] = g.comp[k].min_fp[va];
+    p.proj[k] = g.proj[k];
+  }
+  p.use_tfsf = g.cfg.use_tfsf;
+  if (p.use_tfsf)
+  {
+    p.k[0] = g.inc_k[0];
+    p.k[1] = g.inc_k[1];
+    p.zero[0] = g.zero_inc[ua];
+    p.zero[1] = g.zero_inc[va];
+    p.mod_e = g.mod_e;
+    p.mod_h = g.mod_h;
+    p.inc_len = g.inc_len;
+    ctx->inc_steps += steps;
+    p.inc_cells = (int) std::min<int64_t> (g.inc_len, ctx->inc_steps + 1);
+    p.e_in = ctx->einc[ctx->ecur];
+    p.h_in = ctx->hinc[ctx->hcur];
+    ctx->ecur ^= 1;
+    ctx->hcur ^= 1;
+    p.e_out = ctx->einc[ctx->ecur];
+    p.h_out = ctx->hinc[ctx->hcur];
+  }
+  cudaEvent_t pe;
+  int r = prof_begin (ctx, &pe);
+  if (r != FDTD_OK)
+    return r;
+  if (f64)
+  {
+    ctx->launches += launch_tile2d_fp64 (p, ctx->sm_count, ctx->stream);
+    for (int k = 0; k < 6; ++k)
+      if (slot[k] >= 0)
+      {
+        rotate (ctx->f[k], g.levels);
+        rotate (ctx->dd[k], g.levels);
+      }
+    ctx->step_kernel = "plain_fp64";
+  }
+  else
+  {
+    ctx->launches += launch_tile2d_fast (p, ctx->kind == 2, ctx->sm_count, ctx->stream);
+    ctx->fcur = to;
+    select_fast_set (ctx);
+    ctx->step_kernel = "per_cell";
+  }
+  return prof_end (ctx, pe);
+}
+
 int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
 {
   const Geometry &g = ctx->g;
@@ -1532,9 +1690,22 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
     cfix.scale_h = 1.f;
   }
 
+  const bool tiles = tile2d_ready (ctx);
   for (uint32_t i = 0; i < n; ++i)
   {
     uint32_t t = t_start + i;
+    if (tiles && t > 0)
+    {
+      // an odd number of steps in FP64 (tile2d.cuh says why)
+      int steps = (int) std::min<uint32_t> (kTileSteps, n - i);
+      if (ctx->kind == 0 && steps % 2 == 0)
+        --steps;
+      if ((r = tile2d_run (ctx, i, steps)) != FDTD_OK)
+        return r;
+      ctx->prev_src = 0;
+      i += steps - 1;
+      continue;
+    }
     if (fused && t > 0)
     {
       // incident E then H steps, then one sweep for both field families

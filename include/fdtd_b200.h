@@ -269,8 +269,8 @@ int fdtd_keep_previous_level (fdtd_ctx *ctx, int on);
  * reference counterpart): "plain_fp64" (FP64 plain form), "sweep2_tma"
  * (two steps per pass: the last call ended on a pair), "sweep3d_tma"
  * (TMA-pipelined one-sweep 3-D kernel), "fused3d_regblock" (register-blocked
- * one-sweep 3-D kernel), "per_cell" (one launch per half-step), or
- * "not_stepped" before the first update.  Null for a null context. */
+ * one-sweep 3-D kernel), "per_cell" (the per-cell kernels, one launch per
+ * half-step, or in the 2-D modes up to seven steps), or "not_stepped" before the first update.  Null for a null context. */
 const char *fdtd_step_kernel (const fdtd_ctx *ctx);
 
 /* The cudaStream_t (as void *) every launch of this context goes to, so a

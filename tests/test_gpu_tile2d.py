@@ -1,0 +1,91 @@
+"""2-D modes: several steps per launch (tile2d) against one step per call.
+A call of one step from t > 0 is a launch of one step; calls of n steps take
+launches of up to seven.  FP64: bit for bit, and against the oracle in TMz;
+FP32: to rounding."""
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+MODES = {"tmz": 2, "tex": 4, "tey": 5, "tez": 6, "tmx": 7, "tmy": 8}
+# 3 x 3: one updated cell; 18 x 18: exactly one small tile; 19 x 51 and 51 x
+# 19: one cell past a tile of either kind; 420 x 380 and 330 x 700: large tiles
+SIZES = [(3, 3), (18, 18), (19, 51), (51, 19), (97, 133), (420, 380)]
+
+
+def _setup(fdtd, mode, size, source, seed, mu=False):
+    rng = np.random.default_rng(seed)
+    kw = dict(mode=mode, size=size, teta=40, phi=25, psi=20)
+    if min(size) > 16:
+        kw.update(use_pml=True, pml=4)
+    if source == "tfsf" and min(size) > 16:
+        kw.update(use_tfsf=True, tfsf_left=6, tfsf_right=6)
+    else:
+        kw.update(point_source=tuple(n // 2 for n in size), point_source_mask=0x3f)
+    blocks = rng.uniform(1, 4, tuple(n // 5 + 1 for n in size)).astype(np.float32).astype(np.float64)
+    mats = {"eps": np.kron(blocks, np.ones((5, 5)))[: size[0], : size[1]]}
+    if mu:
+        mats["mu"] = mats["eps"][::-1, ::-1] / 2 + 0.5
+    # noise with nonzero faces: FP64 alternates two levels of the faces
+    fields = {c: rng.standard_normal(size) / (1 if c[0] == "E" else 376.73) for c in fdtd.MODE_COMPONENTS[mode]}
+    return kw, mats, fields
+
+
+def _run(fdtd, kw, mats, fields, prec, calls):
+    with fdtd.Simulation(materials=mats, precision=prec, **kw) as sim:
+        sim.step(3)
+        for c, v in fields.items():
+            sim.set_field(c, v)
+        for n in calls:
+            sim.step(n)
+        return {c: sim.field(c) for c in fields}
+
+
+@pytest.mark.parametrize("mode", sorted(MODES))
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("source", ["tfsf", "point"])
+def test_fp64_launches_of_any_length_agree(fdtd, mode, size, source):
+    for layout in (0, 1):
+        kw, mats, fields = _setup(fdtd, MODES[mode], size, source, 7, mu=layout == 1)
+        kw["layout"] = layout
+        want = _run(fdtd, kw, mats, fields, 0, [1] * 24)
+        for calls in ([24], [7, 2, 15], [4, 6, 14]):
+            got = _run(fdtd, kw, mats, fields, 0, calls)
+            for c in want:
+                assert np.array_equal(got[c].view(np.int64), want[c].view(np.int64)), (layout, calls, c)
+
+
+@pytest.mark.parametrize("size", SIZES[1:])
+def test_fp64_tmz_matches_oracle(fdtd, size):
+    kw, mats, _ = _setup(fdtd, 2, size, "tfsf", 9)
+    o = Oracle(materials=mats, **kw)
+    o.step(40)
+    with fdtd.Simulation(materials=mats, **kw) as sim:
+        sim.step(40)
+        for c in ("Ez", "Hx", "Hy"):
+            got, want = sim.field(c), np.asarray(o.field(c)).reshape(size)
+            assert np.array_equal(got.view(np.int64), want.view(np.int64)), c
+        inc = sim.incident("E")
+        assert np.all(inc[41:] == 0) and np.any(inc[:41] != 0)
+    o.close()
+
+
+@pytest.mark.parametrize("mode", sorted(MODES))
+@pytest.mark.parametrize("size", SIZES[1:])
+@pytest.mark.parametrize("source", ["tfsf", "point"])
+@pytest.mark.parametrize("prec,tol", [(1, 1e-5), (2, 2e-2)])
+def test_fast_forms_match_fp64(fdtd, mode, size, source, prec, tol):
+    for layout in (0, 1):
+        kw, mats, fields = _setup(fdtd, MODES[mode], size, source, 3, mu=layout == 1)
+        kw["layout"] = layout
+        for v in fields.values():   # (FP64 alternates the faces' two levels, the fast forms keep one)
+            v[[0, -1], :] = 0
+            v[:, [0, -1]] = 0
+        want = _run(fdtd, kw, mats, fields, 0, [25])
+        got = _run(fdtd, kw, mats, fields, prec, [4, 21])
+        for fam in "EH":
+            g = np.concatenate([got[c].ravel() for c in got if c[0] == fam])
+            w = np.concatenate([want[c].ravel() for c in want if c[0] == fam])
+            assert np.linalg.norm(g - w) <= tol * np.linalg.norm(w), (layout, fam)
