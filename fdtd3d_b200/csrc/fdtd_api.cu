@@ -178,6 +178,9 @@ struct fdtd_ctx
   // metamaterials with the sweep: the box of the Drude cells, fixed up after
   // each sweep step (drude_fix), and its device scratch
   bool drude_fix = false;
+  // point source with the sweep: 0 inside it, 1 its response after single
+  // steps (PointFix), 2 after pairs too
+  int ps_fix = 0;
   DrudeBox drude_box{};
   int *drude_box_dev = nullptr;
 
@@ -1002,6 +1005,8 @@ int plan_sweep (fdtd_ctx *ctx)
 {
   const Geometry &g = ctx->g;
   ctx->sweep_state = -1;
+  ctx->ps_fix = 0;
+  ctx->fused.ps_mask = g.cfg.point_source_mask;
   if (const char *v = std::getenv ("FDTDB_SWEEP"))
     if (std::atoi (v) == 0)
     {
@@ -1064,6 +1069,29 @@ int plan_sweep (fdtd_ctx *ctx)
     }
   }
   ctx->fused.tfsf_post = ctx->band.cells > 0 ? 1 : 0;   // read only by the sweep kernels
+  // A point source as its linear response after the step (one half-step's
+  // reach: the cell and the one below it outside the PML) or after a pair
+  // (three cells below to two above).  FDTDB_POINT_FIX=0 keeps it inside the
+  // sweep (a test hook).
+  if (g.cfg.point_source_mask && !g.cfg.use_metamaterials)
+  {
+    auto free_of_pml = [&] (int below, int above) {
+      bool in = true;
+      for (int a = 0; a < 3; ++a)
+      {
+        const int c = g.cfg.point_source[a];
+        in = in && c - below >= 0 && c + above <= g.n[a] - 1;
+        for (int k = 0; k < 6 && g.cfg.use_pml; ++k)
+          in = in && c - below >= ctx->fused.ilo[k][a] && c + above < ctx->fused.ihi[k][a];
+      }
+      return in;
+    };
+    const char *v = std::getenv ("FDTDB_POINT_FIX");
+    if ((!v || std::atoi (v) != 0) && free_of_pml (1, 0))
+      ctx->ps_fix = !g.cfg.use_tfsf && free_of_pml (3, 2) ? 2 : 1;
+    if (ctx->ps_fix)
+      ctx->fused.ps_mask = 0;
+  }
   // a first plan gives the CTA count the chunk choice depends on
   std::string why = sweep3d_plan (ctx->sweep, ctx->fused, e, h, aux, ctx->mat32[0], ctx->sm_count, wy, 32,
                                   ctx->sweep_ctr, lean);
@@ -1132,6 +1160,11 @@ int plan_sweep (fdtd_ctx *ctx)
   {
     ctx->sweep_state = 1;
     ctx->sweep_eps = ctx->mat32[0];
+  }
+  else
+  {
+    ctx->ps_fix = 0;
+    ctx->fused.ps_mask = g.cfg.point_source_mask;
   }
   // the two-step sweep for pairs of steps (FDTDB_TB2=0 keeps single steps:
   // a test hook)
@@ -1679,6 +1712,11 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
       for (int a = 0; a < 3; ++a)
         cs_fix = cs_fix && ctx->cs_pos[a] - 1 >= ctx->fused.ilo[k][a] && ctx->cs_pos[a] + 1 < ctx->fused.ihi[k][a];
   const bool fused = ctx->kind != 0 && ctx->has_second && !ctx->mat32[1] && ctx->ps_interior && (!has_cs || cs_fix);
+  PointFix pfix{};
+  for (int a = 0; a < 3; ++a)
+    pfix.pos[a] = g.cfg.point_source[a];
+  pfix.mask = g.cfg.point_source_mask;
+  pfix.scale_h = (float) kEta0;
   CurrentFix cfix{};
   if (has_cs)
   {
@@ -1736,7 +1774,8 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
       if (ctx->sweep_state == 0 || (ctx->sweep_state == 1 && ctx->sweep_eps != ctx->mat32[0]))
         if ((r = plan_sweep (ctx)) != FDTD_OK)
           return r;
-      const bool pair = ctx->tb2_state >= 1 && i + (ctx->keep_prev ? 2 : 1) < n && ctx->dft_comp < 0 && !has_cs;
+      const bool pair = ctx->tb2_state >= 1 && i + (ctx->keep_prev ? 2 : 1) < n && ctx->dft_comp < 0 && !has_cs &&
+                        (!g.cfg.point_source_mask || ctx->ps_fix == 2);
       // On the two-step path with a PML shell only the pair's TF/SF kernel
       // reads the incident grid: its steps run on a stream of their own
       // beside the shell and the core, after every earlier reader (all on s
@@ -1815,6 +1854,8 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
         }
         if (g.cfg.use_tfsf && ctx->tb2_state == 1)
           ctx->launches += launch_tfsf2 (ctx->tf2, f, inc_h1, inc_e1, inc_h2, inc_e2, ctx->d_err, s);
+        if (ctx->ps_fix)
+          ctx->launches += launch_point_fix (f, pfix, ctx->d_src + kSrcStride * i + 1, kSrcStride, true, s);
         ctx->step_kernel = "sweep2_tma";
         if ((r = prof_end (ctx, pe)) != FDTD_OK)
           return r;
@@ -1842,6 +1883,8 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
       }
       if (has_cs)
         ctx->launches += launch_current_fix (f, cfix, ctx->d_src + kSrcStride * i + 3, s);
+      if (ctx->ps_fix)
+        ctx->launches += launch_point_fix (f, pfix, ctx->d_src + kSrcStride * i + 1, kSrcStride, false, s);
       if ((r = prof_end (ctx, pe)) != FDTD_OK)
         return r;
       ctx->fcur = nw;

@@ -792,6 +792,146 @@ int launch_current_fix (const FusedParams &p, const CurrentFix &cf, const double
   return 1;
 }
 
+namespace {
+
+template <typename T>
+__device__ __forceinline__ void add_to (T *f, size_t id, float d);
+template <>
+__device__ __forceinline__ void add_to<float> (float *f, size_t id, float d)
+{
+  f[id] += d;
+}
+template <>
+__device__ __forceinline__ void add_to<__half> (__half *f, size_t id, float d)
+{
+  f[id] = __float2half_rn (__half2float (f[id]) + d);
+}
+
+// Response of a point source, one thread per cell of the 5^3 box around it
+// (the change travels one cell per half-step: E at the source; H there and
+// one cell below; E one cell around; H two below and one above).  In the
+// sweep a source cost its items the general class, 116 of 165 us of a
+// 256 x 224 x 240 step with one CTA at work, and kept the run from pairs;
+// this kernel takes about 4 us a step or pair.
+// Single step: dE = src - E_new, H_new += S curl dE.  Pair: the first step's
+// E at the source is worked out again from the old set, then
+//   dE1 = src1 - E1, dH1 = S curl dE1 (a driven H: src1 - H1),
+//   dE2 = dE1 + S im curl dH1 (at the source src2 - E_new), dH2 likewise.
+template <typename T, bool PAIR>
+__global__ void __launch_bounds__ (128) point_fix_kernel (const __grid_constant__ FusedParams p, PointFix pf,
+                                                          const double *src, int stride)
+{
+  constexpr int W = 5, N = W * W * W, C = (2 * W + 2) * W + 2;   // the source's index
+  __shared__ float dE[3][N], dH[3][N];
+  const int q = threadIdx.x;
+  const int ny = p.g.n[1], pz = p.g.pz;
+  const size_t st[3] = {(size_t) ny * pz, (size_t) pz, 1};
+  const int sd[3] = {W * W, W, 1};
+  const size_t c = (size_t) pf.pos[0] * st[0] + (size_t) pf.pos[1] * st[1] + pf.pos[2];
+  const float S = p.courant;
+  const int l[3] = {q / (W * W), (q / W) % W, q % W};
+  bool upd = q < N, low = false, high = false;   // low / high: on the box's first / last cells
+  for (int a = 0; a < 3; ++a)
+  {
+    const int g = pf.pos[a] + l[a] - 2;
+    upd = upd && g >= 1 && g <= p.g.n[a] - 2;
+    low = low || l[a] == 0;
+    high = high || l[a] == W - 1;
+  }
+  const size_t id = c + (size_t) ((l[0] - 2) * (long long) st[0] + (l[1] - 2) * (long long) st[1] + (l[2] - 2));
+  auto im = [&] (int k, size_t i) { return p.eps ? __fdividef (2.f, p.eps[i] + p.eps[i + st[k]]) : 1.f; };
+  // E component k after the first step, from the old set
+  auto e1 = [&] (int k, size_t i) -> float {
+    const int b = (k + 1) % 3, d = (k + 2) % 3;
+    const T *hb = (const T *) p.h_old[b], *hd = (const T *) p.h_old[d];
+    const float cu = (ldf (hd, i) - ldf (hd, i - st[b])) - (ldf (hb, i) - ldf (hb, i - st[d]));
+    return ldf ((const T *) p.e_old[k], i) + (S * im (k, i)) * cu;
+  };
+  // curl of dE around cell q (its upper neighbours), of dH (its lower ones)
+  auto curl_e = [&] (int m) {
+    const int b = (m + 1) % 3, d = (m + 2) % 3;
+    return (dE[b][q + sd[d]] - dE[b][q]) - (dE[d][q + sd[b]] - dE[d][q]);
+  };
+  auto curl_h = [&] (int k) {
+    const int b = (k + 1) % 3, d = (k + 2) % 3;
+    return (dH[d][q] - dH[d][q - sd[b]]) - (dH[b][q] - dH[b][q - sd[d]]);
+  };
+  if (q < N)
+    for (int k = 0; k < 3; ++k)
+    {
+      dE[k][q] = 0.f;
+      dH[k][q] = 0.f;
+    }
+  __syncthreads ();
+  if (q < 3 && ((pf.mask >> q) & 1))
+    dE[q][C] = (float) src[0] - (PAIR ? e1 (q, c) : ld_new ((const T *) p.e_new[q], c));
+  __syncthreads ();
+  if (upd && !high)
+    for (int m = 0; m < 3; ++m)
+    {
+      float d = S * curl_e (m);
+      if (PAIR && q == C && ((pf.mask >> (3 + m)) & 1))
+      {
+        const int b = (m + 1) % 3, e = (m + 2) % 3;
+        const float cu = (e1 (b, c + st[e]) - e1 (b, c)) - (e1 (e, c + st[b]) - e1 (e, c));
+        d = (float) src[1] * pf.scale_h - (ldf ((const T *) p.h_old[m], c) + S * cu);
+      }
+      dH[m][q] = d;
+    }
+  __syncthreads ();
+  if (PAIR)
+  {
+    float d[3] = {0.f, 0.f, 0.f};
+    if (upd && !low)
+      for (int k = 0; k < 3; ++k)
+      {
+        d[k] = dE[k][q] + (S * im (k, id)) * curl_h (k);
+        if (q == C && ((pf.mask >> k) & 1))
+          d[k] = (float) src[stride] - ld_new ((const T *) p.e_new[k], c);
+      }
+    if (q < N)
+      for (int k = 0; k < 3; ++k)
+        dE[k][q] = d[k];
+    __syncthreads ();
+    if (upd && !high)
+      for (int m = 0; m < 3; ++m)
+        dH[m][q] += S * curl_e (m);
+  }
+  if (!upd)
+    return;
+  const double *last = src + (PAIR ? stride : 0);
+  for (int k = 0; k < 3; ++k)
+  {
+    if (q == C && ((pf.mask >> k) & 1))
+      stf ((T *) p.e_new[k], c, (float) last[0]);
+    else if (dE[k][q] != 0.f)
+      add_to ((T *) p.e_new[k], id, dE[k][q]);
+    if (q == C && ((pf.mask >> (3 + k)) & 1))
+      stf ((T *) p.h_new[k], c, (float) last[1] * pf.scale_h);
+    else if (dH[k][q] != 0.f)
+      add_to ((T *) p.h_new[k], id, dH[k][q]);
+  }
+}
+
+}  // namespace
+
+int launch_point_fix (const FusedParams &p, const PointFix &pf, const double *src, int stride, bool pair,
+                      cudaStream_t s)
+{
+  if (p.fp16)
+  {
+    if (pair)
+      point_fix_kernel<__half, true><<<1, 128, 0, s>>> (p, pf, src, stride);
+    else
+      point_fix_kernel<__half, false><<<1, 128, 0, s>>> (p, pf, src, stride);
+  }
+  else if (pair)
+    point_fix_kernel<float, true><<<1, 128, 0, s>>> (p, pf, src, stride);
+  else
+    point_fix_kernel<float, false><<<1, 128, 0, s>>> (p, pf, src, stride);
+  return 1;
+}
+
 int launch_drude_flags (unsigned char *flags, const float *ome, const float *gae, const float *omm, const float *gam,
                         int nx, int ny, int nz, int pz, cudaStream_t s)
 {

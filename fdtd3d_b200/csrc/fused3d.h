@@ -91,6 +91,21 @@ struct CurrentFix
 };
 int launch_current_fix (const FusedParams &p, const CurrentFix &cf, const double *src, cudaStream_t s);
 
+// Hard point source of a one-sweep step (or of a pair of steps): the sweep
+// updates every cell without it, and the fields take the linear response of
+// the change the source makes at its cell (launch_point_fix in fused3d.cu).
+// Used when the cells the response reaches are outside the PML, not Drude
+// cells, and for a pair outside the TF/SF band.
+struct PointFix
+{
+  int pos[3];
+  int mask;                    // bit k: component k (Ex .. Hz) is driven
+  float scale_h;               // source value -> stored H (eta0)
+};
+// src: the (first) step's source table row; stride: doubles to the next row
+int launch_point_fix (const FusedParams &p, const PointFix &pf, const double *src, int stride, bool pair,
+                      cudaStream_t s);
+
 // Recomputes the per-cell Drude bitmask from the four material arrays.
 int launch_drude_flags (unsigned char *flags, const float *ome, const float *gae, const float *omm, const float *gam,
                         int nx, int ny, int nz, int pz, cudaStream_t s);
