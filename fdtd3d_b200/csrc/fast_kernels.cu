@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "cell_walk.cuh"
 #include "kernels.h"
@@ -359,74 +360,119 @@ __global__ void __launch_bounds__ (256) convert_rows_kernel (D *dst, const S *sr
       put (dst, r * dpitch + z, get (src, r * spitch + z) * scale);
 }
 
-// Neumaier (compensated) accumulation in FP64
-__device__ __forceinline__ void neumaier (double &s, double &c, double v)
+// Compensated FP64 accumulation: (s, c) += v with the rounding error of the
+// sum kept in c (Knuth's two-sum: no branch on the magnitudes).
+__device__ __forceinline__ void two_sum (double &s, double &c, double v)
 {
-  double t = s + v;
-  if (fabs (s) >= fabs (v))
-    c += (s - t) + v;
-  else
-    c += (v - t) + s;
+  const double t = s + v, z = t - s;
+  c += (s - (t - z)) + (v - z);
   s = t;
 }
 
-template <typename T>
-__device__ __forceinline__ double ldd (const void *p, size_t i)
+// The (s, c) pairs of a warp's lanes added up in lane 0.
+__device__ __forceinline__ void warp_sum (double &s, double &c)
 {
-  return (double) ld ((const T *) p, i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+  {
+    const double os = __shfl_down_sync (0xffffffffu, s, o), oc = __shfl_down_sync (0xffffffffu, c, o);
+    two_sum (s, c, os);
+    c += oc;
+  }
+}
+
+// Block `part` of `parts` (256 threads each) of sum w v^2 scale over n values
+// into partials[2 part], [2 part + 1].  Bound by the FP64 pipe (about ten
+// instructions per value): two accumulators per thread hide their latency,
+// and the block's pairs meet in a shuffle tree (a loop over 256 pairs in one
+// thread, and one over the blocks in reduce_final, took more time than the
+// sum: 55 MB 57 + 63 us before).
+template <typename T>
+__device__ __forceinline__ void reduce_block (const T *src, size_t n, const void *weight, int wkind, double scale,
+                                              int part, int parts, double *partials)
+{
+  double s0 = 0.0, c0 = 0.0, s1 = 0.0, c1 = 0.0;
+  auto term = [&] (size_t i) {
+    const double v = get (src, i);
+    const double w = wkind == 1 ? (double) ((const float *) weight)[i] : (wkind == 2 ? ((const double *) weight)[i] : 1.0);
+    return w * v * v * scale;
+  };
+  const size_t step = (size_t) parts * 256;
+  size_t i = (size_t) part * 256 + threadIdx.x;
+  for (; i + step < n; i += 2 * step)
+  {
+    const double a = term (i), b = term (i + step);
+    two_sum (s0, c0, a);
+    two_sum (s1, c1, b);
+  }
+  if (i < n)
+    two_sum (s0, c0, term (i));
+  two_sum (s0, c0, s1);
+  c0 += c1;
+  warp_sum (s0, c0);
+  __shared__ double sh[2][8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0)
+  {
+    sh[0][w] = s0;
+    sh[1][w] = c0;
+  }
+  __syncthreads ();
+  if (w == 0)
+  {
+    s0 = lane < 8 ? sh[0][lane] : 0.0;
+    c0 = lane < 8 ? sh[1][lane] : 0.0;
+    warp_sum (s0, c0);
+    if (lane == 0)
+    {
+      partials[2 * part] = s0;
+      partials[2 * part + 1] = c0;
+    }
+  }
+}
+
+// One warp: the blocks' pairs into one value.
+__device__ __forceinline__ void reduce_parts (const double *partials, int parts, double *out)
+{
+  double s = 0.0, c = 0.0;
+  for (int i = threadIdx.x; i < parts; i += 32)
+  {
+    two_sum (s, c, partials[2 * i]);
+    c += partials[2 * i + 1];
+  }
+  warp_sum (s, c);
+  if (threadIdx.x == 0)
+    *out = s + c;
 }
 
 template <int KIND>
 __global__ void __launch_bounds__ (256) reduce_sq_kernel (const void *src, size_t n, const void *weight,
                                                           int wkind, double scale, double *partials)
 {
-  double s = 0.0, c = 0.0;
-  for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x)
-  {
-    double v;
-    if (KIND == 0)
-      v = ((const double *) src)[i];
-    else if (KIND == 1)
-      v = ldd<float> (src, i);
-    else
-      v = ldd<__half> (src, i);
-    double w = 1.0;
-    if (wkind == 1)
-      w = (double) ((const float *) weight)[i];
-    else if (wkind == 2)
-      w = ((const double *) weight)[i];
-    neumaier (s, c, w * v * v * scale);
-  }
-  __shared__ double ss[256];
-  __shared__ double sc[256];
-  ss[threadIdx.x] = s;
-  sc[threadIdx.x] = c;
-  __syncthreads ();
-  if (threadIdx.x == 0)
-  {
-    double bs = 0.0, bc = 0.0;
-    for (int i = 0; i < blockDim.x; ++i)
-    {
-      neumaier (bs, bc, ss[i]);
-      bc += sc[i];
-    }
-    partials[2 * blockIdx.x] = bs;
-    partials[2 * blockIdx.x + 1] = bc;
-  }
+  using T = typename std::conditional<KIND == 0, double, typename std::conditional<KIND == 1, float, __half>::type>::type;
+  reduce_block ((const T *) src, n, weight, wkind, scale, blockIdx.x, gridDim.x, partials);
 }
 
 __global__ void reduce_final_kernel (const double *partials, int nblocks, double *out)
 {
-  if (threadIdx.x == 0 && blockIdx.x == 0)
-  {
-    double s = 0.0, c = 0.0;
-    for (int i = 0; i < nblocks; ++i)
-    {
-      neumaier (s, c, partials[2 * i]);
-      c += partials[2 * i + 1];
-    }
-    out[0] = s + c;
-  }
+  reduce_parts (partials, nblocks, out);
+}
+
+// every component in one launch: block row y takes item y
+template <int KIND>
+__global__ void __launch_bounds__ (256) reduce_items_kernel (const __grid_constant__ ReduceItems it, size_t n,
+                                                             double *partials)
+{
+  using T = typename std::conditional<KIND == 0, double, typename std::conditional<KIND == 1, float, __half>::type>::type;
+  const int q = blockIdx.y;
+  reduce_block ((const T *) it.src[q], n, it.weight[q], it.wkind[q], it.scale[q], blockIdx.x, gridDim.x,
+                partials + (size_t) 2 * gridDim.x * q);
+}
+
+__global__ void reduce_items_final_kernel (const __grid_constant__ ReduceItems it, const double *partials, int nblocks,
+                                           double *out)
+{
+  reduce_parts (partials + (size_t) 2 * nblocks * blockIdx.x, nblocks, out + it.out[blockIdx.x]);
 }
 
 int grid_for (size_t n, int sm_count)
@@ -528,16 +574,20 @@ int launch_convert_out (double *dst, const void *src, int src_kind, size_t rows,
   return launch_convert (dst, (const __half *) src, rows, nz, nz, pz, scale, s);
 }
 
-int launch_reduce_sq (const void *src, int kind, size_t n, const void *weight, int wkind, double scale,
-                      double *partials, int nblocks, cudaStream_t s)
+int launch_reduce_items (const ReduceItems &it, int kind, size_t n, double *partials, int nblocks, double *out,
+                         cudaStream_t s)
 {
+  if (it.count == 0)
+    return 0;
+  const dim3 grid (nblocks, it.count);
   if (kind == 0)
-    reduce_sq_kernel<0><<<nblocks, 256, 0, s>>> (src, n, weight, wkind, scale, partials);
+    reduce_items_kernel<0><<<grid, 256, 0, s>>> (it, n, partials);
   else if (kind == 1)
-    reduce_sq_kernel<1><<<nblocks, 256, 0, s>>> (src, n, weight, wkind, scale, partials);
+    reduce_items_kernel<1><<<grid, 256, 0, s>>> (it, n, partials);
   else
-    reduce_sq_kernel<2><<<nblocks, 256, 0, s>>> (src, n, weight, wkind, scale, partials);
-  return 1;
+    reduce_items_kernel<2><<<grid, 256, 0, s>>> (it, n, partials);
+  reduce_items_final_kernel<<<it.count, 32, 0, s>>> (it, partials, nblocks, out);
+  return 2;
 }
 
 __global__ void fill_kernel (double *dst, size_t n, double value)
@@ -552,14 +602,8 @@ int launch_fill (double *dst, size_t n, double value, cudaStream_t s)
   return 1;
 }
 
-int launch_reduce_final (const double *partials, int nblocks, double *out, cudaStream_t s)
-{
-  reduce_final_kernel<<<1, 32, 0, s>>> (partials, nblocks, out);
-  return 1;
-}
-
-// The same two launches through cudaLaunchKernel, so that each returns its
-// own launch status and an earlier, unrelated error pending on the calling
+// The allocation-free sum's two launches through cudaLaunchKernel, so that
+// each returns its own launch status and an earlier, unrelated error pending on the calling
 // thread is neither reported nor cleared.
 cudaError_t launch_reduce_sq_checked (const void *src, int kind, size_t n, const void *weight, int wkind,
                                       double scale, double *partials, int nblocks, cudaStream_t s)

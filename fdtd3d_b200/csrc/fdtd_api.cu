@@ -1278,7 +1278,7 @@ int create_impl (const fdtd_config *cfg, int device, fdtd_ctx *ctx)
     }
   }
   ctx->nparts = ctx->sm_count * 4;
-  DALLOC (ctx->partials, (size_t) ctx->nparts * 2 * sizeof (double));
+  DALLOC (ctx->partials, (size_t) ctx->nparts * 6 * 2 * sizeof (double));
   DALLOC (ctx->d_out, 16 * sizeof (double));
   int r = ctx->kind == 0 ? alloc_plain (ctx) : alloc_fast (ctx);
   if (r != FDTD_OK)
@@ -2346,40 +2346,40 @@ int fdtd_reduce (fdtd_ctx *ctx, int what, double *out)
   if (r != FDTD_OK)
     return r;
   const size_t n = ctx->scells;   // (padding cells hold zeros)
+  ReduceItems it;
+  std::memset (&it, 0, sizeof (it));
+  CK (cudaMemsetAsync (ctx->d_out, 0, 6 * sizeof (double), ctx->stream));
   for (int k = 0; k < 6; ++k)
   {
     if (!ctx->g.comp[k].exists)
-    {
-      CK (cudaMemsetAsync (ctx->d_out + k, 0, sizeof (double), ctx->stream));
       continue;
-    }
-    const void *src = ctx->kind == 0 ? (const void *) ctx->f[k][1] : (const void *) ctx->ff[k];
-    const void *w = nullptr;
-    int wkind = 0;
-    double scale = 1.0;
-    bool isH = k >= 3;
+    const bool isH = k >= 3;
+    const int q = it.count++;
+    it.out[q] = k;
+    it.src[q] = ctx->kind == 0 ? (const void *) ctx->f[k][1] : (const void *) ctx->ff[k];
+    it.scale[q] = 1.0;
     if (what == FDTD_REDUCE_ENERGY)
     {
       // (double material precision: the component's own averaged material)
       if (ctx->kind == 0)
       {
-        w = ctx->matc64[k] ? ctx->matc64[k] : ctx->mat64[isH ? 1 : 0];
-        wkind = 2;
-        scale = isH ? kEta0 * kEta0 : 1.0;
+        it.weight[q] = ctx->matc64[k] ? ctx->matc64[k] : ctx->mat64[isH ? 1 : 0];
+        it.wkind[q] = 2;
+        it.scale[q] = isH ? kEta0 * kEta0 : 1.0;
       }
       else
       {
-        w = ctx->matc32[k] ? ctx->matc32[k] : ctx->mat32[isH ? 1 : 0];
-        wkind = w ? 1 : 0;
+        it.weight[q] = ctx->matc32[k] ? ctx->matc32[k] : ctx->mat32[isH ? 1 : 0];
+        it.wkind[q] = it.weight[q] ? 1 : 0;
       }
     }
     else if (ctx->kind != 0 && isH)
     {
-      scale = 1.0 / (kEta0 * kEta0);
+      it.scale[q] = 1.0 / (kEta0 * kEta0);
     }
-    ctx->launches += launch_reduce_sq (src, ctx->kind, n, w, wkind, scale, ctx->partials, ctx->nparts, ctx->stream);
-    ctx->launches += launch_reduce_final (ctx->partials, ctx->nparts, ctx->d_out + k, ctx->stream);
   }
+  ctx->launches += launch_reduce_items (it, ctx->kind, n, ctx->partials, ctx->nparts, ctx->d_out, ctx->stream);
+  CK (cudaGetLastError ());
   double vals[6];
   CK (cudaMemcpyAsync (vals, ctx->d_out, 6 * sizeof (double), cudaMemcpyDeviceToHost, ctx->stream));
   CK (cudaStreamSynchronize (ctx->stream));

@@ -118,15 +118,23 @@ int launch_find_nonfinite (const double *src, size_t n, unsigned long long *firs
 
 // compensated FP64 reductions: out[0..parts) partial pairs (sum, compensation)
 // weight kinds: 0 = none, 1 = float, 2 = double
-int launch_reduce_sq (const void *src, int kind, size_t n, const void *weight, int wkind, double scale,
-                      double *partials, int nblocks, cudaStream_t s);
+struct ReduceItems
+{
+  int count;
+  const void *src[6], *weight[6];
+  int wkind[6], out[6];        // out: the item's place in the result
+  double scale[6];
+};
+// sum of weight v^2 scale over n values of each item (partials: 2 nblocks
+// values per item)
+int launch_reduce_items (const ReduceItems &it, int kind, size_t n, double *partials, int nblocks, double *out,
+                         cudaStream_t s);
 int launch_fill (double *dst, size_t n, double value, cudaStream_t s);
 // one step of the running DFT of a stored field (kind 0 double, 1 float,
 // 2 half) on the plane x_axis = index; phase: (cos, sin) per frequency;
 // acc: (re, re comp., im, im comp.) per frequency and plane cell
 int launch_dft (const void *src, int kind, int axis, int index, const int n[3], int pz, double scale,
                 const double *phase, int nf, double *acc, int sm_count, cudaStream_t s);
-int launch_reduce_final (const double *partials, int nblocks, double *out, cudaStream_t s);
 // the two reduction launches with their own launch status (cudaLaunchKernel)
 cudaError_t launch_reduce_sq_checked (const void *src, int kind, size_t n, const void *weight, int wkind,
                                       double scale, double *partials, int nblocks, cudaStream_t s);
