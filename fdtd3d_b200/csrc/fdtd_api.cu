@@ -1549,6 +1549,9 @@ int tile2d_run (fdtd_ctx *ctx, uint32_t i, int steps)
   const bool f64 = ctx->kind == 0;
   Tile2D p;
   std::memset (&p, 0, sizeof (p));
+  p.form.te = g.comp[ua].exists;
+  p.form.flip = g.drop == 2;
+  p.form.hc = g.cfg.layout == 1;
   p.nu = g.n[ua];
   p.nv = g.n[va];
   p.use_pml = g.cfg.use_pml;
@@ -1573,23 +1576,13 @@ int tile2d_run (fdtd_ctx *ctx, uint32_t i, int steps)
       continue;
     TileComp &c = p.comp[slot[k]];
     const CompDev l = make_comp_dev (g, k);
-    const int h = k >= 3, base = h ? 0 : 3;
-    c.is_h = h;
-    c.opp[0] = slot[base + l.opp1];
-    c.opp[1] = slot[base + l.opp2];
-    const int *d[4] = {l.d11, l.d12, l.d21, l.d22};
+    const int h = k >= 3;
     for (int q = 0; q < 4; ++q)
     {
-      c.d[q][0] = d[q][ua];
-      c.d[q][1] = d[q][va];
       c.m[q][0] = l.m[q][ua];
       c.m[q][1] = l.m[q][va];
     }
     c.nmat = l.nmat;
-    auto axis = [&] (int a) { return a == ua ? 0 : (a == va ? 1 : 2); };
-    c.ax1 = axis (l.sig_cacb);
-    c.ax5 = axis (l.sig5);
-    c.ax4 = axis (l.sig4);
     if (f64)
     {
       c.in = ctx->f[k][1];

@@ -81,6 +81,36 @@ __device__ __forceinline__ double tile_incident (const Tile2D &p, const double *
   return (win[q] * pr1 + win[q + 1] * pr2) * p.proj[k];
 }
 
+// Compile-time structure of a mode (FORM = te + 2 flip + 4 hc).  Axes: 0 u,
+// 1 v, 2 the dropped one (w).  Component a of E has the curl differences
+// H_{a+2} along a + 1 and H_{a+1} along a + 2, of H E_{a+1} along a + 2 and
+// E_{a+2} along a + 1 (a + 1, a + 2: cyclic); PML pairs: curl step along
+// a + 1, field along a + 2, auxiliary along a.
+template <int FORM>
+struct Mode2D
+{
+  static constexpr bool TE = FORM & 1, FLIP = FORM & 2, HC = FORM & 4;
+  static constexpr int axis (int j) { return TE ? (j < 2 ? j : 2) : (j == 0 ? 2 : j - 1); }
+  static constexpr bool is_h (int j) { return TE ? j == 2 : j > 0; }
+  static constexpr int next (int a) { return (a + (FLIP ? 2 : 1)) % 3; }
+  // slot of the component of a family along axis a, -1: not in the mode
+  static constexpr int slot (bool h, int a) { return TE ? (h ? (a == 2 ? 2 : -1) : (a < 2 ? a : -1)) : (h ? (a < 2 ? 1 + a : -1) : (a == 2 ? 0 : -1)); }
+  static constexpr int opp (int j, int q)
+  {
+    const int n = next (axis (j)), m = next (n);
+    return slot (!is_h (j), is_h (j) == (q == 0) ? n : m);
+  }
+  static constexpr int along (int j, int q)
+  {
+    const int n = next (axis (j)), m = next (n);
+    return is_h (j) == (q == 0) ? m : n;
+  }
+  static constexpr int low (int j) { return is_h (j) == HC ? -1 : 0; }
+  static constexpr int ax1 (int j) { return next (axis (j)); }
+  static constexpr int ax5 (int j) { return next (next (axis (j))); }
+  static constexpr int ax4 (int j) { return axis (j); }
+};
+
 // Shared memory of a tile, in values of the arithmetic type: the fields with a
 // border of one cell, per-cell coefficients (FP64: E-from-D's two, or without
 // PML the curl's; FP32: S / m) and the 1-D PML tables along the tile.
@@ -95,12 +125,13 @@ struct TileMem
 
 // T: stored field type, C: arithmetic (double or float).  A thread holds the
 // CU x CV cells (w + 16 j, lane + 32 i) of the 16 CU x 32 CV tile.
-template <typename T, typename C, int CU, int CV>
+template <typename T, typename C, int CU, int CV, int FORM>
 __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_kernel (const __grid_constant__ Tile2D p, int tiles_v,
                                                                int ntiles)
 {
   constexpr bool F64 = sizeof (C) == 8;
   using L = TileMem<C, CU, CV>;
+  using M = Mode2D<FORM>;
   constexpr int TU = L::TU, TV = L::TV, TM = L::TM, R = CU * CV, P = L::P, A = L::A, N = L::N;
   constexpr int OU = TU - 2 * kTileSteps, OV = TV - 2 * kTileSteps;
   extern __shared__ __align__ (16) unsigned char tile_smem[];
@@ -140,9 +171,9 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
   if (p.use_pml)
     for (int q = lane + 32 * w; q < 3 * 6 * TM; q += kTileThreads)
     {
-      const TileComp &c = p.comp[q / (6 * TM)];
-      const int t = (q / TM) % 6, i = q % TM;
-      const int ax = t < 2 ? c.ax1 : (t < 4 ? c.ax5 : c.ax4);
+      const int j = q / (6 * TM), t = (q / TM) % 6, i = q % TM;
+      const TileComp &c = p.comp[j];
+      const int ax = t < 2 ? M::ax1 (j) : (t < 4 ? M::ax5 (j) : M::ax4 (j));
       const int g = ax == 0 ? u0 + i : (ax == 1 ? v0 + i : 0), n = ax == 0 ? p.nu : (ax == 1 ? p.nv : 1);
       Tab[q] = g >= 0 && g < n ? ((const C *) c.tab[t])[g] : C (1);
     }
@@ -150,7 +181,7 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
   // ---- this thread's cells: field and PML auxiliary.  (FP64 face cells keep
   // the other level's field in the auxiliary's place, which they do not have.)
   C f[3][R], x[3][R];
-  unsigned upd = 0, face = 0, in_pml[3] = {0, 0, 0}, terms[R];
+  unsigned upd = 0, face = 0, source = 0, in_pml[3] = {0, 0, 0}, terms[R];
   bool any_term = false;
 #pragma unroll
   for (int r = 0; r < R; ++r)
@@ -162,6 +193,7 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
     const int64_t id = (int64_t) u * p.nv + v;
     upd |= up ? 1u << r : 0u;
     face |= valid && !up ? 1u << r : 0u;
+    source |= up && u == p.pu && v == p.pv ? 1u << r : 0u;
     terms[r] = 0;
 #pragma unroll
     for (int j = 0; j < 3; ++j)
@@ -188,12 +220,13 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
       const int at = j * N + du * TV + dv;
       if constexpr (F64)
       {
-        const double mm = p.mm[c.is_h];
+        const double mm = p.mm[M::is_h (j)];
         if (p.use_pml)
         {
           x[j][r] = ((const C *) c.aux_in)[id];
           const C *const *tab = (const C *const *) c.tab;
-          const int q5 = c.ax5 == 0 ? u : (c.ax5 == 1 ? v : 0), q4 = c.ax4 == 0 ? u : (c.ax4 == 1 ? v : 0);
+          const int q5 = M::ax5 (j) == 0 ? u : (M::ax5 (j) == 1 ? v : 0);
+          const int q4 = M::ax4 (j) == 0 ? u : (M::ax4 (j) == 1 ? v : 0);
           const double modifier = m * mm, dd = tab[3][q5], plus = tab[4][q4], minus = tab[5][q4];
           const double cp = (plus / modifier) / dd;
           K[at] = cp;
@@ -259,11 +292,12 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
       for (int j = 0; j < 3; ++j)
       {
         const TileComp &c = p.comp[j];
-        if (c.is_h != fam)
+        if (M::is_h (j) != (fam == 1))
           continue;
-        const int n11 = c.d[0][0] * P + c.d[0][1], n12 = c.d[1][0] * P + c.d[1][1];
-        const int n21 = c.d[2][0] * P + c.d[2][1], n22 = c.d[3][0] * P + c.d[3][1];
-        const C *const S1 = F + (c.opp[0] >= 0 ? c.opp[0] : 0) * A, *const S2 = F + (c.opp[1] >= 0 ? c.opp[1] : 0) * A;
+        constexpr int kStep[3] = {P, 1, 0};
+        const int s1 = M::opp (j, 0), s2 = M::opp (j, 1);
+        const int n11 = M::low (j) * kStep[M::along (j, 0)], n12 = n11 + kStep[M::along (j, 0)];
+        const int n21 = M::low (j) * kStep[M::along (j, 1)], n22 = n21 + kStep[M::along (j, 1)];
 #pragma unroll
         for (int r = 0; r < R; ++r)
         {
@@ -271,15 +305,15 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
           if ((upd >> r) & 1u)
           {
             C a = C (0), b = C (0), d = C (0), e = C (0);
-            if (c.opp[0] >= 0)
+            if (s1 >= 0)
             {
-              a = S1[at + n11];
-              b = S1[at + n12];
+              a = F[s1 * A + at + n11];
+              b = F[s1 * A + at + n12];
             }
-            if (c.opp[1] >= 0)
+            if (s2 >= 0)
             {
-              d = S2[at + n21];
-              e = S2[at + n22];
+              d = F[s2 * A + at + n21];
+              e = F[s2 * A + at + n22];
             }
             if (unsigned on = (terms[r] >> (4 * j)) & 15u)
             {
@@ -298,7 +332,8 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
             }
             const int du = w + kTileWarps * (r / CV), dv = lane + 32 * (r % CV);
             const C *const t = Tab + 6 * j * TM;
-            const int q1 = c.ax1 == 0 ? du : (c.ax1 == 1 ? dv : 0), q5 = c.ax5 == 0 ? du : (c.ax5 == 1 ? dv : 0);
+            const int q1 = M::ax1 (j) == 0 ? du : (M::ax1 (j) == 1 ? dv : 0);
+            const int q5 = M::ax5 (j) == 0 ? du : (M::ax5 (j) == 1 ? dv : 0);
             const C kc = K[j * N + du * TV + dv];
             if constexpr (F64)
             {
@@ -317,7 +352,7 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
               const C curl = (b - a) - (e - d);
               if ((in_pml[j] >> r) & 1u)
               {
-                const int q4 = c.ax4 == 0 ? du : (c.ax4 == 1 ? dv : 0);
+                const int q4 = M::ax4 (j) == 0 ? du : (M::ax4 (j) == 1 ? dv : 0);
                 const C nx = t[q1] * x[j][r] + t[TM + q1] * curl;
                 f[j][r] = t[2 * TM + q5] * f[j][r]
                           + (t[4 * TM + q4] * nx - t[5 * TM + q4] * x[j][r]) * t[3 * TM + q5] * kc;
@@ -326,7 +361,7 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
               else
                 f[j][r] += kc * curl;
             }
-            if (c.source && u0 + du == p.pu && v0 + dv == p.pv)
+            if (((source >> r) & 1u) && c.source)
               f[j][r] = F64 ? C (p.src[kSrcRow * s + 1 + fam]) : C ((float) p.src[kSrcRow * s + 1 + fam] * p.scale[fam]);
           }
           else if (F64 && ((face >> r) & 1u))
@@ -359,18 +394,34 @@ __global__ void __launch_bounds__ (kTileThreads, CU * CV > 2 ? 1 : 2) tile2d_ker
   }
 }
 
-template <typename T, typename C, int CU, int CV>
-int tile2d_launch (const Tile2D &p, cudaStream_t s)
+template <typename T, typename C, int CU, int CV, int FORM>
+int tile2d_start (const Tile2D &p, cudaStream_t s)
 {
   constexpr int OU = kTileWarps * CU - 2 * kTileSteps, OV = 32 * CV - 2 * kTileSteps;
   constexpr int smem = TileMem<C, CU, CV>::BYTES;
   const int tu = (p.nu + OU - 1) / OU, tv = (p.nv + OV - 1) / OV;
   const int inc = p.use_tfsf ? (p.inc_cells + kIncOwn - 1) / kIncOwn : 0;
-  auto kern = tile2d_kernel<T, C, CU, CV>;
+  auto kern = tile2d_kernel<T, C, CU, CV, FORM>;
   if (smem > 48 * 1024)
     cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   kern<<<tu * tv + inc, dim3 (32, kTileWarps), smem, s>>> (p, tv, tu * tv);
   return 1;
+}
+
+template <typename T, typename C, int CU, int CV>
+int tile2d_launch (const Tile2D &p, cudaStream_t s)
+{
+  switch ((p.form.te ? 1 : 0) + (p.form.flip ? 2 : 0) + (p.form.hc ? 4 : 0))
+  {
+    case 0: return tile2d_start<T, C, CU, CV, 0> (p, s);
+    case 1: return tile2d_start<T, C, CU, CV, 1> (p, s);
+    case 2: return tile2d_start<T, C, CU, CV, 2> (p, s);
+    case 3: return tile2d_start<T, C, CU, CV, 3> (p, s);
+    case 4: return tile2d_start<T, C, CU, CV, 4> (p, s);
+    case 5: return tile2d_start<T, C, CU, CV, 5> (p, s);
+    case 6: return tile2d_start<T, C, CU, CV, 6> (p, s);
+    default: return tile2d_start<T, C, CU, CV, 7> (p, s);
+  }
 }
 
 // Tiles of a launch for a tile of CU x CV cells per thread.

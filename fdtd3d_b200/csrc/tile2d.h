@@ -15,27 +15,32 @@ constexpr int kTileSteps = 7;   // steps per launch at most: the halo of a tile
 // contiguous); a cell's index is u nv + v.
 struct TileComp
 {
-  int is_h;
-  int opp[2];                  // slot of the component each curl difference reads (-1: absent)
-  int d[4][2];                 // (u, v) offsets of the neighbours 11, 12, 21, 22
   int nmat, m[4][2];           // material stencil
   const void *mat;             // double (FP64) or float; null: 1
   const void *in, *aux_in;     // current level: field and PML auxiliary (null without PML)
   void *out, *aux_out;         // level after the steps
   const void *tab[6];          // PML tables: PlainTabs (FP64) or FastHalf order
-  int ax1, ax5, ax4;           // axis of the curl-step, field and auxiliary pair: 0 u, 1 v, 2 dropped
   int ilo[2], ihi[2];          // FP32: sigma = 0 range
   int source;                  // a point source drives it
   int nterms;
   TermDev term[kMaxTerms];     // lo, hi, aux of the axes u, v in [0], [1]
 };
 
+// Shape of a 2-D mode: te: two E components in the plane and one H across it
+// (else one E across, two H in the plane); flip: the kept axes and the
+// dropped one in the cyclic order u, w, v (y dropped); hc: H_CENTERED.
+struct TileForm
+{
+  bool te, flip, hc;
+};
+
 struct Tile2D
 {
+  TileForm form;
   int nu, nv;
   int use_pml;
   int steps;                   // 1 .. kTileSteps, odd in FP64
-  TileComp comp[3];            // E components, then H
+  TileComp comp[3];            // E components (u, then v), then H
   double mm[2];                // FP64: eps0, mu0
   double dt, dx;
   float courant;               // FP32
