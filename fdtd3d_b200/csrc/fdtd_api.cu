@@ -178,6 +178,7 @@ struct fdtd_ctx
   // metamaterials with the sweep: the box of the Drude cells, fixed up after
   // each sweep step (drude_fix), and its device scratch
   bool drude_fix = false;
+  bool drude_levels = true;     // xpp / zpp hold the levels two steps back (false after sweep steps)
   // point source with the sweep: 0 inside it, 1 its response after single
   // steps (PointFix), 2 after pairs too
   int ps_fix = 0;
@@ -1120,8 +1121,9 @@ int plan_sweep (fdtd_ctx *ctx)
       DrudeBox b;
       for (int a = 0; a < 3; ++a)
       {
-        b.lo[a] = hb[a];
-        b.hi[a] = hb[3 + a] + 1;
+        // (face cells are never updated, Drude or not)
+        b.lo[a] = std::max (hb[a], 1);
+        b.hi[a] = std::min (hb[3 + a] + 1, g.n[a] - 1);
       }
       int ext_lo[3];
       for (int a = 0; a < 3; ++a)
@@ -1151,7 +1153,7 @@ int plan_sweep (fdtd_ctx *ctx)
       if (why.empty ())
       {
         ctx->drude_box = b;
-        ctx->drude_fix = true;
+        ctx->drude_fix = b.lo[0] < b.hi[0] && b.lo[1] < b.hi[1] && b.lo[2] < b.hi[2];
       }
     }
   }
@@ -1864,13 +1866,29 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
       {
         ctx->launches += launch_sweep3d (ctx->sweep, o, f, ctx->d_err, s, ctx->sweep_streams);
         if (ctx->drude_fix)
+        {
           ctx->launches += launch_drude_fixup (f, ctx->drude_box, s);
+          ctx->drude_levels = false;
+        }
         if (f.tfsf_post)
           ctx->launches += launch_tfsf_post (ctx->band, f, ctx->d_err, s);
         ctx->step_kernel = "sweep3d_tma";
       }
       else
       {
+        if (g.cfg.use_metamaterials && !ctx->drude_levels)
+        {
+          // after sweep steps the levels two steps back are in the set the
+          // step is about to write
+          for (int k = 0; k < 6; ++k)
+          {
+            CK (cudaMemcpyAsync (ctx->xppb[o][k], ctx->auxb[nw][k], ctx->scells * sizeof (float),
+                                 cudaMemcpyDeviceToDevice, s));
+            CK (cudaMemcpyAsync (ctx->zppb[o][k], ctx->zb[nw][k], ctx->scells * sizeof (float),
+                                 cudaMemcpyDeviceToDevice, s));
+          }
+          ctx->drude_levels = true;
+        }
         ctx->launches += launch_fused3d (f, ctx->d_err, s);
         ctx->step_kernel = "fused3d_regblock";
       }

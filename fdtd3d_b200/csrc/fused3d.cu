@@ -599,50 +599,6 @@ __global__ void drude_box_kernel (const unsigned char *flags, int nx, int ny, in
   }
 }
 
-// Drude fix-up after a TMA sweep step, which updates every cell with the
-// plain (or PML) rule.  E pass: the Drude components of the cells of the box
-// are recomputed from the old buffers with update_drude (curl of H_old, the
-// sweep's operation order).  H pass, after it, over the box moved out by one
-// cell on the low sides (every H cell whose curl reads an E value of the
-// box): H_new recomputed from H_old and the corrected E_new with the rule of
-// the cell (Drude, PML or plain).  The box holds no point source, no PML
-// cell and no TF/SF band cell (the host checks), so no other rule applies.
-template <typename T>
-__global__ void __launch_bounds__ (256) drude_fix_e_kernel (const __grid_constant__ FusedParams p, DrudeBox b)
-{
-  const int ny = p.g.n[1], pz = p.g.pz;
-  const size_t sx = (size_t) ny * pz;
-  const int ez = b.hi[2] - b.lo[2], ey = b.hi[1] - b.lo[1];
-  const long long total = (long long) (b.hi[0] - b.lo[0]) * ey * ez;
-  const T *Ho0 = (const T *) p.h_old[0], *Ho1 = (const T *) p.h_old[1], *Ho2 = (const T *) p.h_old[2];
-  for (long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long) gridDim.x * blockDim.x)
-  {
-    const int z = b.lo[2] + (int) (t % ez);
-    const int y = b.lo[1] + (int) ((t / ez) % ey);
-    const int x = b.lo[0] + (int) (t / ((long long) ez * ey));
-    const size_t id = (size_t) x * sx + (size_t) y * pz + z;
-    const unsigned fl = p.dflag[id];
-    if (!(fl & 7u))
-      continue;
-    if (fl & 1u)
-    {
-      const float c = (ldf (Ho2, id) - ldf (Ho2, id - pz)) - (ldf (Ho1, id) - ldf (Ho1, id - 1));
-      stf ((T *) p.e_new[0], id, update_drude (p, 0, ldf ((const T *) p.e_old[0], id), c, x, y, z, id, true));
-    }
-    if (fl & 2u)
-    {
-      const float c = (ldf (Ho0, id) - ldf (Ho0, id - 1)) - (ldf (Ho2, id) - ldf (Ho2, id - sx));
-      stf ((T *) p.e_new[1], id, update_drude (p, 1, ldf ((const T *) p.e_old[1], id), c, x, y, z, id, true));
-    }
-    if (fl & 4u)
-    {
-      const float c = (ldf (Ho1, id) - ldf (Ho1, id - sx)) - (ldf (Ho0, id) - ldf (Ho0, id - pz));
-      stf ((T *) p.e_new[2], id, update_drude (p, 2, ldf ((const T *) p.e_old[2], id), c, x, y, z, id, true));
-    }
-  }
-}
-
 // E_new values the H pass reads were written by the E pass (or the sweep)
 // before this launch, so plain loads (not the read-only path) are used.
 template <typename T>
@@ -658,39 +614,258 @@ __device__ __forceinline__ float ld_new<__half> (const __half *p, size_t i)
   return __half2float (p[i]);
 }
 
-template <typename T>
-__global__ void __launch_bounds__ (256) drude_fix_h_kernel (const __grid_constant__ FusedParams p, DrudeBox b)
+// Four consecutive z cells (a 16-byte unit of floats, 8 bytes of halves).
+__device__ __forceinline__ void ld4v (const float *p, float v[4])
 {
-  const int ny = p.g.n[1], pz = p.g.pz;
-  const size_t sx = (size_t) ny * pz;
-  const int ez = b.hi[2] - b.lo[2], ey = b.hi[1] - b.lo[1];
-  const long long total = (long long) (b.hi[0] - b.lo[0]) * ey * ez;
-  const T *E0 = (const T *) p.e_new[0], *E1 = (const T *) p.e_new[1], *E2 = (const T *) p.e_new[2];
-  for (long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long) gridDim.x * blockDim.x)
+  const float4 t = *reinterpret_cast<const float4 *> (p);
+  v[0] = t.x;
+  v[1] = t.y;
+  v[2] = t.z;
+  v[3] = t.w;
+}
+__device__ __forceinline__ void ld4v (const __half *p, float v[4])
+{
+  const uint2 t = *reinterpret_cast<const uint2 *> (p);
+  const float2 a = __half22float2 (*reinterpret_cast<const __half2 *> (&t.x));
+  const float2 b = __half22float2 (*reinterpret_cast<const __half2 *> (&t.y));
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = b.x;
+  v[3] = b.y;
+}
+// Stores the cells of mask m.
+__device__ __forceinline__ void st4v (float *p, const float v[4], unsigned m)
+{
+  if (m == 15u)
+    *reinterpret_cast<float4 *> (p) = make_float4 (v[0], v[1], v[2], v[3]);
+  else
   {
-    const int z = b.lo[2] + (int) (t % ez);
-    const int y = b.lo[1] + (int) ((t / ez) % ey);
-    const int x = b.lo[0] + (int) (t / ((long long) ez * ey));
-    const size_t id = (size_t) x * sx + (size_t) y * pz + z;
-    const unsigned fl = p.dflag[id];
-    const float ex = ld_new (E0, id), ey_ = ld_new (E1, id), ez_ = ld_new (E2, id);
-    const float a = (ld_new (E1, id + 1) - ey_) - (ld_new (E2, id + pz) - ez_);
-    const float bb = (ld_new (E2, id + sx) - ez_) - (ld_new (E0, id + 1) - ex);
-    const float c = (ld_new (E0, id + pz) - ex) - (ld_new (E1, id + sx) - ey_);
-    auto inside = [&] (int k) {
-      return x >= p.ilo[k][0] && x < p.ihi[k][0] && y >= p.ilo[k][1] && y < p.ihi[k][1] && z >= p.ilo[k][2] &&
-             z < p.ihi[k][2];
-    };
-    const float h0 = update_any<3, true> (p, fl, inside (3), ldf ((const T *) p.h_old[0], id), a, 1.f, x, y, z, id,
-                                          true);
-    const float h1 = update_any<4, true> (p, fl, inside (4), ldf ((const T *) p.h_old[1], id), bb, 1.f, x, y, z, id,
-                                          true);
-    const float h2 = update_any<5, true> (p, fl, inside (5), ldf ((const T *) p.h_old[2], id), c, 1.f, x, y, z, id,
-                                          true);
-    stf ((T *) p.h_new[0], id, h0);
-    stf ((T *) p.h_new[1], id, h1);
-    stf ((T *) p.h_new[2], id, h2);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if ((m >> j) & 1u)
+        p[j] = v[j];
+  }
+}
+__device__ __forceinline__ void st4v (__half *p, const float v[4], unsigned m)
+{
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if ((m >> j) & 1u)
+      p[j] = __float2half_rn (v[j]);
+}
+
+// The thread's four cells of the box (z rounded down to the vector): false
+// past its end.  own: bit j for cells inside the box.
+__device__ __forceinline__ bool drude_cells (const DrudeBox &b, int &x, int &y, int &z, unsigned &own)
+{
+  const unsigned z0 = (unsigned) b.lo[2] & ~3u, nz4 = ((unsigned) b.hi[2] - z0 + 3u) / 4u;
+  const unsigned ny = (unsigned) (b.hi[1] - b.lo[1]);
+  const unsigned long long t = (unsigned long long) blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned r = (unsigned) (t / nz4);
+  z = (int) (z0 + 4u * (unsigned) (t - (unsigned long long) r * nz4));
+  y = b.lo[1] + (int) (r % ny);
+  x = b.lo[0] + (int) (r / ny);
+  own = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    own |= z + j >= b.lo[2] && z + j < b.hi[2] ? 1u << j : 0u;
+  return x < b.hi[0];
+}
+
+// Drude update of component k on the cells of mask m among four (no PML here,
+// so the curl step is X + S curl and F takes Z_new - Z; see update_drude for
+// the recurrence).  X and Z two steps back are what the new set still holds
+// from the step before last (every step alternates the sets), so no array of
+// previous levels is read or written.  w, g, em: averaged plasma frequency,
+// collision rate and eps.
+__device__ __forceinline__ void drude_four (const FusedParams &p, int k, size_t id, unsigned m, const float w[4],
+                                            const float g[4], const float em[4], const float curl[4], float f[4])
+{
+  float xo[4], xp[4], zo[4], zp[4];
+  ld4v (p.aux_old[k] + id, xo);
+  ld4v (p.aux_new[k] + id, xp);
+  ld4v (p.z_old[k] + id, zo);
+  ld4v (p.z_new[k] + id, zp);
+  const float dt = p.dt, S = p.courant;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+  {
+    const float sq = (dt * w[j]) * (dt * w[j]);
+    const float inv = 1.f / (4.f * em[j] + 2.f * dt * em[j] * g[j] + sq);
+    const float b0 = (4.f + 2.f * dt * g[j]) * inv, b1 = -8.f * inv, b2 = (4.f - 2.f * dt * g[j]) * inv;
+    const float a1 = (2.f * sq - 8.f * em[j]) * inv, a2 = (4.f * em[j] - 2.f * dt * em[j] * g[j] + sq) * inv;
+    const float xn = xo[j] + S * curl[j];
+    const float zn = b0 * xn + b1 * xo[j] + b2 * xp[j] - a1 * zo[j] - a2 * zp[j];
+    if ((m >> j) & 1u)
+      f[j] = f[j] + (zn - zo[j]);
+    xp[j] = xn;
+    zp[j] = zn;
+  }
+  st4v (p.aux_new[k] + id, xp, m);
+  st4v (p.z_new[k] + id, zp, m);
+}
+
+// Drude fix-up after a TMA sweep step, which updates every cell with the
+// plain (or PML) rule.  E pass: the Drude components of the cells of the box
+// are recomputed from the old buffers (curl of H_old, the sweep's operation
+// order).  H pass, after it, over the box moved out by one cell on the low
+// sides (every H cell whose curl reads an E value of the box): H_new
+// recomputed from H_old and the corrected E_new with the rule of the cell
+// (Drude or plain).  The box holds no point source, no PML cell and no TF/SF
+// band cell (the host checks), so no other rule applies.
+// Both passes are bound by memory latency and bytes (about 130 per cell):
+// one cell per thread kept 50 % of the DRAM bandwidth busy, so a thread takes
+// four z cells in 16-byte accesses, and the copies of the levels two steps
+// back are gone.  384^3 with a slab of 7.05 M cells, 20 steps with their
+// read-out: 31.5 -> 27.6 ms.
+template <typename T>
+__global__ void __launch_bounds__ (128) drude_fix_e_kernel (const __grid_constant__ FusedParams p, DrudeBox b)
+{
+  int x, y, z;
+  unsigned own;
+  if (!drude_cells (b, x, y, z, own))
+    return;
+  const size_t pz = p.g.pz, sx = (size_t) p.g.n[1] * pz;
+  const size_t id = (size_t) x * sx + (size_t) y * pz + z;
+  const unsigned fl = *reinterpret_cast<const unsigned *> (p.dflag + id);
+  unsigned on[3] = {0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      on[k] |= ((fl >> (8 * j + k)) & 1u) << j;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    on[k] &= own;
+  if (!(on[0] | on[1] | on[2]))
+    return;
+  const T *H0 = (const T *) p.h_old[0], *H1 = (const T *) p.h_old[1], *H2 = (const T *) p.h_old[2];
+  float h[3][4], n[4], q[4];
+  ld4v (H0 + id, h[0]);
+  ld4v (H1 + id, h[1]);
+  ld4v (H2 + id, h[2]);
+  float om[4], ga[4], ep[4] = {1.f, 1.f, 1.f, 1.f};
+  ld4v (p.omega[0] + id, om);
+  ld4v (p.gamma[0] + id, ga);
+  if (p.eps)
+    ld4v (p.eps + id, ep);
+  // the two-point averages along z take the cell after the four
+  const float omz = p.omega[0][id + 4], gaz = p.gamma[0][id + 4], epz = p.eps ? p.eps[id + 4] : 1.f;
+  const float h0z = ldf (H0, id - 1), h1z = ldf (H1, id - 1);
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+  {
+    float w[4], g[4], em[4], cu[4], f[4];
+    const size_t st = k == 0 ? sx : pz;
+    if (k < 2)
+    {
+      ld4v (p.omega[0] + id + st, w);
+      ld4v (p.gamma[0] + id + st, g);
+      if (p.eps)
+        ld4v (p.eps + id + st, em);
+      // k = 0: Hz at y - 1; k = 1: Hz at x - 1
+      ld4v (H2 + id - (k == 0 ? pz : sx), n);
+    }
+    else
+    {
+      ld4v (H1 + id - sx, n);
+      ld4v (H0 + id - pz, q);
+    }
+    ld4v ((const T *) p.e_old[k] + id, f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      w[j] = 0.5f * (om[j] + (k < 2 ? w[j] : (j < 3 ? om[j + 1 < 4 ? j + 1 : 3] : omz)));
+      g[j] = 0.5f * (ga[j] + (k < 2 ? g[j] : (j < 3 ? ga[j + 1 < 4 ? j + 1 : 3] : gaz)));
+      em[j] = p.eps ? 0.5f * (ep[j] + (k < 2 ? em[j] : (j < 3 ? ep[j + 1 < 4 ? j + 1 : 3] : epz))) : 1.f;
+      const float h1m = j ? h[1][j ? j - 1 : 0] : h1z, h0m = j ? h[0][j ? j - 1 : 0] : h0z;
+      cu[j] = k == 0   ? (h[2][j] - n[j]) - (h[1][j] - h1m)
+              : k == 1 ? (h[0][j] - h0m) - (h[2][j] - n[j])
+                       : (h[1][j] - n[j]) - (h[0][j] - q[j]);
+    }
+    if (on[k])
+    {
+      drude_four (p, k, id, on[k], w, g, em, cu, f);
+      st4v ((T *) p.e_new[k] + id, f, on[k]);
+    }
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__ (128) drude_fix_h_kernel (const __grid_constant__ FusedParams p, DrudeBox b)
+{
+  int x, y, z;
+  unsigned own;
+  if (!drude_cells (b, x, y, z, own))
+    return;
+  const size_t pz = p.g.pz, sx = (size_t) p.g.n[1] * pz;
+  const size_t id = (size_t) x * sx + (size_t) y * pz + z;
+  const unsigned fl = *reinterpret_cast<const unsigned *> (p.dflag + id);
+  unsigned on[3] = {0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+  {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      on[k] |= ((fl >> (8 * j + 3 + k)) & 1u) << j;
+    on[k] &= own;
+  }
+  const T *E0 = (const T *) p.e_new[0], *E1 = (const T *) p.e_new[1], *E2 = (const T *) p.e_new[2];
+  float e[3][4], e2y[4], e2x[4], e0y[4], e1x[4];
+  ld4v (E0 + id, e[0]);
+  ld4v (E1 + id, e[1]);
+  ld4v (E2 + id, e[2]);
+  ld4v (E2 + id + pz, e2y);
+  ld4v (E2 + id + sx, e2x);
+  ld4v (E0 + id + pz, e0y);
+  ld4v (E1 + id + sx, e1x);
+  // (the cell after the four: inside the row or its padding, or the next row
+  // when the box ends on the grid's last updated cell, where it is not used)
+  const float e0z = ld_new (E0, id + 4), e1z = ld_new (E1, id + 4);
+  const bool any = (on[0] | on[1] | on[2]) != 0;
+  // plasma frequency and collision rate at the cell, y + 1, x + 1 and both
+  float om[4][5], ga[4][5];
+  if (any)
+  {
+    const size_t at[4] = {id, id + pz, id + sx, id + sx + pz};
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+    {
+      ld4v (p.omega[1] + at[q], om[q]);
+      ld4v (p.gamma[1] + at[q], ga[q]);
+      om[q][4] = q < 3 ? p.omega[1][at[q] + 4] : 0.f;
+      ga[q][4] = q < 3 ? p.gamma[1][at[q] + 4] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+  {
+    float cu[4], f[4], w[4], g[4];
+    const float one[4] = {1.f, 1.f, 1.f, 1.f};
+    ld4v ((const T *) p.h_old[k] + id, f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      const float e1n = j < 3 ? e[1][j < 3 ? j + 1 : 3] : e1z, e0n = j < 3 ? e[0][j < 3 ? j + 1 : 3] : e0z;
+      cu[j] = k == 0   ? (e1n - e[1][j]) - (e2y[j] - e[2][j])
+              : k == 1 ? (e2x[j] - e[2][j]) - (e0n - e[0][j])
+                       : (e0y[j] - e[0][j]) - (e1x[j] - e[1][j]);
+      if (!((on[k] >> j) & 1u))
+        f[j] = f[j] + p.courant * cu[j];
+      if (any)
+      {
+        // k = 0: cell, z + 1, y + 1, y + 1 z + 1; k = 1: cell, z + 1, x + 1,
+        // x + 1 z + 1; k = 2: cell, y + 1, x + 1, x + 1 y + 1
+        const int q = k == 0 ? 1 : 2;
+        w[j] = 0.25f * (k < 2 ? om[0][j] + om[0][j + 1] + om[q][j] + om[q][j + 1]
+                              : om[0][j] + om[1][j] + om[2][j] + om[3][j]);
+        g[j] = 0.25f * (k < 2 ? ga[0][j] + ga[0][j + 1] + ga[q][j] + ga[q][j + 1]
+                              : ga[0][j] + ga[1][j] + ga[2][j] + ga[3][j]);
+      }
+    }
+    if (on[k])
+      drude_four (p, 3 + k, id, on[k], w, g, one, cu, f);
+    st4v ((T *) p.h_new[k] + id, f, own);
   }
 }
 
@@ -715,20 +890,19 @@ int launch_drude_fixup (const FusedParams &p, const DrudeBox &box, cudaStream_t 
   for (int a = 0; a < 3; ++a)
     hb.lo[a] = max (box.lo[a] - 1, 1);
   auto blocks = [] (const DrudeBox &b) {
-    long long n = 1;
-    for (int a = 0; a < 3; ++a)
-      n *= b.hi[a] - b.lo[a];
-    return (unsigned) std::min<long long> ((n + 255) / 256, 148 * 16);
+    const int z0 = b.lo[2] & ~3;
+    const long long n = (long long) (b.hi[0] - b.lo[0]) * (b.hi[1] - b.lo[1]) * ((b.hi[2] - z0 + 3) / 4);
+    return (unsigned) ((n + 127) / 128);
   };
   if (p.fp16)
   {
-    drude_fix_e_kernel<__half><<<blocks (box), 256, 0, s>>> (p, box);
-    drude_fix_h_kernel<__half><<<blocks (hb), 256, 0, s>>> (p, hb);
+    drude_fix_e_kernel<__half><<<blocks (box), 128, 0, s>>> (p, box);
+    drude_fix_h_kernel<__half><<<blocks (hb), 128, 0, s>>> (p, hb);
   }
   else
   {
-    drude_fix_e_kernel<float><<<blocks (box), 256, 0, s>>> (p, box);
-    drude_fix_h_kernel<float><<<blocks (hb), 256, 0, s>>> (p, hb);
+    drude_fix_e_kernel<float><<<blocks (box), 128, 0, s>>> (p, box);
+    drude_fix_h_kernel<float><<<blocks (hb), 128, 0, s>>> (p, hb);
   }
   return 2;
 }

@@ -41,6 +41,9 @@ struct FusedParams
   // Drude (metamaterials): per-cell bit k set when component k sees a
   // non-zero averaged plasma frequency or collision rate; state of those
   // cells: X (in aux), X two steps back, Z = D1/eps0... scaled, Z one step back
+  // (the sweep's fix-up reads the levels two steps back from the new set's X
+  // and Z instead, which hold them until it writes; only the register-blocked
+  // kernel, whose tiles recompute each other's edge cells, keeps xpp and zpp)
   int use_meta;
   float dt;
   const unsigned char *dflag;
