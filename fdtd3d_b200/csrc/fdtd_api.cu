@@ -1567,6 +1567,7 @@ int tile2d_run (fdtd_ctx *ctx, uint32_t i, int steps)
   p.pu = g.cfg.point_source[ua];
   p.pv = g.cfg.point_source[va];
   p.src = ctx->d_src + kSrcStride * i;
+  p.src_row = kSrcStride;
   p.err = ctx->d_err;
   int slot[6], ns = 0;
   for (int k = 0; k < 6; ++k)

@@ -45,9 +45,11 @@ struct Tile2D
   double dt, dx;
   float courant;               // FP32
   float scale[2];              // FP32: field units of E, H (1, eta0)
-  // point source cell and the steps' source rows (kSrcStride values each)
+  // point source cell; source table: src_row values per step, the incident
+  // grid's source first, then the point source on E and on H
   int pu, pv;
   const double *src;
+  int src_row;
   // TF/SF: the 1-D grid (current and next level) and the incident distance
   int use_tfsf;
   const double *e_in, *h_in;
