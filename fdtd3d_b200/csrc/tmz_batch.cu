@@ -8,16 +8,16 @@
 // cells); the step semantics are the reference's (no field update at t = 0,
 // Source/Scheme/Scheme.inc.h:1032; hard point source after the E update).
 //
-// Work decomposition: a work list of tiles (instance, 30-cell y strip,
-// x chunk).  One warp owns a tile: lane 0 holds the y-1 halo, lanes 1..30
-// the owned cells, lane 31 the y+1 ring whose Ez it recomputes; neighbours
-// along y move by warp shuffles, along x by registers as the warp marches.
-// E and H of one time step are done in that single sweep (fields double
-// buffered, so tiles need no mutual ordering inside a step).  Warps take
-// tiles from a per-step atomic counter; a grid-wide barrier separates time
-// steps.  The barrier is a bounded spin on a global generation counter
-// (globaltimer timeout -> error flag, every CTA leaves); the kernel is
-// launched cooperatively so all CTAs are co-resident.
+// Work decomposition: a work list of tiles, largest instance first, taken by
+// persistent CTAs from an atomic counter.  A round advances every tile up to
+// kTileSteps steps (tile2d.cuh: own cells and halo in registers and shared
+// memory, the halo recomputed), fields double buffered; a grid-wide barrier
+// separates rounds.  One step per round (a warp per 30-cell strip, fields
+// streamed from L2 / HBM) was bound by bytes in flight and the barrier: 20
+// instances, 6.08 M cells: 82 us per step, 49 us now.
+// The barrier is a bounded spin on a global generation counter (globaltimer
+// timeout -> error flag, every CTA leaves); the kernel is launched
+// cooperatively so all CTAs are co-resident.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,12 +29,12 @@
 #include "../../include/fdtd_b200.h"
 #include "kernels.h"
 #include "setup.h"
+#include "tile2d.cuh"
 
 namespace fdtdb {
 
 namespace {
 
-constexpr int kStrip = 30;            // owned y cells per warp tile
 constexpr double kEta0B = 376.730313461770655;
 
 struct InstDev
@@ -48,26 +48,21 @@ struct InstDev
 
 // per instance, 12 tables laid out back to back:
 //   Ez: ca1(x) sq1(x) p5(y) q5(y)    Hx: g4p(x) g4m(x) ca1(y) sq1(y)    Hy: p5(x) q5(x) g4p(y) g4m(y)
-// each of length nx or ny, in that order
+// each of length nx or ny, in that order; the pairs along the dropped axis
+// are the six identity values at the head of the array
 
 struct TileDev
 {
-  int inst, y0, xa, xb;
+  int inst, u0, v0;                   // corner of the tile, halo included
 };
 
 struct BatchParams
 {
-  const InstDev *inst;
+  const Tile2D *inst[2];              // per instance, buffer set 0 / 1 as the current one
   const TileDev *tiles;
-  int ntiles;
-  const float *tab;
-  float *ez[2], *hx[2], *hy[2];
-  float *aez[2], *ahx[2], *ahy[2];
-  const float *eps;
-  const double *src;                  // E source value per step of this launch
-  float courant;
-  int use_pml;
-  unsigned *counters;                 // [0], [1]: tile counters by step parity; [2]: barrier arrivals
+  int ntiles, ninst;
+  const double *src;                  // E source value per step of this launch, from [1]
+  unsigned *counters;                 // [0], [1]: tile counters by round parity; [2]: barrier arrivals
   unsigned *generation;
   int *err;
   long long timeout_ns;
@@ -89,7 +84,7 @@ __device__ bool grid_barrier (const BatchParams &p)
 {
   __shared__ int ok;
   __syncthreads ();
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0 && threadIdx.y == 0)
   {
     volatile unsigned *gen = p.generation;
     unsigned g = *gen;
@@ -121,163 +116,61 @@ __device__ bool grid_barrier (const BatchParams &p)
   return ok != 0;
 }
 
-__device__ __forceinline__ float pml_update (bool interior, float f, float curl, float inv_m, float ca1, float sq1,
-                                             float p5, float q5, float g4p, float g4m, const float *ao, float *an,
-                                             long long id, bool store, float courant)
+template <int CU, int CV>
+__global__ void __launch_bounds__ (kTileThreads, 1) tmz_batch_kernel (BatchParams p)
 {
-  if (interior)
-    return f + courant * inv_m * curl;
-  const float xo = ao[id];
-  const float xn = ca1 * xo + sq1 * curl;
-  if (store)
-    an[id] = xn;
-  return p5 * f + (g4p * xn - g4m * xo) * q5 * inv_m;
-}
-
-__global__ void __launch_bounds__ (512) tmz_batch_kernel (BatchParams p)
-{
-  const int lane = threadIdx.x & 31;
-  const int warps = blockDim.x >> 5;
-  __shared__ int s_tile[32];
+  extern __shared__ __align__ (16) unsigned char tile_smem[];
+  __shared__ double s_inc[2][kTileThreads];
+  __shared__ Tile2D s_p;
+  __shared__ int s_tile;
+  const int tid = threadIdx.x + 32 * threadIdx.y;
   int cur = p.cur;
-  for (unsigned s = 0; s < p.nsteps; ++s)
+  unsigned s = 0;
+  if (p.t_start == 0)
   {
-    const unsigned t = p.t_start + s;
-    const int o = cur, nw = 1 - cur;
-    if (t == 0)
-    {
-      // no field update at t = 0; the hard source still sets Ez
-      if (blockIdx.x == 0)
+    // no field update at t = 0; the hard source still sets Ez
+    if (blockIdx.x == 0)
+      for (int i = tid; i < p.ninst; i += kTileThreads)
       {
-        for (int i = threadIdx.x; i < p.ntiles; i += blockDim.x)
-        {
-          const TileDev td = p.tiles[i];
-          const InstDev in = p.inst[td.inst];
-          if (in.ps && td.y0 == 1 && td.xa == 1)
-          {
-            long long id = in.off + (long long) (in.nx / 2) * in.ny + in.ny / 2;
-            p.ez[o][id] = (float) p.src[s];
-          }
-        }
+        const Tile2D &q = p.inst[cur][i];
+        if (q.comp[0].source)
+          ((float *) q.comp[0].in)[(long long) q.pu * q.nv + q.pv] = (float) p.src[1];
       }
-      if (!grid_barrier (p))
-        return;
-      continue;
-    }
-    const int warp = threadIdx.x >> 5;
-    for (;;)
-    {
-      int tile;
-      if (lane == 0)
-        tile = (int) atomicAdd (&p.counters[t & 1], 1u);
-      tile = __shfl_sync (0xffffffffu, tile, 0);
-      if (tile >= p.ntiles)
-        break;
-      const TileDev td = p.tiles[tile];
-      const InstDev in = p.inst[td.inst];
-      const int nx = in.nx, ny = in.ny;
-      const int y = td.y0 - 1 + lane;
-      const bool valid = y <= ny - 1;
-      const bool inner = y >= 1 && y <= ny - 2;
-      const bool own = lane >= 1 && lane <= kStrip && inner;
-      const long long base = in.off + y;
-      const float *T = p.tab + in.tab;
-      const float *ez_ca1 = T, *ez_sq1 = T + nx, *ez_p5 = T + 2 * nx, *ez_q5 = T + 2 * nx + ny;
-      const float *hx_g4p = T + 2 * nx + 2 * ny, *hx_g4m = T + 3 * nx + 2 * ny, *hx_ca1 = T + 4 * nx + 2 * ny,
-                  *hx_sq1 = T + 4 * nx + 3 * ny;
-      const float *hy_p5 = T + 4 * nx + 4 * ny, *hy_q5 = T + 5 * nx + 4 * ny, *hy_g4p = T + 6 * nx + 4 * ny,
-                  *hy_g4m = T + 6 * nx + 5 * ny;
-      const bool ps_col = in.ps && y == ny / 2;
-      const int psx = nx / 2;
-      const bool y_in_ez = y >= in.ilo[0][1] && y < in.ihi[0][1];
-      const bool y_in_hx = y >= in.ilo[1][1] && y < in.ihi[1][1];
-      const bool y_in_hy = y >= in.ilo[2][1] && y < in.ihi[2][1];
-      const float ez_p5y = valid ? ez_p5[y] : 1.f, ez_q5y = valid ? ez_q5[y] : 1.f;
-      const float hx_ca1y = valid ? hx_ca1[y] : 1.f, hx_sq1y = valid ? hx_sq1[y] : 0.f;
-      const float hy_g4py = valid ? hy_g4p[y] : 1.f, hy_g4my = valid ? hy_g4m[y] : 1.f;
-
-      // state of plane xa - 1
-      float hy_prev = 0.f, hx_prev = 0.f, ez_prev = 0.f;
-      if (valid)
-      {
-        const long long id = base + (long long) (td.xa - 1) * ny;
-        hy_prev = p.hy[o][id];
-        hx_prev = p.hx[o][id];
-      }
-      // the old fields of plane x are loaded three planes ahead (a register
-      // ring), so each warp keeps four planes of loads in flight; loads read
-      // only the old buffers and stores go to the new ones
-      const float *Hx = p.hx[o], *Hy = p.hy[o], *Ez = p.ez[o];
-      auto load = [&] (int x, float &a, float &b, float &c, float &d) {
-        a = b = c = 0.f;
-        d = 1.f;
-        if (valid && x <= td.xb + 1)
-        {
-          const long long id = base + (long long) x * ny;
-          a = Hx[id];
-          b = Hy[id];
-          c = Ez[id];
-          if (p.eps)
-            d = p.eps[id];
-        }
-      };
-      float c_hx, c_hy, c_ez, c_ep, n1_hx, n1_hy, n1_ez, n1_ep, n2_hx, n2_hy, n2_ez, n2_ep, n3_hx, n3_hy, n3_ez,
-          n3_ep;
-      load (td.xa, c_hx, c_hy, c_ez, c_ep);
-      load (td.xa + 1, n1_hx, n1_hy, n1_ez, n1_ep);
-      load (td.xa + 2, n2_hx, n2_hy, n2_ez, n2_ep);
-      load (td.xa + 3, n3_hx, n3_hy, n3_ez, n3_ep);
-      for (int x = td.xa; x <= td.xb + 1; ++x)
-      {
-        const long long id = base + (long long) x * ny;
-        const float hx = c_hx, hy = c_hy, ez = c_ez, ep = c_ep;
-        c_hx = n1_hx, c_hy = n1_hy, c_ez = n1_ez, c_ep = n1_ep;
-        n1_hx = n2_hx, n1_hy = n2_hy, n1_ez = n2_ez, n1_ep = n2_ep;
-        n2_hx = n3_hx, n2_hy = n3_hy, n2_ez = n3_ez, n2_ep = n3_ep;
-        load (x + 4, n3_hx, n3_hy, n3_ez, n3_ep);
-        const float hx_m = __shfl_up_sync (0xffffffffu, hx, 1);
-        float ezn = ez;
-        if (lane >= 1 && inner && x <= nx - 2)
-        {
-          const float curl = (hy - hy_prev) - (hx - hx_m);
-          const bool interior = !p.use_pml || (y_in_ez && x >= in.ilo[0][0] && x < in.ihi[0][0]);
-          ezn = pml_update (interior, ez, curl, 1.f / ep, ez_ca1[x], ez_sq1[x], ez_p5y, ez_q5y, 1.f, 1.f,
-                            p.aez[o], p.aez[nw], id, own && x <= td.xb, p.courant);
-          if (ps_col && x == psx)
-            ezn = (float) p.src[s];
-          if (own && x <= td.xb)
-            p.ez[nw][id] = ezn;
-        }
-        // H at x - 1 from Ez_new(x - 1) (this lane and lane + 1) and Ez_new(x)
-        const float ezp_dn = __shfl_down_sync (0xffffffffu, ez_prev, 1);
-        const int xh = x - 1;
-        if (own && xh >= td.xa && xh <= nx - 2)
-        {
-          const long long hid = id - ny;
-          const float cx = ez_prev - ezp_dn;      // Hx: Ez(y) - Ez(y + 1)
-          const float cy = ezn - ez_prev;         // Hy: Ez(x + 1) - Ez(x)
-          const bool ix = !p.use_pml || (y_in_hx && xh >= in.ilo[1][0] && xh < in.ihi[1][0]);
-          const bool iy = !p.use_pml || (y_in_hy && xh >= in.ilo[2][0] && xh < in.ihi[2][0]);
-          const float hxn = pml_update (ix, hx_prev, cx, 1.f, hx_ca1y, hx_sq1y, 1.f, 1.f, hx_g4p[xh], hx_g4m[xh],
-                                        p.ahx[o], p.ahx[nw], hid, true, p.courant);
-          const float hyn = pml_update (iy, hy_prev, cy, 1.f, 1.f, p.courant, hy_p5[xh], hy_q5[xh], hy_g4py,
-                                        hy_g4my, p.ahy[o], p.ahy[nw], hid, true, p.courant);
-          p.hx[nw][hid] = hxn;
-          p.hy[nw][hid] = hyn;
-        }
-        hx_prev = hx;
-        hy_prev = hy;
-        ez_prev = ezn;
-      }
-    }
-    (void) warp;
-    (void) s_tile;
-    // the counter of the next step (same parity as the previous one) is idle now
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-      atomicExch (&p.counters[(t + 1) & 1], 0u);
     if (!grid_barrier (p))
       return;
-    cur = nw;
+    s = 1;
+  }
+  for (unsigned round = 0; s < p.nsteps; ++round)
+  {
+    const int steps = (int) min ((unsigned) kTileSteps, p.nsteps - s);
+    for (;;)
+    {
+      __syncthreads ();   // (the previous tile's shared values have been used)
+      if (tid == 0)
+        s_tile = (int) atomicAdd (&p.counters[round & 1], 1u);
+      __syncthreads ();
+      if (s_tile >= p.ntiles)
+        break;
+      const TileDev t = p.tiles[s_tile];
+      const unsigned *from = reinterpret_cast<const unsigned *> (p.inst[cur] + t.inst);
+      for (int q = tid; q < (int) (sizeof (Tile2D) / 4); q += kTileThreads)
+        reinterpret_cast<unsigned *> (&s_p)[q] = from[q];
+      __syncthreads ();
+      if (tid == 0)
+      {
+        s_p.steps = steps;
+        s_p.src = p.src + s;
+      }
+      __syncthreads ();
+      tile2d_steps<float, float, CU, CV, 0> (s_p, t.u0, t.v0, tile_smem, s_inc);
+    }
+    // the counter of the next round (same parity as the previous one) is idle now
+    if (blockIdx.x == 0 && tid == 0)
+      atomicExch (&p.counters[(round + 1) & 1], 0u);
+    if (!grid_barrier (p))
+      return;
+    cur ^= 1;
+    s += steps;
   }
 }
 
@@ -299,7 +192,9 @@ struct fdtd_batch
   long long cells = 0;
   int ntab = 0;
   std::vector<float> tab_host;
-  fdtdb::InstDev *d_inst = nullptr;
+  fdtdb::Tile2D *d_inst[2] = {};
+  double *stage = nullptr;            // FP64 copy of one component on its way to the host
+  size_t stage_cells = 0;
   fdtdb::TileDev *d_tiles = nullptr;
   int ntiles = 0;
   float *d_tab = nullptr;
@@ -311,10 +206,10 @@ struct fdtd_batch
   unsigned *d_generation = nullptr;
   int *d_err = nullptr;
   int cur = 0;
-  // launch shape (autotuned)
+  // launch shape (autotuned): tile height in x (64: 64 x 64 cells, 32: 32 x
+  // 32, halo included), CTAs per SM
   int x_chunk = 64;
-  int warps_per_cta = 8;
-  int ctas_per_sm = 2;
+  int ctas_per_sm = 1;
   // graph of (source upload, counter reset, persistent kernel)
   cudaGraphExec_t graph = nullptr;
   unsigned graph_steps = 0;
@@ -380,9 +275,10 @@ int build_tiles (fdtd_batch *b, int x_chunk)
   for (int i : order)
   {
     const fdtdb::InstDev &in = b->inst[i];
-    for (int xa = 1; xa <= in.nx - 2; xa += x_chunk)
-      for (int y0 = 1; y0 <= in.ny - 2; y0 += fdtdb::kStrip)
-        tiles.push_back ({i, y0, xa, std::min (xa + x_chunk - 1, in.nx - 2)});
+    const int own = x_chunk - 2 * fdtdb::kTileSteps;
+    for (int u = 0; u < in.nx; u += own)
+      for (int v = 0; v < in.ny; v += own)
+        tiles.push_back ({i, u - fdtdb::kTileSteps, v - fdtdb::kTileSteps});
   }
   if (b->d_tiles)
   {
@@ -415,23 +311,12 @@ BatchParams params (fdtd_batch *b, uint32_t t_start, uint32_t n)
 {
   BatchParams p;
   std::memset (&p, 0, sizeof (p));
-  p.inst = b->d_inst;
+  p.inst[0] = b->d_inst[0];
+  p.inst[1] = b->d_inst[1];
+  p.ninst = (int) b->inst.size ();
   p.tiles = b->d_tiles;
   p.ntiles = b->ntiles;
-  p.tab = b->d_tab;
-  for (int s = 0; s < 2; ++s)
-  {
-    p.ez[s] = b->ez[s];
-    p.hx[s] = b->hx[s];
-    p.hy[s] = b->hy[s];
-    p.aez[s] = b->aez[s];
-    p.ahx[s] = b->ahx[s];
-    p.ahy[s] = b->ahy[s];
-  }
-  p.eps = b->eps;
   p.src = b->d_src;
-  p.courant = (float) (fdtdb::kC * b->geo[0].dt / b->geo[0].dx);
-  p.use_pml = b->base.use_pml;
   p.counters = b->d_counters;
   p.generation = b->d_generation;
   p.err = b->d_err;
@@ -442,37 +327,65 @@ BatchParams params (fdtd_batch *b, uint32_t t_start, uint32_t n)
   return p;
 }
 
-int max_ctas (fdtd_batch *b, int warps)
+// The kernel of a tile height and its shared memory.
+const void *batch_kernel (int tile, int &smem)
 {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, fdtdb::tmz_batch_kernel, warps * 32, 0)
-      != cudaSuccess)
+  using fdtdb::TileMem;
+  if (tile == 32)
+  {
+    smem = TileMem<float, 2, 1>::BYTES;
+    return (const void *) fdtdb::tmz_batch_kernel<2, 1>;
+  }
+  smem = TileMem<float, 4, 2>::BYTES;
+  return (const void *) fdtdb::tmz_batch_kernel<4, 2>;
+}
+
+// co-resident CTAs per SM (0: the kernel does not fit)
+int max_ctas (int tile)
+{
+  int per_sm = 0, smem = 0;
+  const void *k = batch_kernel (tile, smem);
+  if (cudaFuncSetAttribute (k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, k, fdtdb::kTileThreads, smem) != cudaSuccess)
+  {
+    cudaGetLastError ();
     return 0;
+  }
   return per_sm;
 }
 
 // Enqueues one launch (source upload, counter reset, cooperative kernel).
 int enqueue (fdtd_batch *b, uint32_t t_start, uint32_t n)
 {
-  BCK (cudaMemcpyAsync (b->d_src, b->h_src, (size_t) n * sizeof (double), cudaMemcpyHostToDevice, b->stream));
+  BCK (cudaMemcpyAsync (b->d_src + 1, b->h_src, (size_t) n * sizeof (double), cudaMemcpyHostToDevice, b->stream));
   BCK (cudaMemsetAsync (b->d_counters, 0, 3 * sizeof (unsigned), b->stream));
   BatchParams p = params (b, t_start, n);
   void *args[] = {&p};
-  int ctas = std::min (b->ctas_per_sm, max_ctas (b, b->warps_per_cta)) * b->sm_count;
+  int ctas = std::min (b->ctas_per_sm, max_ctas (b->x_chunk)) * b->sm_count;
   if (ctas <= 0)
     return bfail (b, FDTD_ERR_CUDA, "batch kernel does not fit on the device");
+  int smem = 0;
+  const void *kern = batch_kernel (b->x_chunk, smem);
   cudaLaunchConfig_t lc;
   std::memset (&lc, 0, sizeof (lc));
   lc.gridDim = dim3 (ctas);
-  lc.blockDim = dim3 (b->warps_per_cta * 32);
+  lc.blockDim = dim3 (32, fdtdb::kTileWarps);
+  lc.dynamicSmemBytes = smem;
   lc.stream = b->stream;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeCooperative;
   attr.val.cooperative = 1;
   lc.attrs = &attr;
   lc.numAttrs = 1;
-  BCK (cudaLaunchKernelExC (&lc, (const void *) fdtdb::tmz_batch_kernel, args));
+  BCK (cudaLaunchKernelExC (&lc, kern, args));
   return FDTD_OK;
+}
+
+// Rounds of a launch: the buffer set changes with each.
+uint32_t batch_rounds (uint32_t t_start, uint32_t n)
+{
+  const uint32_t steps = n - (t_start == 0 ? 1 : 0);
+  return (steps + fdtdb::kTileSteps - 1) / fdtdb::kTileSteps;
 }
 
 }  // namespace
@@ -519,8 +432,8 @@ int create_batch (fdtd_batch *b, const fdtd_config *base, int count, const int *
   BCK (cudaEventCreate (&b->ev1));
   b->geo.resize (count);
   b->inst.resize (count);
-  const double S_unused = 0;
-  (void) S_unused;
+  const float identity[6] = {1.f, 0.f, 1.f, 1.f, 1.f, 1.f};   // ([1]: S, once it is known)
+  b->tab_host.assign (identity, identity + 6);
   for (int i = 0; i < count; ++i)
   {
     fdtd_config c = *base;
@@ -544,6 +457,7 @@ int create_batch (fdtd_batch *b, const fdtd_config *base, int count, const int *
     in.ps = c.point_source_mask ? 1 : 0;
     b->cells += (long long) in.nx * in.ny;
     const double S = kC * g.dt / g.dx;
+    b->tab_host[1] = (float) S;
     // tables: Ez ca1(x) sq1(x) p5(y) q5(y); Hx g4p(x) g4m(x) ca1(y) sq1(y); Hy p5(x) q5(x) g4p(y) g4m(y)
     struct Spec
     {
@@ -606,9 +520,63 @@ int create_batch (fdtd_batch *b, const fdtd_config *base, int count, const int *
   BALLOC (b->d_tab, b->tab_host.size () * sizeof (float));
   BCK (cudaMemcpyAsync (b->d_tab, b->tab_host.data (), b->tab_host.size () * sizeof (float), cudaMemcpyHostToDevice,
                         b->stream));
-  BALLOC (b->d_inst, b->inst.size () * sizeof (fdtdb::InstDev));
-  BCK (cudaMemcpyAsync (b->d_inst, b->inst.data (), b->inst.size () * sizeof (fdtdb::InstDev), cudaMemcpyHostToDevice,
-                        b->stream));
+  // per instance, each buffer set as the current one
+  std::vector<Tile2D> dev (b->inst.size ());
+  for (int set = 0; set < 2; ++set)
+  {
+    for (size_t i = 0; i < b->inst.size (); ++i)
+    {
+      const InstDev &in = b->inst[i];
+      Tile2D &t = dev[i];
+      std::memset (&t, 0, sizeof (t));
+      t.nu = in.nx;
+      t.nv = in.ny;
+      t.use_pml = base->use_pml;
+      t.courant = (float) (kC * b->geo[i].dt / b->geo[i].dx);
+      t.scale[0] = 1.f;
+      t.scale[1] = (float) kEta0B;
+      t.pu = in.nx / 2;
+      t.pv = in.ny / 2;
+      t.src_row = 1;
+      const float *T = b->d_tab + in.tab, *I = b->d_tab;
+      const int nx = in.nx, ny = in.ny;
+      const float *ez[4] = {T, T + nx, T + 2 * nx, T + 2 * nx + ny};
+      T += 2 * nx + 2 * ny;
+      const float *hx[4] = {T, T + nx, T + 2 * nx, T + 2 * nx + ny};
+      T += 2 * nx + 2 * ny;
+      const float *hy[4] = {T, T + nx, T + 2 * nx, T + 2 * nx + ny};
+      const float *tab[3][6] = {{ez[0], ez[1], ez[2], ez[3], I + 4, I + 5},
+                                {hx[2], hx[3], I + 2, I + 3, hx[0], hx[1]},
+                                {I + 0, I + 1, hy[0], hy[1], hy[2], hy[3]}};
+      float *const f[3][2] = {{b->ez[0], b->ez[1]}, {b->hx[0], b->hx[1]}, {b->hy[0], b->hy[1]}};
+      float *const x[3][2] = {{b->aez[0], b->aez[1]}, {b->ahx[0], b->ahx[1]}, {b->ahy[0], b->ahy[1]}};
+      for (int j = 0; j < 3; ++j)
+      {
+        TileComp &c = t.comp[j];
+        c.nmat = 1;
+        c.mat = j == 0 ? b->eps + in.off : nullptr;
+        c.in = f[j][set] + in.off;
+        c.out = f[j][1 - set] + in.off;
+        if (base->use_pml)
+        {
+          c.aux_in = x[j][set] + in.off;
+          c.aux_out = x[j][1 - set] + in.off;
+        }
+        for (int q = 0; q < 6; ++q)
+          c.tab[q] = tab[j][q];
+        for (int a = 0; a < 2; ++a)
+        {
+          c.ilo[a] = in.ilo[j][a];
+          c.ihi[a] = in.ihi[j][a];
+        }
+        c.source = j == 0 && in.ps;
+      }
+    }
+    BALLOC (b->d_inst[set], dev.size () * sizeof (Tile2D));
+    BCK (cudaMemcpyAsync (b->d_inst[set], dev.data (), dev.size () * sizeof (Tile2D), cudaMemcpyHostToDevice,
+                          b->stream));
+    BCK (cudaStreamSynchronize (b->stream));
+  }
   BALLOC (b->d_counters, 4 * sizeof (unsigned));
   BALLOC (b->d_generation, sizeof (unsigned));
   BALLOC (b->d_err, sizeof (int));
@@ -633,7 +601,7 @@ int ensure_src (fdtd_batch *b, size_t n)
     b->d_src = nullptr;
   }
   size_t cap = std::max<size_t> (n, 1024);
-  BALLOC (b->d_src, cap * sizeof (double));
+  BALLOC (b->d_src, (cap + 1) * sizeof (double));
   BCK (fdtdb::pinned_malloc ((void **) &b->h_src, cap * sizeof (double)));
   b->src_cap = cap;
   drop_graph (b);
@@ -704,9 +672,8 @@ int step_batch (fdtd_batch *b, uint32_t t_start, uint32_t n, bool allow_graph)
       return r;
   }
   BCK (cudaEventRecord (b->ev1, b->stream));
-  for (uint32_t s = 0; s < n; ++s)
-    if (t_start + s > 0)
-      b->cur ^= 1;
+  if (batch_rounds (t_start, n) & 1u)
+    b->cur ^= 1;
   return FDTD_OK;
 }
 
@@ -802,11 +769,20 @@ int fdtd_batch_download (fdtd_batch *b, int instance, int component, double *hos
   const fdtdb::InstDev &in = b->inst[instance];
   size_t n = (size_t) in.nx * in.ny;
   const float *src = component == FDTD_EZ ? b->ez[b->cur] : (component == FDTD_HX ? b->hx[b->cur] : b->hy[b->cur]);
-  std::vector<float> f (n);
-  BCK (cudaMemcpy (f.data (), src + in.off, n * sizeof (float), cudaMemcpyDeviceToHost));
-  double scale = component == FDTD_EZ ? 1.0 : 1.0 / fdtdb::kEta0B;
-  for (size_t i = 0; i < n; ++i)
-    host[i] = (double) f[i] * scale;
+  // widened on the device, then one copy into the caller's buffer
+  if (n > b->stage_cells)
+  {
+    size_t most = 0;
+    for (const fdtdb::InstDev &i : b->inst)
+      most = std::max (most, (size_t) i.nx * i.ny);
+    BALLOC (b->stage, most * sizeof (double));
+    b->stage_cells = most;
+  }
+  fdtdb::launch_convert_out (b->stage, src + in.off, 1, 1, (int) n, (int) n,
+                             component == FDTD_EZ ? 1.0 : 1.0 / fdtdb::kEta0B, b->stream);
+  BCK (cudaGetLastError ());
+  BCK (cudaMemcpyAsync (host, b->stage, n * sizeof (double), cudaMemcpyDeviceToHost, b->stream));
+  BCK (cudaStreamSynchronize (b->stream));
   return FDTD_OK;
 }
 
@@ -815,41 +791,37 @@ int fdtd_batch_tune (fdtd_batch *b, int steps, int *choice)
   if (!b || steps < 1)
     return FDTD_ERR_ARG;
   BCK (cudaSetDevice (b->device));
-  static const int chunks[] = {16, 32, 64, 128};
-  static const int warps[] = {4, 8, 16};
+  static const int tiles[] = {32, 64};
   static const int per_sm[] = {1, 2, 4};
   double best = 1e30;
-  int bc = b->x_chunk, bw = b->warps_per_cta, bs = b->ctas_per_sm;
-  for (int c : chunks)
+  int bc = b->x_chunk, bs = b->ctas_per_sm;
+  for (int c : tiles)
   {
     int r = build_tiles (b, c);
     if (r != FDTD_OK)
       return r;
-    for (int w : warps)
-      for (int s : per_sm)
+    for (int s : per_sm)
+    {
+      if (s > max_ctas (c))
+        continue;
+      b->ctas_per_sm = s;
+      r = step_batch (b, 1, (uint32_t) steps, false);
+      if (r != FDTD_OK)
+        return r;
+      BCK (cudaStreamSynchronize (b->stream));
+      float ms = 0.f;
+      BCK (cudaEventElapsedTime (&ms, b->ev0, b->ev1));
+      int flag = 0;
+      BCK (cudaMemcpy (&flag, b->d_err, sizeof (int), cudaMemcpyDeviceToHost));
+      if (flag)
+        return bfail (b, FDTD_ERR_DEVICE, "a grid barrier timed out while tuning");
+      if (ms < best)
       {
-        if (s > max_ctas (b, w))
-          continue;
-        b->warps_per_cta = w;
-        b->ctas_per_sm = s;
-        r = step_batch (b, 1, (uint32_t) steps, false);
-        if (r != FDTD_OK)
-          return r;
-        BCK (cudaStreamSynchronize (b->stream));
-        float ms = 0.f;
-        BCK (cudaEventElapsedTime (&ms, b->ev0, b->ev1));
-        int flag = 0;
-        BCK (cudaMemcpy (&flag, b->d_err, sizeof (int), cudaMemcpyDeviceToHost));
-        if (flag)
-          return bfail (b, FDTD_ERR_DEVICE, "a grid barrier timed out while tuning");
-        if (ms < best)
-        {
-          best = ms;
-          bc = c;
-          bw = w;
-          bs = s;
-        }
+        best = ms;
+        bc = c;
+        bs = s;
       }
+    }
   }
   // back to the state before tuning: zero fields and auxiliaries, t = 0
   size_t bytes = (size_t) b->cells * sizeof (float);
@@ -861,7 +833,6 @@ int fdtd_batch_tune (fdtd_batch *b, int steps, int *choice)
         BCK (cudaMemsetAsync (a, 0, bytes, b->stream));
   }
   b->cur = 0;
-  b->warps_per_cta = bw;
   b->ctas_per_sm = bs;
   int r = build_tiles (b, bc);
   if (r != FDTD_OK)
@@ -871,7 +842,7 @@ int fdtd_batch_tune (fdtd_batch *b, int steps, int *choice)
   if (choice)
   {
     choice[0] = bc;
-    choice[1] = bw;
+    choice[1] = fdtdb::kTileWarps;
     choice[2] = bs;
   }
   return FDTD_OK;

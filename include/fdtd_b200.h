@@ -337,7 +337,7 @@ typedef struct fdtd_batch fdtd_batch;
 int fdtd_batch_create (const fdtd_config *base, int count, const int *sizes, int device, fdtd_batch **out);
 /* eps of one instance: nx*ny host doubles, (x, y) with y fastest */
 int fdtd_batch_upload_eps (fdtd_batch *b, int instance, const double *host);
-/* Times every candidate launch shape (x chunk of a warp tile, warps per CTA,
+/* Times every candidate launch shape (x extent of a tile, warps per CTA,
  * CTAs per SM) over `steps` steps of the real batch, keeps the fastest,
  * then resets the fields to t = 0.  choice[3] receives the shape. */
 int fdtd_batch_tune (fdtd_batch *b, int steps, int *choice);
