@@ -18,15 +18,19 @@
 // overwritten).  dJ/d eps = sum over the Ez cells whose average includes
 // the cell of dJ/d im * (-im^2 / n_points).
 //
-// Execution: one persistent cooperative kernel runs many half-steps with a
-// bounded grid barrier between them (a 512^2 grid is a few MB per field and
-// lives in L2, so a half-step is far shorter than a kernel launch).  The
-// forward run is one launch that also stores the checkpoints (the state
-// before every K-th step) and, for the last segment, dEz/dim and the probe
-// values the reverse sweep needs.  Every reverse launch splits its CTAs in
-// two groups with a barrier each: one group reverses segment j from the
-// stored per-step data while the other recomputes segment j - 1 from its
-// checkpoint into the other half of the double buffer.
+// Execution: one persistent cooperative kernel runs many steps in rounds of up
+// to kRound with a bounded grid barrier between them.  In a round a CTA takes
+// tiles of the grid with a halo of kRound cells, holds its cells in registers
+// and the values neighbours read in shared memory, and recomputes the halo
+// instead of exchanging it; the state is double buffered between rounds.
+// (With a grid barrier per half-step the run was bound by barrier and L2
+// latency, about 6 us each: 512^2, 800 steps, checkpoint 100: forward 11.3 ms,
+// backward 26.3 ms; now 2.3 and 10.8 ms.)  The forward run is one launch that
+// also stores the checkpoints (the state before every K-th step) and, for the
+// last segment, dEz/dim and the probe values the reverse sweep needs.  Every
+// reverse launch splits its CTAs in two groups with a barrier each: one group
+// reverses segment j from the stored per-step data while the other recomputes
+// segment j - 1 from its checkpoint into the other half of the double buffer.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -44,6 +48,7 @@ namespace {
 constexpr int kEz = 0, kHx = 1, kHy = 2;   // local component slots
 constexpr double kEta0Adj = 376.730313461770655;
 constexpr int kThreads = 512;
+constexpr int kRound = 7;                  // steps per round at most: the halo of a tile
 constexpr int kBarStride = 64;             // words per group barrier: arrivals at [0], generation at [32]
 constexpr long long kDefaultBarrierLimitNs = 2000000000LL;   // 2 s
 
@@ -55,8 +60,6 @@ struct AdjDev
   int ilo[3][2], ihi[3][2];    // sigma == 0 range per component and axis
   int tax[3][3];               // axis of the (ca1, sq1), (p5, q5), (g4p, g4m) pairs
   const R *tab[3][6];          // tables indexed by the coordinate along the pair's axis
-  int o1[3], o2[3];            // curl sources (local slots, -1 = absent)
-  int d11[3][2], d12[3][2], d21[3][2], d22[3][2];
   const R *im;                 // 1 / averaged eps of Ez
   int ps[2];
   int ps_on[3];                // point source on Ez / Hx / Hy
@@ -74,21 +77,23 @@ struct Launch
   // forward group
   int fwd_ctas;
   uint32_t fk0, fk1;
-  R *F[6];                     // Ez, Hx, Hy, Xz, Xx, Xy
-  const R *load;               // state to start from (6 N values) or null
+  R *F[2];                     // two sets of Ez, Hx, Hy, Xz, Xx, Xy (N values each); a launch starts in set 0
+  const R *load;               // state to start from (6 N values) instead of set 0, or null
   R *ck;                       // state before step k stored at ck + (k / every) 6 N when k % every == 0, or null
   uint32_t every;
   R *dedm;                     // dEz/dim of step k at dedm + (k - keep0) N for k >= keep0, or null
   double *keep;                // probe Ez of step k at keep + (k - keep0) npr
   uint32_t keep0;
-  double *acc;                 // compensated J (sum, compensation) or null
+  double *jpart;               // sum of Ez^2 over the probe cells of step k and probe tile q at k nprt + q, or null
+  int prt_u0, prt_v0, prt_nv, nprt;   // tiles that hold probe cells
   // reverse group
   uint32_t rk0, rk1;
-  R *aE, *aXz, *aHx, *aHy, *aXx, *aXy;
-  R *acx, *acy, *acz;          // curl adjoints of the H cells and of the Ez cells
+  R *A[2];                     // two sets of aE, aXz, aHx, aHy, aXx, aXy, acz (N values each)
+  int rcur;                    // set the reverse steps start from
   const R *rdedm;              // dEz/dim of step k at rdedm + (k - rk0) N
   const double *rprobe;        // probe Ez of step k at rprobe + (k - rk0) npr
   double *gim;
+  int tiles_u, tiles_v;
   // barriers: arrivals at [0] and generation at [32] for the forward group,
   // the same from [kBarStride] for the reverse group (each word in its own
   // 128-byte line, so polling does not slow the arrivals)
@@ -148,338 +153,571 @@ __device__ bool group_barrier (unsigned *bar, unsigned ctas, int *err, long long
   return ok != 0;
 }
 
-template <typename R>
-__device__ __forceinline__ bool interior (const AdjDev<R> &p, int c, int x, int y)
+// Tile of 16 RU x 32 RV cells, halo included: warp w holds the RU rows u0 + RU
+// w ..., a lane RV neighbouring cells of each.  Differences along y cross lanes
+// by shuffles, those along x cross warps by one shared row per component.
+template <typename R, int RU, int RV>
+struct AdjTile
 {
-  return x >= p.ilo[c][0] && x < p.ihi[c][0] && y >= p.ilo[c][1] && y < p.ihi[c][1];
-}
+  static constexpr int TU = 16 * RU, TV = 32 * RV, TM = TU > TV ? TU : TV, C = RU * RV;
+  static constexpr int OU = TU - 2 * kRound, OV = TV - 2 * kRound;
+  static constexpr int A = 16 * TV;                    // one component's exchanged rows
+  static constexpr int BYTES = (2 * A + 18 * TM) * (int) sizeof (R);
+};
 
-template <typename R>
-__device__ __forceinline__ bool updated (const AdjDev<R> &p, int x, int y)
+// What a thread knows of its cells (bit RV i + j for row i, column j): `upd`:
+// an updated cell, `own`: of the tile's own part and inside the grid, `pml[c]`:
+// component c has PML there.
+template <typename R, int RU, int RV>
+struct AdjCells
 {
-  return x >= 1 && x <= p.nx - 2 && y >= 1 && y <= p.ny - 2;
-}
-
-template <typename R>
-__device__ __forceinline__ R tabv (const AdjDev<R> &p, int c, int j, int x, int y)
-{
-  const int ax = p.tax[c][j / 2];
-  return p.tab[c][j][ax == 0 ? x : (ax == 1 ? y : 0)];   // z has one (sigma = 0) entry in 2-D
-}
-
-template <typename R>
-__device__ __forceinline__ R curl_of (const AdjDev<R> &p, int c, const R *const F[3], int x, int y)
-{
-  R v0 = 0, v1 = 0, v2 = 0, v3 = 0;
-  const int ny = p.ny;
-  if (p.o1[c] >= 0)
+  using L = AdjTile<R, RU, RV>;
+  int u0, v0, w, lane;
+  unsigned valid = 0, upd = 0, own = 0, source = 0, pml[3] = {0, 0, 0};
+  __device__ AdjCells (const AdjDev<R> &p, int u0_, int v0_) : u0 (u0_), v0 (v0_)
   {
-    const R *f = F[p.o1[c]];
-    v0 = ld (f + (x + p.d11[c][0]) * ny + y + p.d11[c][1]);
-    v1 = ld (f + (x + p.d12[c][0]) * ny + y + p.d12[c][1]);
+    w = threadIdx.x >> 5;
+    lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < L::C; ++r)
+    {
+      const int x = u0 + du (r), y = v0 + dv (r);
+      const unsigned bit = 1u << r;
+      const bool in = x >= 0 && x < p.nx && y >= 0 && y < p.ny;
+      const bool up = x >= 1 && x <= p.nx - 2 && y >= 1 && y <= p.ny - 2;
+      valid |= in ? bit : 0u;
+      upd |= up ? bit : 0u;
+      own |= in && du (r) >= kRound && du (r) < L::TU - kRound && dv (r) >= kRound && dv (r) < L::TV - kRound ? bit : 0u;
+      source |= up && x == p.ps[0] && y == p.ps[1] ? bit : 0u;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        pml[c] |= up && !(x >= p.ilo[c][0] && x < p.ihi[c][0] && y >= p.ilo[c][1] && y < p.ihi[c][1]) ? bit : 0u;
+    }
   }
-  if (p.o2[c] >= 0)
+  __device__ int du (int r) const { return RU * w + r / RV; }
+  __device__ int dv (int r) const { return RV * lane + r % RV; }
+  __device__ int id (const AdjDev<R> &p, int r) const { return (u0 + du (r)) * p.ny + v0 + dv (r); }
+};
+
+// The PML coefficients of component c for a thread's cells, from the tile's
+// tables (entry j of component c at T[(6 c + j) TM + q], q the offset along the
+// pair's axis, 0 along the dropped one): ca1, sq1, p5, q5, g4p, g4m, each a
+// value per row, per column or one.
+template <typename R, int RU, int RV>
+struct AdjCoef
+{
+  static constexpr int N = RU > RV ? RU : RV;
+  R t[6][N];
+  // Ez: x, y, z; Hx: y, z, x; Hy: z, x, y
+  __device__ static constexpr int axis (int c, int pair)
   {
-    const R *f = F[p.o2[c]];
-    v2 = ld (f + (x + p.d21[c][0]) * ny + y + p.d21[c][1]);
-    v3 = ld (f + (x + p.d22[c][0]) * ny + y + p.d22[c][1]);
+    return c == kEz ? pair : (c == kHx ? (pair + 1) % 3 : (pair + 2) % 3);
   }
-  return (v1 - v0) - (v3 - v2);
+  __device__ AdjCoef (const R *T, int TM, int c, int row, int col)
+  {
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+    {
+      const int ax = axis (c, j / 2);
+      const R *from = T + (6 * c + j) * TM + (ax == 0 ? row : (ax == 1 ? col : 0));
+#pragma unroll
+      for (int i = 0; i < (ax == 0 ? RU : (ax == 1 ? RV : 1)); ++i)
+        t[j][i] = from[i];
+    }
+  }
+  __device__ R at (int c, int j, int r) const
+  {
+    const int ax = axis (c, j / 2);
+    return t[j][ax == 0 ? r / RV : (ax == 1 ? r % RV : 0)];
+  }
+};
+
+// Shared PML tables of a tile.
+template <typename R, int RU, int RV>
+__device__ __forceinline__ void adj_tables (const AdjDev<R> &p, R *T, int u0, int v0)
+{
+  using L = AdjTile<R, RU, RV>;
+  for (int q = threadIdx.x; q < 18 * L::TM; q += kThreads)
+  {
+    const int c = q / (6 * L::TM), j = (q / L::TM) % 6, i = q % L::TM;
+    const int ax = p.tax[c][j / 2];
+    const int g = ax == 0 ? u0 + i : (ax == 1 ? v0 + i : 0), n = ax == 0 ? p.nx : (ax == 1 ? p.ny : 1);
+    T[q] = g >= 0 && g < n ? p.tab[c][j][g] : R (1);
+  }
 }
 
-// one component update at (x, y); returns dF/d(im) for the gradient
-template <typename R>
-__device__ __forceinline__ R update_cell (const AdjDev<R> &p, int c, R *F, R *X, R cu, R im, int x, int y)
+// A thread's row r of component f as its neighbours see it: the value one
+// cell lower (D = -1) or higher (D = +1) in y, and the row of the warp before
+// or after in x (row: the warps' exchanged rows).
+template <typename R, int RU, int RV, int D>
+__device__ __forceinline__ void adj_far_y (const R f[RU * RV], R far[RU * RV])
 {
-  const int id = x * p.ny + y;
-  R f = ld (F + id);
-  R dfdm;
-  if (interior (p, c, x, y))
+#pragma unroll
+  for (int i = 0; i < RU; ++i)
   {
-    f += p.S * im * cu;
-    dfdm = p.S * cu;
+    const R o = D < 0 ? __shfl_up_sync (0xffffffffu, f[RV * i + RV - 1], 1) : __shfl_down_sync (0xffffffffu, f[RV * i], 1);
+#pragma unroll
+    for (int j = 0; j < RV; ++j)
+      far[RV * i + j] = D < 0 ? (j > 0 ? f[RV * i + (j > 0 ? j - 1 : 0)] : o)
+                              : (j < RV - 1 ? f[RV * i + (j < RV - 1 ? j + 1 : 0)] : o);
   }
-  else
-  {
-    const R ca1 = tabv (p, c, 0, x, y), sq1 = tabv (p, c, 1, x, y);
-    const R p5 = tabv (p, c, 2, x, y), q5 = tabv (p, c, 3, x, y);
-    const R g4p = tabv (p, c, 4, x, y), g4m = tabv (p, c, 5, x, y);
-    const R xo = ld (X + id);
-    const R xn = ca1 * xo + sq1 * cu;
-    X[id] = xn;
-    dfdm = (g4p * xn - g4m * xo) * q5;
-    f = p5 * f + (g4p * xn - g4m * xo) * q5 * im;
-  }
-  F[id] = f;
-  return dfdm;
 }
-
-__device__ __forceinline__ void kahan_add (double &s, double &c, double v)
+template <typename R, int RU, int RV, int D>
+__device__ __forceinline__ void adj_far_x (const R f[RU * RV], R far[RU * RV], const R *row, int w, int lane)
 {
-  const double t = s + v;
-  if (fabs (s) >= fabs (v))
-    c += (s - t) + v;
-  else
-    c += (v - t) + s;
-  s = t;
-}
-
-// sum over the probe of Ez^2 by one CTA (the result is valid in thread 0);
-// the probe values are optionally kept
-template <typename R>
-__device__ double probe_sum (const AdjDev<R> &p, const R *Ez, double *keep)
-{
-  __shared__ double part[kThreads / 32];
-  const int w = p.pr_hi[1] - p.pr_lo[1];
-  const int n = (p.pr_hi[0] - p.pr_lo[0]) * w;
-  double s = 0.0;
-  for (int t = threadIdx.x; t < n; t += blockDim.x)
+  const int nb = D < 0 ? max (w - 1, 0) : min (w + 1, 15);
+#pragma unroll
+  for (int j = 0; j < RV; ++j)
   {
-    const int x = p.pr_lo[0] + t / w, y = p.pr_lo[1] + t % w;
-    const double v = (double) ld (Ez + x * p.ny + y);
-    if (keep)
-      keep[t] = v;
-    s += v * v;
+    const R o = row[nb * 32 * RV + RV * lane + j];
+#pragma unroll
+    for (int i = 0; i < RU; ++i)
+      far[RV * i + j] = D < 0 ? (i > 0 ? f[RV * (i > 0 ? i - 1 : 0) + j] : o)
+                              : (i < RU - 1 ? f[RV * (i < RU - 1 ? i + 1 : 0) + j] : o);
   }
-  for (int o = 16; o > 0; o >>= 1)
-    s += __shfl_down_sync (0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0)
-    part[threadIdx.x >> 5] = s;
-  __syncthreads ();
-  double tot = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int) (blockDim.x >> 5); ++i)
-      tot += part[i];
-  return tot;
+}
+// The row the warp next to this one reads: the last where it looks down, the
+// first where it looks up.
+template <typename R, int RU, int RV, int D>
+__device__ __forceinline__ void adj_publish (const R f[RU * RV], R *row, int w, int lane)
+{
+#pragma unroll
+  for (int j = 0; j < RV; ++j)
+    row[w * 32 * RV + RV * lane + j] = f[RV * (D < 0 ? RU - 1 : 0) + j];
 }
 
 // ---- forward group
 
-template <typename R>
-__device__ void forward_part (const Launch<R> &L, int cta, int ctas)
+// Component c's update on a thread's cells given their curls; d gets dF/d(im).
+template <typename R, int RU, int RV>
+__device__ __forceinline__ void adj_update (const R *T, int c, const AdjCells<R, RU, RV> &cells, R S,
+                                            const R cu[RU * RV], const R *im, R f[RU * RV], R x[RU * RV], R d[RU * RV])
 {
+  using G = AdjTile<R, RU, RV>;
+  if (!__any_sync (0xffffffffu, cells.pml[c]))
+  {
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+    {
+      d[r] = S * cu[r];
+      f[r] = (cells.upd >> r) & 1u ? f[r] + S * (im ? im[r] : R (1)) * cu[r] : f[r];
+    }
+    return;
+  }
+  const AdjCoef<R, RU, RV> k (T, G::TM, c, RU * cells.w, RV * cells.lane);
+#pragma unroll
+  for (int r = 0; r < G::C; ++r)
+  {
+    const R m = im ? im[r] : R (1);
+    const R xn = k.at (c, 0, r) * x[r] + k.at (c, 1, r) * cu[r];
+    const R pd = (k.at (c, 4, r) * xn - k.at (c, 5, r) * x[r]) * k.at (c, 3, r);
+    const R pf = k.at (c, 2, r) * f[r] + pd * m, nf = f[r] + S * m * cu[r];
+    const bool pm = (cells.pml[c] >> r) & 1u, up = (cells.upd >> r) & 1u;
+    d[r] = pm ? pd : S * cu[r];
+    f[r] = pm ? pf : (up ? nf : f[r]);
+    x[r] = pm ? xn : x[r];
+  }
+}
+
+// Steps k0 .. k0 + steps - 1 of one tile, from `in` to `out`.
+template <typename R, int RU, int RV>
+__device__ void forward_tile (const Launch<R> &L, const R *in, R *out, int tu, int tv, uint32_t k0, int steps, R *S,
+                              double *s_sum)
+{
+  using G = AdjTile<R, RU, RV>;
   const AdjDev<R> &p = L.p;
-  const int N = L.N;
-  const int tid = cta * blockDim.x + threadIdx.x, stride = ctas * blockDim.x;
-  unsigned *bar = L.bar;
-  R *Ez = L.F[0], *Hx = L.F[1], *Hy = L.F[2], *Xz = L.F[3], *Xx = L.F[4], *Xy = L.F[5];
-  const R *Fc[3] = {Ez, Hx, Hy};
-  if (L.load)
+  const size_t N = L.N;
+  const int u0 = tu * G::OU - kRound, v0 = tv * G::OV - kRound;
+  R *const ERow = S, *const HRow = S + G::A, *const T = S + 2 * G::A;
+  const AdjCells<R, RU, RV> c (p, u0, v0);
+  R f[3][G::C], x[3][G::C], im[G::C];
+#pragma unroll
+  for (int r = 0; r < G::C; ++r)
   {
-    for (int i = tid; i < N; i += stride)
-      for (int q = 0; q < 6; ++q)
-        L.F[q][i] = L.load[(size_t) q * N + i];
-    if (!group_barrier (bar, ctas, L.err, L.limit_ns))
-      return;
+    const bool v = (c.valid >> r) & 1u;
+    const int id = v ? c.id (p, r) : 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+    {
+      f[q][r] = v ? ld (in + q * N + id) : R (0);
+      x[q][r] = (c.pml[q] >> r) & 1u ? ld (in + (3 + q) * N + id) : R (0);
+    }
+    im[r] = (c.upd >> r) & 1u ? p.im[id] : R (0);
   }
-  const bool accum = L.acc && cta == 0 && threadIdx.x == 0;
-  double js = 0.0, jc = 0.0;
-  if (accum)
+  adj_tables<R, RU, RV> (p, T, u0, v0);
+  if (L.ck && k0 % L.every == 0)
   {
-    js = L.acc[0];
-    jc = L.acc[1];
+    R *const save = L.ck + (size_t) (k0 / L.every) * 6 * N;
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      if ((c.own >> r) & 1u)
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+        {
+          save[q * N + c.id (p, r)] = f[q][r];
+          save[(3 + q) * N + c.id (p, r)] = x[q][r];
+        }
   }
-  for (uint32_t k = L.fk0; k < L.fk1; ++k)
+  const bool probe = u0 + kRound < p.pr_hi[0] && u0 + kRound + G::OU > p.pr_lo[0] && v0 + kRound < p.pr_hi[1] &&
+                     v0 + kRound + G::OV > p.pr_lo[1];
+  // Ez reads Hy one row lower, Hy reads Ez one row higher
+  adj_publish<R, RU, RV, -1> (f[2], HRow, c.w, c.lane);
+  __syncthreads ();
+#pragma unroll 1
+  for (int s = 0; s < steps; ++s)
   {
-    const bool upd = k > 0;
+    const uint32_t k = k0 + s;
     const bool kept = L.dedm && k >= L.keep0;
-    R *dd = kept ? L.dedm + (size_t) (k - L.keep0) * N : nullptr;
-    R *save = (L.ck && k % L.every == 0) ? L.ck + (size_t) (k / L.every) * 6 * N : nullptr;
-    // E half-step (and the checkpoint of the state before it)
-    for (int i = tid; i < N; i += stride)
+    R *const dd = kept ? L.dedm + (size_t) (k - L.keep0) * N : nullptr;
+    double sum = 0.0;
+    R cu[G::C], d[G::C];
+    if (k > 0)
     {
-      if (save)
-        for (int q = 0; q < 6; ++q)
-          save[(size_t) q * N + i] = ld (L.F[q] + i);
-      const int x = i / p.ny, y = i % p.ny;
-      if (!updated (p, x, y))
-        continue;
-      R d = 0;
-      if (upd)
-        d = update_cell (p, kEz, Ez, Xz, curl_of (p, kEz, Fc, x, y), p.im[i], x, y);
-      if (p.ps_on[kEz] && x == p.ps[0] && y == p.ps[1])
-        Ez[i] = p.src[2 * k];
-      if (dd)
-        dd[i] = d;
+      R a[G::C], b[G::C];
+      adj_far_x<R, RU, RV, -1> (f[2], a, HRow, c.w, c.lane);
+      adj_far_y<R, RU, RV, -1> (f[1], b);
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        cu[r] = (f[2][r] - a[r]) - (f[1][r] - b[r]);
+      adj_update<R, RU, RV> (T, kEz, c, p.S, cu, im, f[0], x[0], d);
     }
-    if (!group_barrier (bar, ctas, L.err, L.limit_ns))
-      return;
-    // probe term of Ez_k, then the H half-step
-    if (cta == 0 && (L.acc || kept))
+    else
     {
-      const double v = probe_sum (p, Ez, kept ? L.keep + (size_t) (k - L.keep0) * L.npr : nullptr);
-      if (accum)
-        kahan_add (js, jc, v);
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        d[r] = 0;
     }
-    for (int i = tid; i < N; i += stride)
+    if (p.ps_on[kEz] && c.source)
     {
-      const int x = i / p.ny, y = i % p.ny;
-      if (!updated (p, x, y))
-        continue;
-      if (upd)
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        if ((c.source >> r) & 1u)
+          f[0][r] = p.src[2 * k];
+    }
+    if (dd)
+    {
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        if ((c.own & c.upd) >> r & 1u)
+          dd[c.id (p, r)] = d[r];
+    }
+    if (probe)
+    {
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
       {
-        const R cx = curl_of (p, kHx, Fc, x, y), cy = curl_of (p, kHy, Fc, x, y);
-        update_cell (p, kHx, Hx, Xx, cx, R (1), x, y);
-        update_cell (p, kHy, Hy, Xy, cy, R (1), x, y);
-      }
-      if (x == p.ps[0] && y == p.ps[1])
-      {
-        if (p.ps_on[kHx])
-          Hx[i] = p.src[2 * k + 1];
-        if (p.ps_on[kHy])
-          Hy[i] = p.src[2 * k + 1];
+        const int a = u0 + c.du (r) - p.pr_lo[0], b = v0 + c.dv (r) - p.pr_lo[1], n = p.pr_hi[1] - p.pr_lo[1];
+        if (((c.own & c.upd) >> r & 1u) && a >= 0 && a < p.pr_hi[0] - p.pr_lo[0] && b >= 0 && b < n)
+        {
+          const double v = (double) f[0][r];
+          sum += v * v;
+          if (kept)
+            L.keep[(size_t) (k - L.keep0) * L.npr + a * n + b] = v;
+        }
       }
     }
-    if (!group_barrier (bar, ctas, L.err, L.limit_ns))
-      return;
+    adj_publish<R, RU, RV, 1> (f[0], ERow, c.w, c.lane);
+    __syncthreads ();
+    if (probe && L.jpart)
+    {
+      for (int o = 16; o > 0; o >>= 1)
+        sum += __shfl_down_sync (0xffffffffu, sum, o);
+      if (c.lane == 0)
+        s_sum[c.w] = sum;
+    }
+    if (k > 0)
+    {
+      adj_far_y<R, RU, RV, 1> (f[0], cu);
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        cu[r] = f[0][r] - cu[r];
+      adj_update<R, RU, RV> (T, kHx, c, p.S, cu, nullptr, f[1], x[1], d);
+      adj_far_x<R, RU, RV, 1> (f[0], cu, ERow, c.w, c.lane);
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        cu[r] = cu[r] - f[0][r];
+      adj_update<R, RU, RV> (T, kHy, c, p.S, cu, nullptr, f[2], x[2], d);
+    }
+    if (c.source)
+    {
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        if ((c.source >> r) & 1u)
+        {
+          if (p.ps_on[kHx])
+            f[1][r] = p.src[2 * k + 1];
+          if (p.ps_on[kHy])
+            f[2][r] = p.src[2 * k + 1];
+        }
+    }
+    adj_publish<R, RU, RV, -1> (f[2], HRow, c.w, c.lane);
+    __syncthreads ();
+    if (probe && L.jpart && threadIdx.x == 0)
+    {
+      double tot = 0.0;
+      for (int q = 0; q < kThreads / 32; ++q)
+        tot += s_sum[q];
+      L.jpart[(size_t) k * L.nprt + (tu - L.prt_u0) * L.prt_nv + (tv - L.prt_v0)] = tot;
+    }
   }
-  if (accum)
+#pragma unroll
+  for (int r = 0; r < G::C; ++r)
+    if ((c.own & c.upd) >> r & 1u)
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+      {
+        out[q * N + c.id (p, r)] = f[q][r];
+        if ((c.pml[q] >> r) & 1u)
+          out[(3 + q) * N + c.id (p, r)] = x[q][r];
+      }
+}
+
+template <typename R, int RU, int RV>
+__device__ void forward_part (const Launch<R> &L, int cta, int ctas, R *S, double *s_sum)
+{
+  const R *in = L.load ? L.load : L.F[0];
+  int to = 1;
+  for (uint32_t k = L.fk0; k < L.fk1;)
   {
-    L.acc[0] = js;
-    L.acc[1] = jc;
+    // a round ends where a checkpoint is taken
+    uint32_t end = min (k + (uint32_t) kRound, L.fk1);
+    if (L.ck)
+      end = min (end, (k / L.every + 1) * L.every);
+    for (int t = cta; t < L.tiles_u * L.tiles_v; t += ctas)
+    {
+      __syncthreads ();   // (the shared arrays of the previous tile have been used)
+      forward_tile<R, RU, RV> (L, in, L.F[to], t / L.tiles_v, t % L.tiles_v, k, (int) (end - k), S, s_sum);
+    }
+    if (!group_barrier (L.bar, ctas, L.err, L.limit_ns))
+      return;
+    in = L.F[to];
+    to ^= 1;
+    k = end;
   }
 }
 
 // ---- reverse group
 
-// H phase at H cell t: gather acz, transpose of the H update and H source
-template <typename R>
-__device__ __forceinline__ void adj_h_cell (const Launch<R> &L, int t)
+// Transpose of component c's update on a thread's cells: a = the adjoint of F
+// (in: gathered, out: of the old F), ax of X; cu gets the adjoint of the curl
+// (0 on cells that are not updated).
+template <typename R, int RU, int RV>
+__device__ __forceinline__ void adj_transpose (const R *T, int c, const AdjCells<R, RU, RV> &cells, R S, const R *im,
+                                               R a[RU * RV], R ax[RU * RV], R cu[RU * RV])
 {
-  const AdjDev<R> &p = L.p;
-  const int x = t / p.ny, y = t % p.ny;
-  // Ez's curl reads H comp o at e + d: the H cell (x, y) is read by e = (x, y) - d
-  auto take = [&] (const int d[2], R sgn) -> R {
-    const int ex = x - d[0], ey = y - d[1];
-    return updated (p, ex, ey) ? sgn * ld (L.acz + ex * p.ny + ey) : R (0);
-  };
-  R g[2] = {0, 0};
-#pragma unroll
-  for (int q = 0; q < 2; ++q)
+  using G = AdjTile<R, RU, RV>;
+  if (!__any_sync (0xffffffffu, cells.pml[c]))
   {
-    const int slot = q ? kHy : kHx;
-    if (p.o1[kEz] == slot)
-      g[q] += take (p.d12[kEz], R (1)) + take (p.d11[kEz], R (-1));
-    if (p.o2[kEz] == slot)
-      g[q] += take (p.d22[kEz], R (-1)) + take (p.d21[kEz], R (1));
-  }
-  if (!updated (p, x, y))
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      cu[r] = (cells.upd >> r) & 1u ? S * (im ? im[r] : R (1)) * a[r] : R (0);
     return;
-  const bool at_src = x == p.ps[0] && y == p.ps[1];
+  }
+  const AdjCoef<R, RU, RV> k (T, G::TM, c, RU * cells.w, RV * cells.lane);
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
+  for (int r = 0; r < G::C; ++r)
   {
-    const int c = q ? kHy : kHx;
-    R *aH = q ? L.aHy : L.aHx;
-    R *aX = q ? L.aXy : L.aXx;
-    R a = ld (aH + t) + g[q];
-    if (at_src && p.ps_on[c])
-      a = 0;
-    R acu;
-    if (interior (p, c, x, y))
-    {
-      acu = p.S * a;
-      aH[t] = a;
-    }
-    else
-    {
-      const R ca1 = tabv (p, c, 0, x, y), sq1 = tabv (p, c, 1, x, y);
-      const R p5 = tabv (p, c, 2, x, y), q5 = tabv (p, c, 3, x, y);
-      const R g4p = tabv (p, c, 4, x, y), g4m = tabv (p, c, 5, x, y);
-      const R t1 = ld (aX + t) + g4p * q5 * a;
-      acu = sq1 * t1;
-      aX[t] = ca1 * t1 - g4m * q5 * a;
-      aH[t] = p5 * a;
-    }
-    (q ? L.acy : L.acx)[t] = acu;
+    const R m = im ? im[r] : R (1);
+    const bool pm = (cells.pml[c] >> r) & 1u, up = (cells.upd >> r) & 1u;
+    const R t1 = ax[r] + k.at (c, 4, r) * k.at (c, 3, r) * m * a[r];
+    const R nx = k.at (c, 0, r) * t1 - k.at (c, 5, r) * k.at (c, 3, r) * m * a[r];
+    cu[r] = pm ? k.at (c, 1, r) * t1 : (up ? S * m * a[r] : R (0));
+    ax[r] = pm ? nx : ax[r];
+    a[r] = pm ? k.at (c, 2, r) * a[r] : a[r];
   }
 }
 
-// E phase at Ez cell t: gather acx, acy, probe term, gradient of im,
-// transpose of the E update and E source
-template <typename R>
-__device__ __forceinline__ void adj_e_cell (const Launch<R> &L, int t, const R *dedm, const double *probe)
+// Reverse steps k1 - 1 down to k1 - steps (all > 0) of one tile.  Ez at (x, y)
+// reads Hx at y and y - 1 and Hy at x and x - 1, Hx reads Ez at y and y + 1, Hy
+// at x and x + 1: the gathers below are their transposes.
+template <typename R, int RU, int RV>
+__device__ void reverse_tile (const Launch<R> &L, const R *in, R *out, int tu, int tv, uint32_t k1, int steps, R *S)
 {
+  using G = AdjTile<R, RU, RV>;
   const AdjDev<R> &p = L.p;
-  const int x = t / p.ny, y = t % p.ny;
-  if (!updated (p, x, y))
-    return;
-  R g = 0;
+  const size_t N = L.N;
+  const int u0 = tu * G::OU - kRound, v0 = tv * G::OV - kRound;
+  R *const ZRow = S, *const YRow = S + G::A, *const T = S + 2 * G::A;
+  const AdjCells<R, RU, RV> c (p, u0, v0);
+  R aE[G::C], aH[2][G::C], ax[3][G::C], z[G::C], im[G::C];
+  double gim[G::C];
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
+  for (int r = 0; r < G::C; ++r)
   {
-    const int c = q ? kHy : kHx;
-    const R *acu = q ? L.acy : L.acx;
-    // H cell h reads Ez at h + d: the Ez cell (x, y) is read by h = (x, y) - d
-    auto take = [&] (const int d[2], R sgn) {
-      const int hx = x - d[0], hy = y - d[1];
-      if (updated (p, hx, hy))
-        g += sgn * ld (acu + hx * p.ny + hy);
-    };
-    if (p.o1[c] == kEz)
-    {
-      take (p.d12[c], R (1));
-      take (p.d11[c], R (-1));
-    }
-    if (p.o2[c] == kEz)
-    {
-      take (p.d22[c], R (-1));
-      take (p.d21[c], R (1));
-    }
+    const bool up = (c.upd >> r) & 1u;
+    const int id = up ? c.id (p, r) : 0;
+    aE[r] = up ? ld (in + id) : R (0);
+    aH[0][r] = up ? ld (in + 2 * N + id) : R (0);
+    aH[1][r] = up ? ld (in + 3 * N + id) : R (0);
+    ax[kEz][r] = (c.pml[kEz] >> r) & 1u ? ld (in + N + id) : R (0);
+    ax[kHx][r] = (c.pml[kHx] >> r) & 1u ? ld (in + 4 * N + id) : R (0);
+    ax[kHy][r] = (c.pml[kHy] >> r) & 1u ? ld (in + 5 * N + id) : R (0);
+    z[r] = up ? ld (in + 6 * N + id) : R (0);
+    im[r] = up ? p.im[id] : R (0);
+    gim[r] = up && ((c.own >> r) & 1u) ? L.gim[id] : 0.0;
   }
-  R a = ld (L.aE + t) + g;
-  if (x >= p.pr_lo[0] && x < p.pr_hi[0] && y >= p.pr_lo[1] && y < p.pr_hi[1])
-    a += (R) (2.0 * probe[(x - p.pr_lo[0]) * (p.pr_hi[1] - p.pr_lo[1]) + (y - p.pr_lo[1])]);
-  if (x == p.ps[0] && y == p.ps[1] && p.ps_on[kEz])
-    a = 0;
-  L.gim[t] += (double) a * (double) dedm[t];
-  const R im = p.im[t];
-  if (interior (p, kEz, x, y))
+  adj_tables<R, RU, RV> (p, T, u0, v0);
+  adj_publish<R, RU, RV, 1> (z, ZRow, c.w, c.lane);
+  // probe cells of the thread
+  unsigned probed = 0;
+  const int pw = p.pr_hi[1] - p.pr_lo[1];
+#pragma unroll
+  for (int r = 0; r < G::C; ++r)
   {
-    L.acz[t] = p.S * im * a;
-    L.aE[t] = a;
+    const int x = u0 + c.du (r), y = v0 + c.dv (r);
+    probed |= ((c.upd >> r) & 1u) && x >= p.pr_lo[0] && x < p.pr_hi[0] && y >= p.pr_lo[1] && y < p.pr_hi[1] ? 1u << r : 0u;
   }
-  else
+  __syncthreads ();
+#pragma unroll 1
+  for (int s = 0; s < steps; ++s)
   {
-    const R ca1 = tabv (p, kEz, 0, x, y), sq1 = tabv (p, kEz, 1, x, y);
-    const R p5 = tabv (p, kEz, 2, x, y), q5 = tabv (p, kEz, 3, x, y);
-    const R g4p = tabv (p, kEz, 4, x, y), g4m = tabv (p, kEz, 5, x, y);
-    const R t1 = ld (L.aXz + t) + g4p * q5 * im * a;
-    L.acz[t] = sq1 * t1;
-    L.aXz[t] = ca1 * t1 - g4m * q5 * im * a;
-    L.aE[t] = p5 * a;
+    const uint32_t k = k1 - 1 - s;
+    const R *const dedm = L.rdedm + (size_t) (k - L.rk0) * N;
+    const double *const probe = L.rprobe + (size_t) (k - L.rk0) * L.npr;
+    R far[G::C], cx[G::C], cy[G::C], dm[G::C];
+    // (needed after the H phase: the loads are under way meanwhile)
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      dm[r] = (c.own & c.upd) >> r & 1u ? ld (dedm + c.id (p, r)) : R (0);
+    adj_far_y<R, RU, RV, 1> (z, far);
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      aH[0][r] = (c.upd >> r) & 1u ? aH[0][r] + (-z[r] + far[r]) : R (0);
+    adj_far_x<R, RU, RV, 1> (z, far, ZRow, c.w, c.lane);
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      aH[1][r] = (c.upd >> r) & 1u ? aH[1][r] + (z[r] - far[r]) : R (0);
+    if (c.source)
+    {
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        if ((c.source >> r) & 1u)
+        {
+          aH[0][r] = p.ps_on[kHx] ? R (0) : aH[0][r];
+          aH[1][r] = p.ps_on[kHy] ? R (0) : aH[1][r];
+        }
+    }
+    adj_transpose<R, RU, RV> (T, kHx, c, p.S, nullptr, aH[0], ax[kHx], cx);
+    adj_transpose<R, RU, RV> (T, kHy, c, p.S, nullptr, aH[1], ax[kHy], cy);
+    adj_publish<R, RU, RV, -1> (cy, YRow, c.w, c.lane);
+    __syncthreads ();
+    adj_far_y<R, RU, RV, -1> (cx, far);
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      cx[r] = cx[r] - far[r];
+    adj_far_x<R, RU, RV, -1> (cy, far, YRow, c.w, c.lane);
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      aE[r] = (c.upd >> r) & 1u ? aE[r] + ((cx[r] + far[r]) - cy[r]) : R (0);
+    if (probed)
+    {
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        if ((probed >> r) & 1u)
+          aE[r] += (R) (2.0 * __ldcg (probe + (u0 + c.du (r) - p.pr_lo[0]) * pw + (v0 + c.dv (r) - p.pr_lo[1])));
+    }
+    if (p.ps_on[kEz] && c.source)
+    {
+#pragma unroll
+      for (int r = 0; r < G::C; ++r)
+        if ((c.source >> r) & 1u)
+          aE[r] = 0;
+    }
+#pragma unroll
+    for (int r = 0; r < G::C; ++r)
+      gim[r] += (double) aE[r] * (double) dm[r];
+    adj_transpose<R, RU, RV> (T, kEz, c, p.S, im, aE, ax[kEz], z);
+    adj_publish<R, RU, RV, 1> (z, ZRow, c.w, c.lane);
+    __syncthreads ();
+  }
+#pragma unroll
+  for (int r = 0; r < G::C; ++r)
+    if ((c.own & c.upd) >> r & 1u)
+    {
+      const int id = c.id (p, r);
+      out[id] = aE[r];
+      out[2 * N + id] = aH[0][r];
+      out[3 * N + id] = aH[1][r];
+      out[6 * N + id] = z[r];
+      if ((c.pml[kEz] >> r) & 1u)
+        out[N + id] = ax[kEz][r];
+      if ((c.pml[kHx] >> r) & 1u)
+        out[4 * N + id] = ax[kHx][r];
+      if ((c.pml[kHy] >> r) & 1u)
+        out[5 * N + id] = ax[kHy][r];
+      L.gim[id] = gim[r];
+    }
+}
+
+// Rounds of the reverse steps rk1 - 1 .. max (rk0, 1): the set changes with
+// each.
+__host__ __device__ inline int reverse_rounds (uint32_t rk0, uint32_t rk1)
+{
+  const uint32_t lo = rk0 > 1 ? rk0 : 1;
+  return rk1 > lo ? (int) ((rk1 - lo + kRound - 1) / kRound) : 0;
+}
+
+template <typename R, int RU, int RV>
+__device__ void reverse_part (const Launch<R> &L, int cta, int ctas, R *S)
+{
+  int cur = L.rcur;
+  const uint32_t lo = L.rk0 > 1 ? L.rk0 : 1;
+  for (uint32_t k = L.rk1; k > lo;)
+  {
+    const int steps = (int) min ((uint32_t) kRound, k - lo);
+    for (int t = cta; t < L.tiles_u * L.tiles_v; t += ctas)
+    {
+      __syncthreads ();
+      reverse_tile<R, RU, RV> (L, L.A[cur], L.A[cur ^ 1], t / L.tiles_v, t % L.tiles_v, k, steps, S);
+    }
+    if (!group_barrier (L.bar + kBarStride, ctas, L.err, L.limit_ns))
+      return;
+    cur ^= 1;
+    k -= steps;
   }
 }
 
-template <typename R>
-__device__ void reverse_part (const Launch<R> &L, int cta, int ctas)
+template <typename R, int RU, int RV>
+__global__ void __launch_bounds__ (kThreads, 1) adjoint_kernel (const __grid_constant__ Launch<R> L)
 {
-  const int N = L.N;
-  const int tid = cta * blockDim.x + threadIdx.x, stride = ctas * blockDim.x;
-  unsigned *bar = L.bar + kBarStride;
-  for (int64_t k = (int64_t) L.rk1 - 1; k >= (int64_t) L.rk0 && k > 0; --k)
-  {
-    const size_t off = (size_t) (k - L.rk0);
-    for (int t = tid; t < N; t += stride)
-      adj_h_cell (L, t);
-    if (!group_barrier (bar, ctas, L.err, L.limit_ns))
-      return;
-    const R *dedm = L.rdedm + off * N;
-    const double *probe = L.rprobe + off * L.npr;
-    for (int t = tid; t < N; t += stride)
-      adj_e_cell (L, t, dedm, probe);
-    if (!group_barrier (bar, ctas, L.err, L.limit_ns))
-      return;
-  }
-}
-
-template <typename R>
-__global__ void __launch_bounds__ (kThreads) adjoint_kernel (Launch<R> L)
-{
+  extern __shared__ __align__ (16) unsigned char adj_smem[];
+  __shared__ double s_sum[kThreads / 32];
+  R *const S = reinterpret_cast<R *> (adj_smem);
   if ((int) blockIdx.x < L.fwd_ctas)
-    forward_part (L, blockIdx.x, L.fwd_ctas);
+    forward_part<R, RU, RV> (L, blockIdx.x, L.fwd_ctas, S, s_sum);
   else
-    reverse_part (L, blockIdx.x - L.fwd_ctas, gridDim.x - L.fwd_ctas);
+    reverse_part<R, RU, RV> (L, blockIdx.x - L.fwd_ctas, gridDim.x - L.fwd_ctas, S);
+}
+
+// Compensated sum of n doubles (one block of 256).
+__global__ void adj_sum_kernel (const double *v, size_t n, double *acc)
+{
+  __shared__ double ss[256], sc[256];
+  auto add = [] (double &s, double &c, double y) {
+    const double t = s + y, z = t - s;
+    c += (s - (t - z)) + (y - z);
+    s = t;
+  };
+  double s = 0.0, c = 0.0;
+  for (size_t i = threadIdx.x; i < n; i += 256)
+    add (s, c, v[i]);
+  ss[threadIdx.x] = s;
+  sc[threadIdx.x] = c;
+  __syncthreads ();
+  for (int o = 128; o > 0; o >>= 1)
+  {
+    if ((int) threadIdx.x < o)
+    {
+      add (ss[threadIdx.x], sc[threadIdx.x], ss[threadIdx.x + o]);
+      sc[threadIdx.x] += sc[threadIdx.x + o];
+    }
+    __syncthreads ();
+  }
+  if (threadIdx.x == 0)
+  {
+    acc[0] = ss[0];
+    acc[1] = sc[0];
+  }
 }
 
 // dJ/d eps from dJ/d im (gather over the Ez cells that average the cell)
@@ -592,24 +830,42 @@ struct Arena
   }
 };
 
-int local_slot (int k)
+// The kernel of a tile size (64: 64 x 64 cells in FP32, 64 x 32 in FP64; else
+// 32 x 32), its own cells per tile and shared memory.
+template <typename R>
+const void *adjoint_pick (int tile, int &ou, int &ov, int &smem)
 {
-  return k == EZ ? kEz : (k == HX ? kHx : (k == HY ? kHy : -1));
+  constexpr int CV = sizeof (R) == 4 ? 2 : 1;
+  if (tile == 64)
+  {
+    using G = AdjTile<R, 4, CV>;
+    ou = G::OU;
+    ov = G::OV;
+    smem = G::BYTES;
+    return (const void *) adjoint_kernel<R, 4, CV>;
+  }
+  using G = AdjTile<R, 2, 1>;
+  ou = G::OU;
+  ov = G::OV;
+  smem = G::BYTES;
+  return (const void *) adjoint_kernel<R, 2, 1>;
 }
 
 template <typename R>
-cudaError_t launch (const Launch<R> &L, int ctas, cudaStream_t s)
+cudaError_t launch (const Launch<R> &L, const void *kern, int smem, int ctas, cudaStream_t s)
 {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3 (ctas);
   lc.blockDim = dim3 (kThreads);
+  lc.dynamicSmemBytes = smem;
   lc.stream = s;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeCooperative;
   attr.val.cooperative = 1;
   lc.attrs = &attr;
   lc.numAttrs = 1;
-  return cudaLaunchKernelEx (&lc, adjoint_kernel<R>, L);
+  void *args[] = {(void *) &L};
+  return cudaLaunchKernelExC (&lc, kern, args);
 }
 
 template <typename R>
@@ -633,18 +889,19 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
       return "probe box outside the updated cells";
   const int npr = (run.probe_hi[0] - run.probe_lo[0]) * (run.probe_hi[1] - run.probe_lo[1]);
 
-  // co-resident CTAs of the cooperative kernel (at most three per SM: each
-  // half-step is latency-bound, so more resident threads help)
+  // 32 x 32 tiles while half of the SMs (one group) hold them at once, else
+  // the large ones, whose halo is a smaller share
+  int ou = 0, ov = 0, smem = 0;
+  const void *kern = adjoint_pick<R> (32, ou, ov, smem);
+  if ((int64_t) ((nx + ou - 1) / ou) * ((ny + ov - 1) / ov) > sm_count / 2)
+    kern = adjoint_pick<R> (64, ou, ov, smem);
+  const int tiles_u = (nx + ou - 1) / ou, tiles_v = (ny + ov - 1) / ov;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, adjoint_kernel<R>, kThreads, 0) != cudaSuccess ||
-      per_sm < 1)
+  if (cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor (&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
     return "the adjoint kernel does not fit on an SM";
-  // 3 CTAs per SM and an even split between the reversing and the
-  // recomputing group measured fastest
-  const int cap = 3;
-  const int ctas = sm_count * std::min (per_sm, cap);
-  const double split = 0.5;
-  const int fwd_split = std::max (1, std::min (ctas - 1, (int) std::lround (ctas * split)));
+  const int ctas = sm_count;
+  const int fwd_split = std::max (1, ctas / 2);
 
   AdjDev<R> p{};
   p.nx = nx;
@@ -659,15 +916,6 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   {
     const int k = kmap[c];
     const CompLayout &CL = g.comp[k];
-    p.o1[c] = g.comp[CL.opp1].exists ? local_slot (CL.opp1) : -1;
-    p.o2[c] = g.comp[CL.opp2].exists ? local_slot (CL.opp2) : -1;
-    for (int a = 0; a < 2; ++a)
-    {
-      p.d11[c][a] = CL.d11[a];
-      p.d12[c][a] = CL.d12[a];
-      p.d21[c][a] = CL.d21[a];
-      p.d22[c][a] = CL.d22[a];
-    }
     const int axes[3] = {CL.sig_cacb, CL.sig5, CL.sig4};
     for (int q = 0; q < 3; ++q)
       p.tax[c][q] = axes[q];
@@ -738,7 +986,12 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   for (const auto &v : tabs)
     i_tab.push_back (ar.reserve<R> (v.size ()));
   const int i_src = ar.reserve<R> (src.size ());
-  const int i_state = ar.reserve<R> (6 * N);
+  const int i_state = ar.reserve<R> (12 * N);
+  // probe tiles, and a sum per step and probe tile
+  const int pt_u0 = run.probe_lo[0] / ou, pt_u1 = (run.probe_hi[0] - 1) / ou;
+  const int pt_v0 = run.probe_lo[1] / ov, pt_v1 = (run.probe_hi[1] - 1) / ov;
+  const int nprt = (pt_u1 - pt_u0 + 1) * (pt_v1 - pt_v0 + 1);
+  const int i_jpart = ar.reserve<double> ((size_t) run.steps * nprt);
   const int i_im = ar.reserve<R> (N);
   const int i_imd = ar.reserve<double> (N);
   const int i_acc = ar.reserve<double> (2);
@@ -753,7 +1006,7 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
       i_dedm[b] = ar.reserve<R> ((size_t) K * N);
       i_probe[b] = ar.reserve<double> ((size_t) K * npr);
     }
-    i_adj = ar.reserve<R> (9 * N);
+    i_adj = ar.reserve<R> (14 * N);
     i_gim = ar.reserve<double> (N);
     i_gout = ar.reserve<double> (N);
   }
@@ -776,7 +1029,7 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   double *acc = ar.at<double> (i_acc);
   unsigned *bar = ar.at<unsigned> (i_bar);
   int *err = ar.at<int> (i_err);
-  if (cudaMemsetAsync (state, 0, 6 * N * sizeof (R), s) != cudaSuccess ||
+  if (cudaMemsetAsync (state, 0, 12 * N * sizeof (R), s) != cudaSuccess ||
       cudaMemsetAsync (acc, 0, 2 * sizeof (double), s) != cudaSuccess ||
       cudaMemsetAsync (bar, 0, 2 * kBarStride * sizeof (unsigned), s) != cudaSuccess ||
       cudaMemsetAsync (err, 0, sizeof (int), s) != cudaSuccess)
@@ -798,15 +1051,21 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   L.bar = bar;
   L.err = err;
   L.limit_ns = run.wait_limit_ns > 0 ? run.wait_limit_ns : kDefaultBarrierLimitNs;
-  for (int q = 0; q < 6; ++q)
-    L.F[q] = state + (size_t) q * N;
+  L.F[0] = state;
+  L.F[1] = state + 6 * N;
+  L.tiles_u = tiles_u;
+  L.tiles_v = tiles_v;
+  L.prt_u0 = pt_u0;
+  L.prt_v0 = pt_v0;
+  L.prt_nv = pt_v1 - pt_v0 + 1;
+  L.nprt = nprt;
 
   // forward run: checkpoints, and the per-step data of the last segment
   const uint32_t last0 = (nck - 1) * K;
   L.fwd_ctas = ctas;
   L.fk0 = 0;
   L.fk1 = run.steps;
-  L.acc = acc;
+  L.jpart = ar.at<double> (i_jpart);
   L.every = K;
   if (grad)
   {
@@ -815,8 +1074,9 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
     L.keep = ar.at<double> (i_probe[0]);
     L.keep0 = last0;
   }
-  if (launch (L, ctas, s) != cudaSuccess)
+  if (launch (L, kern, smem, ctas, s) != cudaSuccess)
     return std::string ("adjoint forward launch failed: ") + cudaGetErrorString (cudaGetLastError ());
+  adj_sum_kernel<<<1, 256, 0, s>>> (L.jpart, (size_t) run.steps * nprt, acc);
   double hacc[2];
   int herr = 0;
   if (cudaMemcpyAsync (hacc, acc, sizeof (hacc), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -834,23 +1094,14 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   // idx & 1 and recomputes segment j - 1 into the other buffer
   R *adj = ar.at<R> (i_adj);
   double *gim = ar.at<double> (i_gim);
-  if (cudaMemsetAsync (adj, 0, 9 * N * sizeof (R), s) != cudaSuccess ||
+  if (cudaMemsetAsync (adj, 0, 14 * N * sizeof (R), s) != cudaSuccess ||
       cudaMemsetAsync (gim, 0, N * sizeof (double), s) != cudaSuccess)
     return "device initialisation failed";
-  R *A[9];
-  for (int q = 0; q < 9; ++q)
-    A[q] = adj + (size_t) q * N;
-  L.aE = A[0];
-  L.aXz = A[1];
-  L.aHx = A[2];
-  L.aHy = A[3];
-  L.aXx = A[4];
-  L.aXy = A[5];
-  L.acx = A[6];
-  L.acy = A[7];
-  L.acz = A[8];
+  L.A[0] = adj;
+  L.A[1] = adj + 7 * N;
+  L.rcur = 0;
   L.gim = gim;
-  L.acc = nullptr;
+  L.jpart = nullptr;
   L.ck = nullptr;
   const R *ck = ar.at<R> (i_ck);
   for (uint32_t idx = 0; idx < nck; ++idx)
@@ -878,8 +1129,9 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
       L.dedm = nullptr;
       L.keep = nullptr;
     }
-    if (launch (L, ctas, s) != cudaSuccess)
+    if (launch (L, kern, smem, ctas, s) != cudaSuccess)
       return std::string ("adjoint reverse launch failed: ") + cudaGetErrorString (cudaGetLastError ());
+    L.rcur ^= reverse_rounds (L.rk0, L.rk1) & 1;
   }
   double *gout = ar.at<double> (i_gout);
   grad_eps_kernel<R><<<blocks, 256, 0, s>>> (p, gim, imd, LE.nmat, LE.m[0][0], LE.m[0][1], LE.m[1][0], LE.m[1][1],
