@@ -201,6 +201,11 @@ struct fdtd_ctx
   int nparts = 0;
 
   std::vector<void *> allocs;
+  // one device allocation that later DALLOCs are carved from while it lasts
+  // (slab_reserve, slab_close): cudaMalloc and cudaFree take 0.2 to 0.6 ms
+  // each, and a context holds 30 to 90 arrays
+  char *slab = nullptr;
+  size_t slab_left = 0;
 
   // field-kernel timing
   bool profiling = false;
@@ -226,8 +231,46 @@ int fail (fdtd_ctx *ctx, int code, const std::string &msg)
                    std::string (#call) + ": " + cudaGetErrorString (e_));                           \
   } while (0)
 
+constexpr size_t slab_size (size_t bytes)
+{
+  return (bytes + 255) & ~(size_t) 255;
+}
+
+// Takes `bytes` (zeroed) from the device in one allocation for the DALLOCs
+// that follow; what does not fit is allocated by itself.
+int slab_reserve (fdtd_ctx *ctx, size_t bytes)
+{
+  ctx->slab_left = 0;
+  void *p = nullptr;
+  cudaError_t e = device_malloc (&p, bytes);
+  if (e != cudaSuccess)
+    return fail (ctx, FDTD_ERR_NOMEM, std::string ("cudaMalloc: ") + cudaGetErrorString (e));
+  ctx->allocs.push_back (p);
+  e = cudaMemsetAsync (p, 0, bytes, ctx->stream);
+  if (e != cudaSuccess)
+    return fail (ctx, FDTD_ERR_CUDA, std::string ("cudaMemset: ") + cudaGetErrorString (e));
+  ctx->slab = (char *) p;
+  ctx->slab_left = bytes;
+  return FDTD_OK;
+}
+
+// The rest of the slab is not handed out any more (later allocations may be
+// freed one by one).
+void slab_close (fdtd_ctx *ctx)
+{
+  ctx->slab_left = 0;
+}
+
 int dalloc (fdtd_ctx *ctx, void **p, size_t bytes, bool zero = true)
 {
+  const size_t need = slab_size (bytes ? bytes : 16);
+  if (need <= ctx->slab_left)
+  {
+    *p = ctx->slab;
+    ctx->slab += need;
+    ctx->slab_left -= need;
+    return FDTD_OK;
+  }
   cudaError_t e = device_malloc (p, bytes ? bytes : 16);
   if (e != cudaSuccess)
   {
@@ -268,6 +311,14 @@ int row_pitch (const Geometry &g, int kind)
   const int unit = kind == 2 ? 8 : 4;
   return (nz + unit - 1) / unit * unit;
 }
+
+#define SLAB(bytes)                                                                                \
+  do                                                                                               \
+  {                                                                                                \
+    int r_ = slab_reserve (ctx, (bytes));                                                          \
+    if (r_ != FDTD_OK)                                                                             \
+      return r_;                                                                                   \
+  } while (0)
 
 GeomDev make_geom_dev (const Geometry &g, int pz)
 {
@@ -424,12 +475,25 @@ int ensure_src (fdtd_ctx *ctx, size_t steps)
 
 PlainHalf plain_half (fdtd_ctx *ctx, int h);
 
+// 2-D modes without metamaterials advance several steps per launch (tile2d).
+bool tile2d_mode (const Geometry &g)
+{
+  return (g.drop == 1 || g.drop == 2 || g.drop == 4) && !g.cfg.use_metamaterials;
+}
+
 int alloc_plain (fdtd_ctx *ctx)
 {
   const Geometry &g = ctx->g;
   size_t nb = (size_t) g.cells * sizeof (double);
+  int family[2] = {0, 0}, comps = 0;
+  for (int k = 0; k < 6; ++k)
+    family[k / 3] += g.comp[k].exists ? 1 : 0;
+  comps = family[0] + family[1];
   for (int k = 0; k < 6; ++k)
   {
+    if (k % 3 == 0)
+      SLAB ((size_t) family[k / 3] * g.levels * (1 + (g.cfg.use_pml ? 1 : 0) + (g.cfg.use_metamaterials ? 1 : 0)) *
+            slab_size (nb));
     if (!g.comp[k].exists)
       continue;
     for (int l = 0; l < g.levels; ++l)
@@ -442,11 +506,16 @@ int alloc_plain (fdtd_ctx *ctx)
     }
   }
   int nmat = g.cfg.use_metamaterials ? 6 : 2;
+  SLAB (nmat * slab_size (nb));
   for (int m = 0; m < nmat; ++m)
   {
     DALLOC (ctx->mat64[m], nb);
     if (m < 2)
       ctx->launches += launch_fill (ctx->mat64[m], (size_t) g.cells, 1.0, ctx->stream);
+  }
+  {
+    const size_t nmax = std::max (g.nf[0], std::max (g.nf[1], g.nf[2]));
+    SLAB ((size_t) (3 + 9 * comps) * slab_size (nmax * sizeof (double)));
   }
   for (int a = 0; a < 3; ++a)
   {
@@ -535,12 +604,6 @@ int upload_fine_material (fdtd_ctx *ctx, int which, const double *src, cudaMemcp
   return FDTD_OK;
 }
 
-// 2-D modes without metamaterials advance several steps per launch (tile2d).
-bool tile2d_mode (const Geometry &g)
-{
-  return (g.drop == 1 || g.drop == 2 || g.drop == 4) && !g.cfg.use_metamaterials;
-}
-
 int alloc_fast (fdtd_ctx *ctx)
 {
   const Geometry &g = ctx->g;
@@ -550,8 +613,12 @@ int alloc_fast (fdtd_ctx *ctx)
   // precision and the 2-D / 1-D modes run the per-cell kernels on one buffer set
   ctx->has_second = g.drop == 0 && g.cfg.layout == 0 && !g.dmp;
   // (the 2-D modes' several-step launches write a second set as well)
+  size_t comps = 0;
+  for (int k = 0; k < 6; ++k)
+    comps += g.comp[k].exists ? 1 : 0;
   for (int b = 0; b < (ctx->has_second || tile2d_mode (g) ? 2 : 1); ++b)
   {
+    SLAB (comps * (slab_size (n * elem_size (ctx->kind)) + (g.cfg.use_pml ? slab_size (n * sizeof (float)) : 0)));
     for (int k = 0; k < 6; ++k)
     {
       if (!g.comp[k].exists)
@@ -568,6 +635,7 @@ int alloc_fast (fdtd_ctx *ctx)
   }
   if (g.cfg.use_metamaterials)
   {
+    SLAB ((4 + 2 * 6 * 3) * slab_size (n * sizeof (float)) + slab_size (n));
     for (int m = 0; m < 4; ++m)
       DALLOC (ctx->drude32[m], n * sizeof (float));
     DALLOC (ctx->dflag, n);
@@ -845,6 +913,9 @@ std::string plan_shell (fdtd_ctx *ctx, void *const e[2][3], void *const h[2][3],
   // set T (fields as the step stores them, PML auxiliaries), starting as a
   // copy of the current set (its never-updated faces must hold the fields)
   const size_t n = ctx->scells;
+  if (!ctx->tfb[0] &&
+      slab_reserve (ctx, 6 * (slab_size (n * elem_size (ctx->kind)) + slab_size (n * sizeof (float)))) != FDTD_OK)
+    return "allocation of the shell buffer set failed";
   for (int k = 0; k < 6; ++k)
   {
     if (!ctx->tfb[k])
@@ -858,6 +929,7 @@ std::string plan_shell (fdtd_ctx *ctx, void *const e[2][3], void *const h[2][3],
                          ctx->stream) != cudaSuccess)
       return "shell buffer copy failed";
   }
+  slab_close (ctx);
   // x cuts: step 1 owns planes < cx0 + 1 and >= cx1 - 1 of the x slabs, step
   // 2 those < cx0 and >= cx1; the core planes in chunks of at most 64
   auto cuts_for = [&] (int a, int b) {
@@ -1187,6 +1259,7 @@ int plan_sweep (fdtd_ctx *ctx)
       {
         // PML: the x / y PML shell in single steps beside the two-step core
         ctx->tb2_why = plan_shell (ctx, e, h, aux);
+        slab_close (ctx);
         if (ctx->tb2_why.empty ())
           ctx->tb2_state = 2;
       }
@@ -1273,6 +1346,7 @@ int create_impl (const fdtd_config *cfg, int device, fdtd_ctx *ctx)
   const Geometry &g = ctx->g;
   if (g.cfg.use_tfsf)
   {
+    SLAB (4 * slab_size ((size_t) g.inc_len * sizeof (double)));
     for (int l = 0; l < 2; ++l)
     {
       DALLOC (ctx->einc[l], (size_t) g.inc_len * sizeof (double));
@@ -1280,9 +1354,11 @@ int create_impl (const fdtd_config *cfg, int device, fdtd_ctx *ctx)
     }
   }
   ctx->nparts = ctx->sm_count * 4;
+  slab_close (ctx);
   DALLOC (ctx->partials, (size_t) ctx->nparts * 6 * 2 * sizeof (double));
   DALLOC (ctx->d_out, 16 * sizeof (double));
   int r = ctx->kind == 0 ? alloc_plain (ctx) : alloc_fast (ctx);
+  slab_close (ctx);
   if (r != FDTD_OK)
     return r;
   if (ctx->kind != 0)
