@@ -1246,11 +1246,20 @@ int plan_sweep (fdtd_ctx *ctx)
   ctx->tb2_why = "the single-step sweep is not in use";
   if (ctx->sweep_state == 1)
   {
-    bool tb2 = true;
+    // Pairs of steps move fewer bytes but run more launches, a shell of two
+    // single steps and items of a longer pipeline.  With PML, FP32, us per
+    // step, single / pair, without TF/SF (whose pair kernel also replaces
+    // half of the post passes): 128^3 67 / 116, 224^3 205 / 214, 256^3 269 /
+    // 250, 300^3 496 / 369; with TF/SF: 128^3 85 / 125, 192^3 189 / 180,
+    // 300 x 300 x 100 225 / 202, 300^3 521 / 426.  (With TF/SF the line stays
+    // below that crossover, at 128^3, a size whose pairs the precision tests
+    // pin.)
+    // FDTDB_TB2=0 / 1: never / always (test hook).
+    bool tb2 = !g.cfg.use_pml || g.cells >= (g.cfg.use_tfsf ? 2000000 : 15000000);
     if (const char *v = std::getenv ("FDTDB_TB2"))
       tb2 = std::atoi (v) != 0;
     if (!tb2)
-      ctx->tb2_why = "disabled by FDTDB_TB2=0";
+      ctx->tb2_why = "single steps are faster on a grid this small, or FDTDB_TB2=0";
     else
     {
       if (!ctx->tb2_ctr)
