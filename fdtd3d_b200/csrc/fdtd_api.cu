@@ -1871,10 +1871,18 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
         CK (cudaEventRecord (ctx->inc_free, s));
         CK (cudaStreamWaitEvent (si, ctx->inc_free, 0));
       }
+      IncidentPair inc{};
       if (g.cfg.use_tfsf)
       {
-        ctx->launches += launch_incident_e (incident_e_job (ctx, i), si);
-        ctx->launches += launch_incident_h (incident_h_job (ctx), si);
+        inc.e = incident_e_job (ctx, i);
+        inc.h = incident_h_job (ctx);
+        // (a single sweep step whose corrections are a post pass takes the
+        // incident step in its own launch)
+        if (pair || ctx->sweep_state != 1 || !f.tfsf_post)
+        {
+          ctx->launches += launch_incident (inc, si);
+          inc = IncidentPair{};
+        }
       }
       f.inc_h = ctx->hinc[hprev];
       f.inc_e = ctx->einc[ctx->ecur];
@@ -1893,9 +1901,10 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
           inc_h1 = ctx->hinc_keep;
           inc_e1 = ctx->einc[ctx->ecur];
           inc_h2 = ctx->hinc[ctx->hcur];
-          ctx->launches += launch_incident_e (incident_e_job (ctx, i + 1), si);
+          inc.e = incident_e_job (ctx, i + 1);
           inc_e2 = ctx->einc[ctx->ecur];
-          ctx->launches += launch_incident_h (incident_h_job (ctx), si);
+          inc.h = incident_h_job (ctx);
+          ctx->launches += launch_incident (inc, si);
           if (inc_side)
             CK (cudaEventRecord (ctx->inc_done, si));
         }
@@ -1950,7 +1959,7 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
         return r;
       if (ctx->sweep_state == 1)
       {
-        ctx->launches += launch_sweep3d (ctx->sweep, o, f, ctx->d_err, s, ctx->sweep_streams);
+        ctx->launches += launch_sweep3d (ctx->sweep, o, f, ctx->d_err, s, ctx->sweep_streams, inc);
         if (ctx->drude_fix)
         {
           ctx->launches += launch_drude_fixup (f, ctx->drude_box, s);

@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include "incident.h"
 #include "params.h"
 
 namespace fdtdb {
@@ -73,19 +74,12 @@ int launch_plain_fast (const PlainHalf &p, const PlainTabs &t, int inc_len, int 
 // form by columns (plain_march_kernel), with the half-step's update of the
 // 1-D incident grid in the same launch (inc.cells > 0).  mat_uniform: the
 // family's material was never uploaded (1 everywhere).
-struct IncidentJob
-{
-  double *now;                 // level written
-  const double *old;           // the same family's previous level
-  const double *other;         // E: HInc before its update; H: EInc after its update
-  int cells;                   // cells 0 .. cells - 1 are updated (0: nothing to do)
-  double modifier;
-  const double *src;           // E: value of cell 0
-};
 int launch_plain_march (const PlainHalf &p, const PlainTabs &t, const IncidentJob &inc, bool mat_uniform, int inc_len,
                         int *err, int sm_count, cudaStream_t s);
 int launch_incident_e (const IncidentJob &j, cudaStream_t s);
 int launch_incident_h (const IncidentJob &j, cudaStream_t s);
+// both updates of a step in one launch
+int launch_incident (const IncidentPair &j, cudaStream_t s);
 int launch_point_source (double *f, size_t index, const double *src, int src_index, cudaStream_t s);
 
 // Double material precision: per coarse cell, the average of the fine cells

@@ -65,6 +65,11 @@ __global__ void incident_h_kernel (IncidentJob j)
     j.now[i] = j.old[i] + (j.other[i] - j.other[i + 1]) * j.modifier;
 }
 
+__global__ void incident_kernel (IncidentPair j)
+{
+  incident_pair (j, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 __global__ void point_source_kernel (double *f, size_t index, const double *src, int src_index)
 {
   if (threadIdx.x == 0 && blockIdx.x == 0)
@@ -696,6 +701,12 @@ int launch_incident_e (const IncidentJob &j, cudaStream_t s)
 int launch_incident_h (const IncidentJob &j, cudaStream_t s)
 {
   incident_h_kernel<<<(j.cells + 255) / 256, 256, 0, s>>> (j);
+  return 1;
+}
+
+int launch_incident (const IncidentPair &j, cudaStream_t s)
+{
+  incident_kernel<<<(std::max (j.e.cells, j.h.cells) + 255) / 256, 256, 0, s>>> (j);
   return 1;
 }
 

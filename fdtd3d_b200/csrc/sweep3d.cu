@@ -388,7 +388,7 @@ __host__ __device__ inline int sweep_item_class (const FusedParams &p, const Swe
 template <typename T, int WY, int MODE>
 __global__ void __launch_bounds__ (32 * WY, 1)
     sweep3d_kernel (const __grid_constant__ SweepMaps maps, const __grid_constant__ FusedParams p,
-                    const SweepWork wk, int *err)
+                    const SweepWork wk, const __grid_constant__ IncidentPair inc, int *err)
 {
   using L = Smem<T, WY>;
   constexpr int HZ = L::HZ, HW = L::HW, EW = L::EW, AN = L::AN, XW = L::XW;
@@ -488,6 +488,9 @@ __global__ void __launch_bounds__ (32 * WY, 1)
       }
     }
   };
+
+  // the step's incident grid (nothing of this launch reads it)
+  incident_pair (inc, blockIdx.x * 32 * WY + tid, gridDim.x * 32 * WY);
 
   unsigned phase = 0;   // bit s: parity of the next completion of stage s
   bool aborted = false;
@@ -1245,12 +1248,16 @@ std::string plan_t (SweepPlan &pl, const FusedParams &p, void *const e[2][3], vo
 }
 
 template <typename T, int WY>
-int launch_t (const SweepPlan &pl, int set, const FusedParams &p, int *err, cudaStream_t s, const SweepStreams &ss)
+int launch_t (const SweepPlan &pl, int set, const FusedParams &p, int *err, cudaStream_t s, const SweepStreams &ss,
+              IncidentPair inc)
 {
   // on side streams the next class's CTAs take the SMs as the previous
   // class's persistent CTAs run out of items
   constexpr unsigned sm = Smem<T, WY>::TOTAL;
-  const bool conc = ss.side[0] && ss.side[1];
+  // (one class alone needs no side stream: small grids are bound by their
+  // launches, and the events cost as much as one)
+  const int classes = (pl.items[0] > 0) + (pl.items[1] > 0) + (pl.items[2] > 0) + (pl.items[3] > 0);
+  const bool conc = ss.side[0] && ss.side[1] && classes > 1;
   cudaStream_t s1 = s, s0 = s;
   if (conc)
   {
@@ -1263,7 +1270,8 @@ int launch_t (const SweepPlan &pl, int set, const FusedParams &p, int *err, cuda
   int n = 0;
   if (pl.items[2] > 0)
   {
-    sweep3d_kernel<T, WY, 2><<<pl.ctas, dim3 (32, WY), sm, s>>> (pl.maps[set], p, pl.work, err);
+    sweep3d_kernel<T, WY, 2><<<pl.ctas, dim3 (32, WY), sm, s>>> (pl.maps[set], p, pl.work, inc, err);
+    inc = IncidentPair{};   // the first launch takes it
     ++n;
   }
   // launch order of the PML (3), z-edge (1) and lean (0) classes on s, s1,
@@ -1277,11 +1285,12 @@ int launch_t (const SweepPlan &pl, int set, const FusedParams &p, int *err, cuda
     if (pl.items[c] <= 0)
       continue;
     if (c == 3)
-      sweep3d_kernel<T, WY, 3><<<pl.ctas, dim3 (32, WY), sm, on[j]>>> (pl.maps[set], p, pl.work, err);
+      sweep3d_kernel<T, WY, 3><<<pl.ctas, dim3 (32, WY), sm, on[j]>>> (pl.maps[set], p, pl.work, inc, err);
     else if (c == 1)
-      sweep3d_kernel<T, WY, 1><<<pl.ctas, dim3 (32, WY), sm, on[j]>>> (pl.maps[set], p, pl.work, err);
+      sweep3d_kernel<T, WY, 1><<<pl.ctas, dim3 (32, WY), sm, on[j]>>> (pl.maps[set], p, pl.work, inc, err);
     else
-      sweep3d_kernel<T, WY, 0><<<pl.ctas, dim3 (32, WY), sm, on[j]>>> (pl.maps[set], p, pl.work, err);
+      sweep3d_kernel<T, WY, 0><<<pl.ctas, dim3 (32, WY), sm, on[j]>>> (pl.maps[set], p, pl.work, inc, err);
+    inc = IncidentPair{};
     ++n;
   }
   if (conc)
@@ -1410,9 +1419,10 @@ std::string sweep3d_plan_list (SweepPlan &plan, const FusedParams &p, void *cons
 }
 
 int launch_sweep3d (const SweepPlan &plan, int set, const FusedParams &p, int *err, cudaStream_t s,
-                    const SweepStreams &ss)
+                    const SweepStreams &ss, const IncidentPair &inc)
 {
-  return p.fp16 ? launch_t<__half, 8> (plan, set, p, err, s, ss) : launch_t<float, 8> (plan, set, p, err, s, ss);
+  return p.fp16 ? launch_t<__half, 8> (plan, set, p, err, s, ss, inc)
+                : launch_t<float, 8> (plan, set, p, err, s, ss, inc);
 }
 
 }  // namespace fdtdb

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "fused3d.h"
+#include "incident.h"
 
 namespace fdtdb {
 
@@ -92,9 +93,11 @@ struct SweepStreams
 
 // One time step with buffer set `set` as the old set (one launch per item
 // class that has items; returns how many).  With side streams the z-edge
-// and the lean class run on them, joined back into s before returning.
+// and the lean class run on them, joined back into s before returning.  The
+// first launch also takes the incident step `inc` (which the sweep itself must
+// not read: tfsf_post).
 int launch_sweep3d (const SweepPlan &plan, int set, const FusedParams &p, int *err, cudaStream_t s,
-                    const SweepStreams &ss = SweepStreams ());
+                    const SweepStreams &ss = SweepStreams (), const IncidentPair &inc = IncidentPair ());
 
 }  // namespace fdtdb
 
