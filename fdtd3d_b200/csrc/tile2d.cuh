@@ -12,7 +12,7 @@
 // cell's arithmetic is the per-cell kernels', so FP64 fields keep their bits;
 // FP16 storage rounds once per launch instead of once per half-step.  A run
 // of 100 steps at 120 x 100 in FP64, its three fields read by the host: 2133
-// -> 440 us; 200 steps at 512^2 in FP32: 4820 -> 1270 us (of which reading the
+// -> 306 us; 200 steps at 512^2 in FP32: 4890 -> 1194 us (of which reading the
 // fields is 465).
 // The part of the 1-D incident grid a tile's TF/SF terms can reach advances
 // in shared memory with it; a few CTAs advance the whole grid.
@@ -180,7 +180,9 @@ struct TileMem
 // rows u0 + RU w ..., a lane RV neighbouring cells of each: differences along
 // v cross lanes by shuffles, those along u cross warps by one shared row per
 // component, all others stay in the thread's registers.
-template <typename T, typename C, int RU, int RV, int FORM>
+// CHAIN: the coefficients, tables and border terms are set up before the launch
+// in front of this one is over, the fields loaded after it.
+template <typename T, typename C, int RU, int RV, int FORM, bool CHAIN>
 __device__ __forceinline__ void tile2d_steps (const Tile2D &p, int u0, int v0, unsigned char *smem,
                                               double (*s_inc)[kTileThreads])
 {
@@ -215,6 +217,21 @@ __device__ __forceinline__ void tile2d_steps (const Tile2D &p, int u0, int v0, u
   C f[3][RU][RV], x[3][RU][RV];
   unsigned upd = 0, face = 0, source = 0, in_pml[3] = {0, 0, 0};
   int64_t ids[RU];
+  auto load = [&] (int j, int r, int c, bool valid, bool up, bool pm) __attribute__ ((always_inline)) {
+    const TileComp &q = p.comp[j];
+    f[j][r][c] = C (0);
+    x[j][r][c] = C (0);
+    if (valid)
+      f[j][r][c] = C (tile_ld ((const T *) q.in, ids[r] + c));
+    if constexpr (F64)
+    {
+      const C *const src = !up ? (const C *) q.out : (const C *) q.aux_in;
+      if (valid && src)
+        x[j][r][c] = src[ids[r] + c];
+    }
+    else if (pm)
+      x[j][r][c] = ((const float *) q.aux_in)[ids[r] + c];
+  };
 #pragma unroll
   for (int r = 0; r < RU; ++r)
   {
@@ -234,23 +251,11 @@ __device__ __forceinline__ void tile2d_steps (const Tile2D &p, int u0, int v0, u
       for (int j = 0; j < 3; ++j)
       {
         const TileComp &q = p.comp[j];
-        f[j][r][c] = C (0);
-        x[j][r][c] = C (0);
-        if (valid)
-          f[j][r][c] = C (tile_ld ((const T *) q.in, ids[r] + c));
-        if constexpr (F64)
-        {
-          const C *const src = !up ? (const C *) q.out : (const C *) q.aux_in;
-          if (valid && src)
-            x[j][r][c] = src[ids[r] + c];
-        }
-        else
-        {
-          const bool pm = up && p.use_pml && !(u >= q.ilo[0] && u < q.ihi[0] && v >= q.ilo[1] && v < q.ihi[1]);
-          in_pml[j] |= pm ? bit : 0u;
-          if (pm)
-            x[j][r][c] = ((const float *) q.aux_in)[ids[r] + c];
-        }
+        const bool pm =
+            !F64 && up && p.use_pml && !(u >= q.ilo[0] && u < q.ihi[0] && v >= q.ilo[1] && v < q.ihi[1]);
+        if constexpr (!CHAIN)
+          load (j, r, c, valid, up, pm);
+        in_pml[j] |= pm ? bit : 0u;
       }
     }
   }
@@ -336,17 +341,21 @@ __device__ __forceinline__ void tile2d_steps (const Tile2D &p, int u0, int v0, u
     }
   const bool has_terms = __syncthreads_or (mine) != 0;
   int wc = 0, first[2] = {0, 0};
-  if (has_terms)
-  {
-    const double a0 = ((double) (u0 - 1) - p.zero[0]) * p.k[0], a1 = ((double) (u0 + TU + 1) - p.zero[0]) * p.k[0];
-    const double b0 = ((double) (v0 - 1) - p.zero[1]) * p.k[1], b1 = ((double) (v0 + TV + 1) - p.zero[1]) * p.k[1];
-    wc = max (0, (int) (fmin (a0, a1) + fmin (b0, b1)) - kTileSteps - 3);
+  auto window = [&] () __attribute__ ((always_inline)) {
     const int q = lane + 32 * w, i = wc + q;
     if (q < kWindow)
     {
       s_inc[0][q] = i < p.inc_len ? p.e_in[i] : 0.0;
       s_inc[1][q] = i < p.inc_len ? p.h_in[i] : 0.0;
     }
+  };
+  if (has_terms)
+  {
+    const double a0 = ((double) (u0 - 1) - p.zero[0]) * p.k[0], a1 = ((double) (u0 + TU + 1) - p.zero[0]) * p.k[0];
+    const double b0 = ((double) (v0 - 1) - p.zero[1]) * p.k[1], b1 = ((double) (v0 + TV + 1) - p.zero[1]) * p.k[1];
+    wc = max (0, (int) (fmin (a0, a1) + fmin (b0, b1)) - kTileSteps - 3);
+    if constexpr (!CHAIN)
+      window ();
     if (mine)
     {
       int e = atomicAdd (&s_terms, mine);
@@ -366,6 +375,22 @@ __device__ __forceinline__ void tile2d_steps (const Tile2D &p, int u0, int v0, u
                     Terms[e] = tile_term (&p, &p.comp[j].term[__ffs ((int) t) - 1], wc, ub + r, vb + c);
       }
     }
+  }
+
+  // (all above reads only what no step writes)
+  if constexpr (CHAIN)
+  {
+    cudaGridDependencySynchronize ();
+    if (has_terms)
+      window ();
+#pragma unroll
+    for (int r = 0; r < RU; ++r)
+#pragma unroll
+      for (int c = 0; c < RV; ++c)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          load (j, r, c, ((upd | face) >> (RV * r + c)) & 1u, (upd >> (RV * r + c)) & 1u,
+                (in_pml[j] >> (RV * r + c)) & 1u);
   }
 
   // the row a neighbouring warp reads of component j: the last one where the
@@ -609,6 +634,16 @@ __global__ void __launch_bounds__ (kTileThreads, 1) tile2d_kernel (const __grid_
   constexpr int OU = kTileWarps * RU - 2 * kTileSteps, OV = 32 * RV - 2 * kTileSteps;
   extern __shared__ __align__ (16) unsigned char tile_smem[];
   __shared__ double s_inc[2][kTileThreads];
+  // The next launch may begin while this one steps: its launch latency, and on
+  // the SMs that small tiles leave free its set-up, are then not in the chain.
+  // Seven steps: 120 x 100 with TF/SF FP64 24.7 -> 16.2 us, FP32 21.8 -> 14.6;
+  // 200 x 200 FP32 13.3 -> 9.6.  (Tiles of more cells fill the SMs' registers,
+  // so nothing of the next launch runs before this one ends: with the late
+  // loads they spill and 512 x 512 FP32 takes 27.9 us instead of 26.6.)
+  constexpr bool CHAIN = RU * RV == 2;
+  cudaTriggerProgrammaticLaunchCompletion ();
+  if (!CHAIN || (int) blockIdx.x >= ntiles)
+    cudaGridDependencySynchronize ();
   if ((int) blockIdx.x >= ntiles)
   {
     const int lane = threadIdx.x, w = threadIdx.y;
@@ -634,7 +669,7 @@ __global__ void __launch_bounds__ (kTileThreads, 1) tile2d_kernel (const __grid_
     }
     return;
   }
-  tile2d_steps<T, C, RU, RV, FORM> (p, ((int) blockIdx.x / tiles_v) * OU - kTileSteps,
+  tile2d_steps<T, C, RU, RV, FORM, CHAIN> (p, ((int) blockIdx.x / tiles_v) * OU - kTileSteps,
                                     ((int) blockIdx.x % tiles_v) * OV - kTileSteps, tile_smem, s_inc);
 }
 
@@ -648,7 +683,17 @@ int tile2d_start (const Tile2D &p, cudaStream_t s)
   auto kern = tile2d_kernel<T, C, RU, RV, FORM>;
   if (smem > 48 * 1024)
     cudaFuncSetAttribute (kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  kern<<<tu * tv + inc, dim3 (32, kTileWarps), smem, s>>> (p, tv, tu * tv);
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3 (tu * tv + inc);
+  lc.blockDim = dim3 (32, kTileWarps);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = &at;
+  lc.numAttrs = 1;
+  cudaLaunchKernelEx (&lc, kern, p, tv, tu * tv);
   return 1;
 }
 

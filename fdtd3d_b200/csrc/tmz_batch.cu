@@ -162,7 +162,7 @@ __global__ void __launch_bounds__ (kTileThreads, 1) tmz_batch_kernel (BatchParam
         s_p.src = p.src + s;
       }
       __syncthreads ();
-      tile2d_steps<float, float, CU, CV, 0> (s_p, t.u0, t.v0, tile_smem, s_inc);
+      tile2d_steps<float, float, CU, CV, 0, false> (s_p, t.u0, t.v0, tile_smem, s_inc);
     }
     // the counter of the next round (same parity as the previous one) is idle now
     if (blockIdx.x == 0 && tid == 0)
