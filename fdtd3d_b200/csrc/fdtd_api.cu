@@ -1197,6 +1197,13 @@ int plan_sweep (fdtd_ctx *ctx)
         b.lo[a] = std::max (hb[a], 1);
         b.hi[a] = std::min (hb[3 + a] + 1, g.n[a] - 1);
       }
+      b.zfree[0] = 0;
+      b.zfree[1] = ctx->pz;
+      for (int k = 0; k < 6 && g.cfg.use_pml; ++k)
+      {
+        b.zfree[0] = std::max (b.zfree[0], ctx->fused.ilo[k][2]);
+        b.zfree[1] = std::min (b.zfree[1], ctx->fused.ihi[k][2]);
+      }
       int ext_lo[3];
       for (int a = 0; a < 3; ++a)
         ext_lo[a] = std::max (b.lo[a] - 1, 1);
@@ -1974,14 +1981,8 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
         if (g.cfg.use_metamaterials && !ctx->drude_levels)
         {
           // after sweep steps the levels two steps back are in the set the
-          // step is about to write
-          for (int k = 0; k < 6; ++k)
-          {
-            CK (cudaMemcpyAsync (ctx->xppb[o][k], ctx->auxb[nw][k], ctx->scells * sizeof (float),
-                                 cudaMemcpyDeviceToDevice, s));
-            CK (cudaMemcpyAsync (ctx->zppb[o][k], ctx->zb[nw][k], ctx->scells * sizeof (float),
-                                 cudaMemcpyDeviceToDevice, s));
-          }
+          // step is about to write (and for some vectors in xpp already)
+          ctx->launches += launch_drude_levels (f, ctx->drude_box, s);
           ctx->drude_levels = true;
         }
         ctx->launches += launch_fused3d (f, ctx->d_err, s);

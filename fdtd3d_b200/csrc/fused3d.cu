@@ -672,18 +672,26 @@ __device__ __forceinline__ bool drude_cells (const DrudeBox &b, int &x, int &y, 
   return x < b.hi[0];
 }
 
+// Whether the vector at z may hold PML cells too.
+__device__ __forceinline__ bool drude_shared (const DrudeBox &b, int z)
+{
+  return z < b.zfree[0] || z + 4 > b.zfree[1];
+}
+
 // Drude update of component k on the cells of mask m among four (no PML here,
 // so the curl step is X + S curl and F takes Z_new - Z; see update_drude for
 // the recurrence).  X and Z two steps back are what the new set still holds
 // from the step before last (every step alternates the sets), so no array of
-// previous levels is read or written.  w, g, em: averaged plasma frequency,
-// collision rate and eps.
-__device__ __forceinline__ void drude_four (const FusedParams &p, int k, size_t id, unsigned m, const float w[4],
-                                            const float g[4], const float em[4], const float curl[4], float f[4])
+// previous levels is read or written; but in a vector that PML cells share the
+// sweep has stored over that X, and xpp keeps it (two such vectors a row at
+// most).  w, g, em: averaged plasma frequency, collision rate and eps.
+__device__ __forceinline__ void drude_four (const FusedParams &p, int k, size_t id, unsigned m, bool shared,
+                                            const float w[4], const float g[4], const float em[4],
+                                            const float curl[4], float f[4])
 {
   float xo[4], xp[4], zo[4], zp[4];
   ld4v (p.aux_old[k] + id, xo);
-  ld4v (p.aux_new[k] + id, xp);
+  ld4v ((shared ? p.xpp_old[k] : p.aux_new[k]) + id, xp);
   ld4v (p.z_old[k] + id, zo);
   ld4v (p.z_new[k] + id, zp);
   const float dt = p.dt, S = p.courant;
@@ -703,6 +711,8 @@ __device__ __forceinline__ void drude_four (const FusedParams &p, int k, size_t 
   }
   st4v (p.aux_new[k] + id, xp, m);
   st4v (p.z_new[k] + id, zp, m);
+  if (shared)
+    st4v (p.xpp_new[k] + id, xo, m);
 }
 
 // Drude fix-up after a TMA sweep step, which updates every cell with the
@@ -785,7 +795,7 @@ __global__ void __launch_bounds__ (128) drude_fix_e_kernel (const __grid_constan
     }
     if (on[k])
     {
-      drude_four (p, k, id, on[k], w, g, em, cu, f);
+      drude_four (p, k, id, on[k], drude_shared (b, z), w, g, em, cu, f);
       st4v ((T *) p.e_new[k] + id, f, on[k]);
     }
   }
@@ -864,12 +874,39 @@ __global__ void __launch_bounds__ (128) drude_fix_h_kernel (const __grid_constan
       }
     }
     if (on[k])
-      drude_four (p, 3 + k, id, on[k], w, g, one, cu, f);
+      drude_four (p, 3 + k, id, on[k], drude_shared (b, z), w, g, one, cu, f);
     st4v ((T *) p.h_new[k] + id, f, own);
   }
 }
 
+__global__ void __launch_bounds__ (256) drude_levels_kernel (const __grid_constant__ FusedParams p, DrudeBox b)
+{
+  const size_t pz = p.g.pz, n4 = (size_t) p.g.n[0] * p.g.n[1] * pz / 4;
+  for (size_t q = (size_t) blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (size_t) gridDim.x * blockDim.x)
+  {
+    const size_t id = 4 * q;
+    const bool shared = drude_shared (b, (int) (id % pz));
+    for (int k = 0; k < 6; ++k)
+    {
+      float v[4];
+      if (!shared)
+      {
+        ld4v (p.aux_new[k] + id, v);
+        st4v (const_cast<float *> (p.xpp_old[k]) + id, v, 15u);
+      }
+      ld4v (p.z_new[k] + id, v);
+      st4v (const_cast<float *> (p.zpp_old[k]) + id, v, 15u);
+    }
+  }
+}
+
 }  // namespace
+
+int launch_drude_levels (const FusedParams &p, const DrudeBox &box, cudaStream_t s)
+{
+  drude_levels_kernel<<<148 * 8, 256, 0, s>>> (p, box);
+  return 1;
+}
 
 int launch_drude_box (const unsigned char *flags, int nx, int ny, int pz, int *box, cudaStream_t s)
 {

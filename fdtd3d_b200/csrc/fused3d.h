@@ -42,8 +42,9 @@ struct FusedParams
   // non-zero averaged plasma frequency or collision rate; state of those
   // cells: X (in aux), X two steps back, Z = D1/eps0... scaled, Z one step back
   // (the sweep's fix-up reads the levels two steps back from the new set's X
-  // and Z instead, which hold them until it writes; only the register-blocked
-  // kernel, whose tiles recompute each other's edge cells, keeps xpp and zpp)
+  // and Z instead, which hold them until it writes, except where the sweep
+  // writes that X: DrudeBox; only the register-blocked kernel, whose tiles
+  // recompute each other's edge cells, keeps xpp and zpp everywhere)
   int use_meta;
   float dt;
   const unsigned char *dflag;
@@ -61,16 +62,25 @@ int launch_fused3d (const FusedParams &p, int *err, cudaStream_t s);
 // owned y rows of one CTA for a shape variant
 int fused_rows_per_cta (int shape);
 
-// Cells x = lo[0] .. hi[0] - 1 (and the same for y, z).
+// Cells x = lo[0] .. hi[0] - 1 (and the same for y, z).  The sweep stores the
+// PML auxiliaries as vectors of four z cells, so in a vector that reaches past
+// the z cells zfree[0] .. zfree[1] - 1 (no PML for any component) it may write
+// over the X two steps back of the vector's Drude cells: those vectors keep it
+// in xpp.
 struct DrudeBox
 {
   int lo[3], hi[3];
+  int zfree[2];
 };
 
 // Bounding box of the cells with a Drude flag into box[6] (device ints:
 // lowest x, y, z, then highest; INT_MAX / -1 when no cell has one); rows of
 // pz stored cells.
 int launch_drude_box (const unsigned char *flags, int nx, int ny, int pz, int *box, cudaStream_t s);
+
+// Before a register-blocked step that follows sweep steps: the old set's xpp
+// and zpp from where the fix-up left the levels two steps back.
+int launch_drude_levels (const FusedParams &p, const DrudeBox &box, cudaStream_t s);
 
 // Drude fix-up of a TMA sweep step over the Drude cells of `box` (two
 // launches; returns how many).
