@@ -393,7 +393,9 @@ __global__ void __launch_bounds__ (kMarchBlock, 5)
     e2 = tb.t[2][2][y];
   }
   // what the current E-from-D coefficients (without PML: cb) were made from
-  double m_of[3] = {-1, -1, -1}, np0 = 0, nm0 = 0, dd1 = 0;
+  // (at first nothing: NaN differs from every material)
+  const double none = __longlong_as_double (0x7ff8000000000000ll);
+  double m_of[3] = {none, none, none}, np0 = 0, nm0 = 0, dd1 = 0;
   double cp[3] = {0, 0, 0}, cm[3] = {0, 0, 0};
   // x coefficients of the plane: component 2's ca, cb and component 1's ca2
   double cax = 1, cbx = 0, e1 = 1;

@@ -74,3 +74,33 @@ def test_columns_match_cells_in_h_centered_grids(fdtd, mu, double):
         far[5:9, 4:8, 3:7] = False   # (the current acts on its cell and the H cells around it)
         for c in COMPS:
             assert np.array_equal(out[0][c][far].view(np.int64), out[1][c][far].view(np.int64)), (layout, c)
+
+
+# a material of -1 on a column's first plane: the coefficients must be formed
+# from it (with PML every component but the last is formed anew by the x
+# coefficients all the same)
+@pytest.mark.parametrize("where", ["everywhere", "first planes", "a block"])
+@pytest.mark.parametrize("pml", [0, 3])
+@pytest.mark.parametrize("which", [("eps",), ("mu",), ("eps", "mu")])
+def test_material_of_minus_one(fdtd, where, pml, which):
+    shape = (20, 13, 14)
+    mats = {}
+    for name in which:
+        m = np.full(shape, -1.0)
+        if where == "first planes":
+            m[6:] = 2.5
+        elif where == "a block":
+            m[:] = 1.5
+            m[1:5, 4:9, 3:8] = -1.0
+        mats[name] = m
+    kw = dict(mode=3, size=shape, point_source=(10, 6, 7), point_source_mask=1 << 2)
+    if pml:
+        kw.update(use_pml=True, pml=pml)
+    o = Oracle(materials=mats, **kw)
+    o.step(12)
+    with fdtd.Simulation(materials=mats, **kw) as sim:
+        sim.step(12)
+        for c in COMPS:
+            got, want = sim.field(c), o.field(c)
+            assert np.array_equal(got.view(np.int64), want.view(np.int64)), (c, np.max(np.abs(got - want)))
+    o.close()
