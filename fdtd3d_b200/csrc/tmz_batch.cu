@@ -381,6 +381,9 @@ int enqueue (fdtd_batch *b, uint32_t t_start, uint32_t n)
   return FDTD_OK;
 }
 
+// Cells of the read-out's staging buffer at most (64 MB; no row is longer).
+constexpr size_t kStageCells = (size_t) 1 << 23;
+
 // Rounds of a launch: the buffer set changes with each.
 uint32_t batch_rounds (uint32_t t_start, uint32_t n)
 {
@@ -769,19 +772,28 @@ int fdtd_batch_download (fdtd_batch *b, int instance, int component, double *hos
   const fdtdb::InstDev &in = b->inst[instance];
   size_t n = (size_t) in.nx * in.ny;
   const float *src = component == FDTD_EZ ? b->ez[b->cur] : (component == FDTD_HX ? b->hx[b->cur] : b->hy[b->cur]);
-  // widened on the device, then one copy into the caller's buffer
-  if (n > b->stage_cells)
+  // widened on the device a piece of rows at a time (an instance may have more
+  // than 2^31 cells, and a batch that fills the device has no room for a second
+  // copy of its largest one), each copied into the caller's buffer
+  if (!b->stage)
   {
     size_t most = 0;
     for (const fdtdb::InstDev &i : b->inst)
       most = std::max (most, (size_t) i.nx * i.ny);
+    most = std::min (most, kStageCells);
     BALLOC (b->stage, most * sizeof (double));
     b->stage_cells = most;
   }
-  fdtdb::launch_convert_out (b->stage, src + in.off, 1, 1, (int) n, (int) n,
-                             component == FDTD_EZ ? 1.0 : 1.0 / fdtdb::kEta0B, b->stream);
-  BCK (cudaGetLastError ());
-  BCK (cudaMemcpyAsync (host, b->stage, n * sizeof (double), cudaMemcpyDeviceToHost, b->stream));
+  const double scale = component == FDTD_EZ ? 1.0 : 1.0 / fdtdb::kEta0B;
+  // (whole groups of four rows keep every piece on a 16-byte boundary)
+  const size_t fit = b->stage_cells / in.ny, piece = (fit >= 4 ? fit / 4 * 4 : fit) * in.ny;
+  for (size_t at = 0; at < n; at += piece)
+  {
+    const size_t m = std::min (piece, n - at);
+    fdtdb::launch_convert_out (b->stage, src + in.off + at, 1, m / in.ny, in.ny, in.ny, scale, b->stream);
+    BCK (cudaGetLastError ());
+    BCK (cudaMemcpyAsync (host + at, b->stage, m * sizeof (double), cudaMemcpyDeviceToHost, b->stream));
+  }
   BCK (cudaStreamSynchronize (b->stream));
   return FDTD_OK;
 }
