@@ -2665,7 +2665,8 @@ int fdtd_ntff (fdtd_ctx *re, fdtd_ctx *im, const int left[3], const int right[3]
     len[a] = right[a] - left[a];
   }
   p.points = 2 * (len[1] * len[2] + len[0] * len[2] + len[0] * len[1]);
-  p.pz = re->pz;   // (the same form and grid: the same rows)
+  p.pz[0] = re->pz;
+  p.pz[1] = im->pz;
   p.dx = g.cfg.dx;
   p.k = 2 * kPi / g.cfg.wavelength;
   p.teta = teta;

@@ -48,32 +48,38 @@ enum { EX, EY, EZ, HX, HY, HZ };
 // Cell of a position relative to the component's first position (integer
 // valued by construction; the reference's convertCoord truncates).  Clamped
 // into the grid as a guard; the host checks the box so that it never acts.
-__device__ __forceinline__ int64_t cell (const NtffParams &p, const double q[3])
+struct Cell
+{
+  int64_t row;   // z row
+  int z;
+};
+__device__ __forceinline__ Cell cell (const NtffParams &p, const double q[3])
 {
   int i[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
     i[a] = min (max ((int) q[a], 0), p.n[a] - 1);
-  return ((int64_t) i[0] * p.n[1] + i[1]) * p.pz + i[2];
+  return {(int64_t) i[0] * p.n[1] + i[1], i[2]};
 }
 
 // A stored field value in physical units (FP64 as stored; FP32 / FP16
 // storage converted and scaled: H is kept as eta0 H there)
-__device__ __forceinline__ double fval (const NtffParams &p, const void *a, int c, int64_t id)
+__device__ __forceinline__ double fval (const NtffParams &p, int run, const void *a, int c, Cell at)
 {
+  const int64_t id = at.row * p.pz[run] + at.z;
   if (p.kind == 0)
     return static_cast<const double *> (a)[id];
   if (p.kind == 1)
     return (double) static_cast<const float *> (a)[id] * p.scale[c];
   return (double) __half2float (static_cast<const __half *> (a)[id]) * p.scale[c];
 }
-__device__ __forceinline__ Cx cur (const NtffParams &p, int c, int64_t id)
+__device__ __forceinline__ Cx cur (const NtffParams &p, int c, Cell at)
 {
-  return {fval (p, p.cur[0][c], c, id), fval (p, p.cur[1][c], c, id)};
+  return {fval (p, 0, p.cur[0][c], c, at), fval (p, 1, p.cur[1][c], c, at)};
 }
-__device__ __forceinline__ Cx prev (const NtffParams &p, int c, int64_t id)
+__device__ __forceinline__ Cx prev (const NtffParams &p, int c, Cell at)
 {
-  return {fval (p, p.prev[0][c], c, id), fval (p, p.prev[1][c], c, id)};
+  return {fval (p, 0, p.prev[0][c], c, at), fval (p, 1, p.prev[1][c], c, at)};
 }
 
 // Component c at position x: one cell, or the two cells at -/+ 1/2 along
@@ -86,13 +92,13 @@ __device__ Cx sample (const NtffParams &p, int c, const double x[3], int avg_axi
     q[a] = x[a] - p.min_fp[c][a];
   if (avg_axis < 0)
   {
-    const int64_t id = cell (p, q);
+    const Cell id = cell (p, q);
     return tavg ? (cur (p, c, id) + prev (p, c, id)) / 2.0 : cur (p, c, id);
   }
   double q1[3] = {q[0], q[1], q[2]}, q2[3] = {q[0], q[1], q[2]};
   q1[avg_axis] -= 0.5;
   q2[avg_axis] += 0.5;
-  const int64_t i1 = cell (p, q1), i2 = cell (p, q2);
+  const Cell i1 = cell (p, q1), i2 = cell (p, q2);
   if (tavg)
     return (cur (p, c, i1) + cur (p, c, i2) + prev (p, c, i1) + prev (p, c, i2)) / 4.0;
   return (cur (p, c, i1) + cur (p, c, i2)) / 2.0;

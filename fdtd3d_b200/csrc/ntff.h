@@ -15,7 +15,7 @@ namespace fdtdb {
 struct NtffParams
 {
   int n[3];                    // grid size
-  int pz;                      // stored cells per z row
+  int pz[2];                   // stored cells per z row of each run (double material precision pads no rows)
   int left[3], right[3];       // the box: faces at left and right on every axis
   double diff0[3];             // phase origin: n / 2 (integer division)
   double dx;                   // grid step

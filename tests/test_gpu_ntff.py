@@ -161,6 +161,36 @@ def test_fdtd_ntff_fast_forms(fdtd, layout, prec, steps):
     assert "sweep2_tma" not in kernels   # every call ends on a single step
 
 
+@pytest.mark.parametrize("prec,tol", [(1, 1e-4), (2, 2e-2)])
+@pytest.mark.parametrize("dmp", [(True, False), (False, True)])
+def test_fdtd_ntff_of_runs_with_different_rows(fdtd, prec, tol, dmp):
+    """One run with double material precision, which stores rows of nz cells,
+    one without, whose rows are padded to whole 16-byte units at this nz: the
+    same physics (the fine map repeats the coarse one), against the FP64 form
+    (the bounds of test_fdtd_ntff_fast_forms)."""
+    n = (24, 22, 37)
+    kw = dict(mode=3, size=n, use_pml=True, pml=4, use_tfsf=True, tfsf_left=7, tfsf_right=7, teta=30, phi=40, psi=10)
+    x, y, z = np.indices(n)
+    eps = np.where((x - 12) ** 2 + (y - 11) ** 2 + (z - 18) ** 2 < 16, 4.0, 1.0)
+    vals = {}
+    for p in (fdtd.PREC_FP64_PLAIN, prec):
+        sims = [fdtd.Simulation(precision=p, source_phase=ph, double_material_precision=d,
+                                materials={"eps": np.kron(eps, np.ones((2, 2, 2))) if d else eps}, **kw)
+                for ph, d in enumerate(dmp)]
+        try:
+            for s in sims:
+                s.keep_previous_level()
+                s.step(41)
+            vals[p] = fdtd.ntff(sims[0], sims[1], (5, 5, 5), tuple(v - 4 for v in n), fdtd.f32(30) * np.pi / 180.0,
+                                np.linspace(0, 2 * np.pi, 25))
+        finally:
+            for s in sims:
+                s.close()
+    want, got = vals[fdtd.PREC_FP64_PLAIN], vals[prec]
+    assert np.all(want > 0)
+    assert np.max(np.abs(got - want) / want) <= tol, np.max(np.abs(got - want) / want)
+
+
 def test_cli_fp32_ntff_close_to_reference_complex_build(fdtd, tmp_path):
     """fdtd3d-b200 --precision fp32 --complex-field-values --use-ntff: the
     same NTFF files as the reference's complex build, values within 1e-4
