@@ -1254,13 +1254,21 @@ int plan_sweep (fdtd_ctx *ctx)
   if (ctx->sweep_state == 1)
   {
     // Pairs of steps move fewer bytes but run more launches, a shell of two
-    // single steps and items of a longer pipeline.  With PML, FP32, us per
-    // step, single / pair, without TF/SF (whose pair kernel also replaces
-    // half of the post passes): 128^3 67 / 116, 224^3 205 / 214, 256^3 269 /
-    // 250, 300^3 496 / 369; with TF/SF: 128^3 85 / 125, 192^3 189 / 180,
-    // 300 x 300 x 100 225 / 202, 300^3 521 / 426.  (With TF/SF the line stays
-    // below that crossover, at 128^3, a size whose pairs the precision tests
-    // pin.)
+    // single steps and items of a longer pipeline.  us per step, single / pair
+    // (FP32; FP16 storage differs by 5 %):
+    //  PML: 128^3 67 / 116, 192^3 161 / 177, 240^3 223 / 236, 256^3 264 / 243,
+    //   280^3 398 / 305; a point source changes both by 4 to 7 us;
+    //  PML, TF/SF (whose pair kernel also replaces half of the post passes):
+    //   128^3 78 / 125, 192^3 189 / 180, 300^3 521 / 426;
+    //  no PML: 64^3 21 / 42, 128^3 22 / 80, 1000 x 64 x 64 72 / 80, 160^3 70 /
+    //   53, 192^3 95 / 62, 256^3 145 / 152, 320^3 311 / 238; with TF/SF 128^3
+    //   34 / 99, 160^3 84 / 78, 320^3 338 / 298;
+    //  rows of at most half of the single sweep's z tile (its lanes idle, the
+    //   pair's tile is 60 cells): PML 200 x 200 x 33 104 / 123, 300 x 300 x 33
+    //   200 / 120, 600 x 600 x 33 694 / 276; no PML 46 / 63, 87 / 64, 310 / 147.
+    // The lines lie at the crossovers, but with PML and TF/SF: there it is near
+    // 7 M cells, and 128^3 stays with pairs, which the long-run precision tests
+    // of that grid ask for.
     // FP16 storage rounds the fields once per pass, so pairs are the more
     // exact form (against FP64 after 40 to 60 steps from noise or a plane wave:
     // 1.19e-3 / 1.33e-3 at 80^3, 1.41e-3 / 1.67e-3 at 128^3, pairs / single):
@@ -1268,7 +1276,10 @@ int plan_sweep (fdtd_ctx *ctx)
     // (padded rows, a point source), where only the time decides.
     // FDTDB_TB2=0 / 1: never / always (test hook).
     const bool exact_pairs = ctx->kind == 2 && ctx->pz == g.n[2] && !g.cfg.point_source_mask;
-    bool tb2 = exact_pairs || !g.cfg.use_pml || g.cells >= (g.cfg.use_tfsf ? 2000000 : 15000000);
+    const int64_t line = g.n[2] <= kSweepTileZ / 2 || (g.cfg.use_pml && g.cfg.use_tfsf) ? 2000000
+                         : g.cfg.use_pml                                       ? 15000000
+                                                                               : 3000000;
+    bool tb2 = exact_pairs || (int64_t) g.cells >= line;
     if (const char *v = std::getenv ("FDTDB_TB2"))
       tb2 = std::atoi (v) != 0;
     if (!tb2)
