@@ -1142,10 +1142,12 @@ int plan_sweep (fdtd_ctx *ctx)
     }
   }
   ctx->fused.tfsf_post = ctx->band.cells > 0 ? 1 : 0;   // read only by the sweep kernels
-  // A point source as its linear response after the step (one half-step's
-  // reach: the cell and the one below it outside the PML) or after a pair
-  // (three cells below to two above).  FDTDB_POINT_FIX=0 keeps it inside the
-  // sweep (a test hook).
+  // A point source outside the sweep, its neighbourhood worked out again after
+  // the step (H reaches from one cell below the source to the source itself)
+  // or after a pair (three below to two above): those cells, and the E values
+  // one cell above them that H reads across, must be free of the PML, and of
+  // the TF/SF corrections.  FDTDB_POINT_FIX=0 keeps it inside the sweep (a
+  // test hook).
   if (g.cfg.point_source_mask && !g.cfg.use_metamaterials)
   {
     auto free_of_pml = [&] (int below, int above) {
@@ -1155,12 +1157,21 @@ int plan_sweep (fdtd_ctx *ctx)
         const int c = g.cfg.point_source[a];
         in = in && c - below >= 0 && c + above <= g.n[a] - 1;
         for (int k = 0; k < 6 && g.cfg.use_pml; ++k)
-          in = in && c - below >= ctx->fused.ilo[k][a] && c + above < ctx->fused.ihi[k][a];
+          in = in && c - below >= ctx->fused.ilo[k][a] &&
+               c + above + (k < 3 && k != a ? 1 : 0) < ctx->fused.ihi[k][a];
       }
       return in;
     };
+    bool free_of_tfsf = !g.cfg.use_tfsf || ctx->fused.tfsf_post;
+    for (const BandBox &bb : ctx->band_host)
+    {
+      bool hit = true;
+      for (int a = 0; a < 3; ++a)
+        hit = hit && bb.lo[a] <= g.cfg.point_source[a] + 1 && g.cfg.point_source[a] - 1 < bb.hi[a];
+      free_of_tfsf = free_of_tfsf && !hit;
+    }
     const char *v = std::getenv ("FDTDB_POINT_FIX");
-    if ((!v || std::atoi (v) != 0) && free_of_pml (1, 0))
+    if ((!v || std::atoi (v) != 0) && free_of_tfsf && free_of_pml (1, 0))
       ctx->ps_fix = !g.cfg.use_tfsf && free_of_pml (3, 2) ? 2 : 1;
     if (ctx->ps_fix)
       ctx->fused.ps_mask = 0;
@@ -1826,7 +1837,11 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
   if (has_cs)
   {
     for (int a = 0; a < 3; ++a)
+    {
       cfix.pos[a] = ctx->cs_pos[a];
+      cfix.ps_pos[a] = g.cfg.point_source[a];
+    }
+    cfix.ps_mask = g.cfg.point_source_mask;
     cfix.mask_e = ctx->cs_mask[0];
     cfix.mask_h = ctx->cs_mask[1];
     cfix.scale_e = (float) kEta0;
@@ -2005,10 +2020,10 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
         ctx->launches += launch_fused3d (f, ctx->d_err, s);
         ctx->step_kernel = "fused3d_regblock";
       }
-      if (has_cs)
-        ctx->launches += launch_current_fix (f, cfix, ctx->d_src + kSrcStride * i + 3, s);
       if (ctx->ps_fix)
         ctx->launches += launch_point_fix (f, pfix, ctx->d_src + kSrcStride * i + 1, kSrcStride, false, s);
+      if (has_cs)
+        ctx->launches += launch_current_fix (f, cfix, ctx->d_src + kSrcStride * i + 3, s);
       if ((r = prof_end (ctx, pe)) != FDTD_OK)
         return r;
       ctx->fcur = nw;

@@ -961,6 +961,10 @@ __global__ void current_fix_kernel (FusedParams p, CurrentFix cf, const double *
     else
       static_cast<float *> (f)[id] += d;
   };
+  // a hard point source sets its components after the current has acted
+  auto driven = [&] (const int q[3], int k) {
+    return ((cf.ps_mask >> k) & 1) && q[0] == cf.ps_pos[0] && q[1] == cf.ps_pos[1] && q[2] == cf.ps_pos[2];
+  };
   // H at cell q: the update adds S times its curl; a change dE of E
   // component k at c changes the curls of the two other H components
   // (E_CENTERED: Hx = (Ey(z+1) - Ey) - (Ez(y+1) - Ez), and its rotations)
@@ -972,12 +976,14 @@ __global__ void current_fix_kernel (FusedParams p, CurrentFix cf, const double *
     for (int a = 0; a < 3; ++a)
       if (!((p.g.drop >> a) & 1) && (q[a] < 1 || q[a] > p.g.n[a] - 2))
         return;   // a face cell: the step does not update it
+    if (driven (q, 3 + m))
+      return;
     rmw (p.h_new[m], (size_t) q[0] * st[0] + (size_t) q[1] * st[1] + q[2], S * d);
   };
   const float ie = (float) (src[0] * p.g.dx) * cf.scale_e;
   for (int k = 0; k < 3; ++k)
   {
-    if (!((cf.mask_e >> k) & 1))
+    if (!((cf.mask_e >> k) & 1) || driven (cf.pos, k))
       continue;
     const float im = p.eps ? __fdividef (2.f, p.eps[c] + p.eps[c + st[k]]) : 1.f;
     const float de = S * im * -ie;
@@ -993,7 +999,7 @@ __global__ void current_fix_kernel (FusedParams p, CurrentFix cf, const double *
   }
   const float ih = (float) (src[1] * p.g.dx) * cf.scale_h;
   for (int m = 0; m < 3; ++m)
-    if ((cf.mask_h >> m) & 1)
+    if (((cf.mask_h >> m) & 1) && !driven (cf.pos, 3 + m))
       rmw (p.h_new[m], c, S * -ih);
 }
 
@@ -1005,122 +1011,93 @@ int launch_current_fix (const FusedParams &p, const CurrentFix &cf, const double
 
 namespace {
 
-template <typename T>
-__device__ __forceinline__ void add_to (T *f, size_t id, float d);
-template <>
-__device__ __forceinline__ void add_to<float> (float *f, size_t id, float d)
-{
-  f[id] += d;
-}
-template <>
-__device__ __forceinline__ void add_to<__half> (__half *f, size_t id, float d)
-{
-  f[id] = __float2half_rn (__half2float (f[id]) + d);
-}
-
-// Response of a point source, one thread per cell of the 5^3 box around it
-// (the change travels one cell per half-step: E at the source; H there and
-// one cell below; E one cell around; H two below and one above).  In the
-// sweep a source cost its items the general class, 116 of 165 us of a
-// 256 x 224 x 240 step with one CTA at work, and kept the run from pairs;
-// this kernel takes about 4 us a step or pair.
-// Single step: dE = src - E_new, H_new += S curl dE.  Pair: the first step's
-// E at the source is worked out again from the old set, then
-//   dE1 = src1 - E1, dH1 = S curl dE1 (a driven H: src1 - H1),
-//   dE2 = dE1 + S im curl dH1 (at the source src2 - E_new), dH2 likewise.
+// The cells a point source's value reaches, one thread per cell of an 8^3 box
+// with the source at (4, 4, 4): worked out again from the old set with the
+// source in place, in the sweep's arithmetic and in FP32 between the half-steps
+// (adding the change the source makes to the sweep's result instead rounds H
+// twice, and FP16 storage has rounded E before the change is formed).  The
+// value travels one cell per half-step: E at the source; H there and one cell
+// below; in a pair then E one cell around, H two below and one above.  The box
+// holds every value these depend on; cells of it further out come out wrong and
+// are not stored.
+// Inside the sweep a source cost its items the general class, 116 of 165 us of
+// a 256 x 224 x 240 step with one CTA at work, and kept the run from pairs;
+// this kernel is one CTA's latency, about 4 us a step or pair.
 template <typename T, bool PAIR>
-__global__ void __launch_bounds__ (128) point_fix_kernel (const __grid_constant__ FusedParams p, PointFix pf,
+__global__ void __launch_bounds__ (512) point_fix_kernel (const __grid_constant__ FusedParams p, PointFix pf,
                                                           const double *src, int stride)
 {
-  constexpr int W = 5, N = W * W * W, C = (2 * W + 2) * W + 2;   // the source's index
-  __shared__ float dE[3][N], dH[3][N];
+  constexpr int W = 8, SRC = 4;
+  __shared__ float sE[3][W * W * W], sH[3][W * W * W];
   const int q = threadIdx.x;
-  const int ny = p.g.n[1], pz = p.g.pz;
-  const size_t st[3] = {(size_t) ny * pz, (size_t) pz, 1};
+  const int l[3] = {q / (W * W), q / W % W, q % W};
   const int sd[3] = {W * W, W, 1};
-  const size_t c = (size_t) pf.pos[0] * st[0] + (size_t) pf.pos[1] * st[1] + pf.pos[2];
+  const size_t st[3] = {(size_t) p.g.n[1] * p.g.pz, (size_t) p.g.pz, 1};
   const float S = p.courant;
-  const int l[3] = {q / (W * W), (q / W) % W, q % W};
-  bool upd = q < N, low = false, high = false;   // low / high: on the box's first / last cells
+  bool in = true, upd = true, low = true, high = true, at = true, e_out = true, h_out = true;
+  size_t id = 0;
   for (int a = 0; a < 3; ++a)
   {
-    const int g = pf.pos[a] + l[a] - 2;
+    const int g = pf.pos[a] + l[a] - SRC;
+    in = in && g >= 0 && g < p.g.n[a];
     upd = upd && g >= 1 && g <= p.g.n[a] - 2;
-    low = low || l[a] == 0;
-    high = high || l[a] == W - 1;
+    low = low && l[a] > 0;            // has its lower neighbours in the box
+    high = high && l[a] < W - 1;
+    at = at && l[a] == SRC;
+    e_out = e_out && l[a] >= SRC - 1 && l[a] <= SRC + 1;
+    h_out = h_out && l[a] >= SRC - (PAIR ? 2 : 1) && l[a] <= SRC + (PAIR ? 1 : 0);
+    id += (size_t) (in ? g : 0) * st[a];
   }
-  const size_t id = c + (size_t) ((l[0] - 2) * (long long) st[0] + (l[1] - 2) * (long long) st[1] + (l[2] - 2));
-  auto im = [&] (int k, size_t i) { return p.eps ? __fdividef (2.f, p.eps[i] + p.eps[i + st[k]]) : 1.f; };
-  // E component k after the first step, from the old set
-  auto e1 = [&] (int k, size_t i) -> float {
-    const int b = (k + 1) % 3, d = (k + 2) % 3;
-    const T *hb = (const T *) p.h_old[b], *hd = (const T *) p.h_old[d];
-    const float cu = (ldf (hd, i) - ldf (hd, i - st[b])) - (ldf (hb, i) - ldf (hb, i - st[d]));
-    return ldf ((const T *) p.e_old[k], i) + (S * im (k, i)) * cu;
-  };
-  // curl of dE around cell q (its upper neighbours), of dH (its lower ones)
-  auto curl_e = [&] (int m) {
-    const int b = (m + 1) % 3, d = (m + 2) % 3;
-    return (dE[b][q + sd[d]] - dE[b][q]) - (dE[d][q + sd[b]] - dE[d][q]);
-  };
-  auto curl_h = [&] (int k) {
-    const int b = (k + 1) % 3, d = (k + 2) % 3;
-    return (dH[d][q] - dH[d][q - sd[b]]) - (dH[b][q] - dH[b][q - sd[d]]);
-  };
-  if (q < N)
+  float e[3] = {0.f, 0.f, 0.f}, h[3] = {0.f, 0.f, 0.f}, im[3] = {1.f, 1.f, 1.f};
+  if (in)
     for (int k = 0; k < 3; ++k)
     {
-      dE[k][q] = 0.f;
-      dH[k][q] = 0.f;
+      e[k] = ldf ((const T *) p.e_old[k], id);
+      h[k] = ldf ((const T *) p.h_old[k], id);
+      if (p.eps && upd)
+        im[k] = __fdividef (2.f, p.eps[id] + p.eps[id + st[k]]);
     }
-  __syncthreads ();
-  if (q < 3 && ((pf.mask >> q) & 1))
-    dE[q][C] = (float) src[0] - (PAIR ? e1 (q, c) : ld_new ((const T *) p.e_new[q], c));
-  __syncthreads ();
-  if (upd && !high)
-    for (int m = 0; m < 3; ++m)
-    {
-      float d = S * curl_e (m);
-      if (PAIR && q == C && ((pf.mask >> (3 + m)) & 1))
-      {
-        const int b = (m + 1) % 3, e = (m + 2) % 3;
-        const float cu = (e1 (b, c + st[e]) - e1 (b, c)) - (e1 (e, c + st[b]) - e1 (e, c));
-        d = (float) src[1] * pf.scale_h - (ldf ((const T *) p.h_old[m], c) + S * cu);
-      }
-      dH[m][q] = d;
-    }
-  __syncthreads ();
-  if (PAIR)
-  {
-    float d[3] = {0.f, 0.f, 0.f};
-    if (upd && !low)
-      for (int k = 0; k < 3; ++k)
-      {
-        d[k] = dE[k][q] + (S * im (k, id)) * curl_h (k);
-        if (q == C && ((pf.mask >> k) & 1))
-          d[k] = (float) src[stride] - ld_new ((const T *) p.e_new[k], c);
-      }
-    if (q < N)
-      for (int k = 0; k < 3; ++k)
-        dE[k][q] = d[k];
-    __syncthreads ();
-    if (upd && !high)
-      for (int m = 0; m < 3; ++m)
-        dH[m][q] += S * curl_e (m);
-  }
-  if (!upd)
-    return;
-  const double *last = src + (PAIR ? stride : 0);
   for (int k = 0; k < 3; ++k)
   {
-    if (q == C && ((pf.mask >> k) & 1))
-      stf ((T *) p.e_new[k], c, (float) last[0]);
-    else if (dE[k][q] != 0.f)
-      add_to ((T *) p.e_new[k], id, dE[k][q]);
-    if (q == C && ((pf.mask >> (3 + k)) & 1))
-      stf ((T *) p.h_new[k], c, (float) last[1] * pf.scale_h);
-    else if (dH[k][q] != 0.f)
-      add_to ((T *) p.h_new[k], id, dH[k][q]);
+    sE[k][q] = e[k];
+    sH[k][q] = h[k];
+  }
+  __syncthreads ();
+  for (int s = 0; s < (PAIR ? 2 : 1); ++s)
+  {
+    for (int k = 0; k < 3; ++k)
+    {
+      const int b = (k + 1) % 3, d = (k + 2) % 3;
+      if (upd && low)
+      {
+        const float cu = (h[d] - sH[d][q - sd[b]]) - (h[b] - sH[b][q - sd[d]]);
+        e[k] = e[k] + (S * im[k]) * cu;
+      }
+      if (at && ((pf.mask >> k) & 1))
+        e[k] = (float) src[s * stride];
+      sE[k][q] = e[k];
+    }
+    __syncthreads ();
+    for (int m = 0; m < 3; ++m)
+    {
+      const int b = (m + 1) % 3, d = (m + 2) % 3;
+      if (upd && high)
+      {
+        const float cu = (sE[b][q + sd[d]] - e[b]) - (sE[d][q + sd[b]] - e[d]);
+        h[m] = h[m] + S * cu;
+      }
+      if (at && ((pf.mask >> (3 + m)) & 1))
+        h[m] = (float) src[s * stride + 1] * pf.scale_h;
+      sH[m][q] = h[m];
+    }
+    __syncthreads ();
+  }
+  for (int k = 0; k < 3; ++k)
+  {
+    if (upd && (PAIR ? e_out : at))
+      stf ((T *) p.e_new[k], id, e[k]);
+    if (upd && h_out)
+      stf ((T *) p.h_new[k], id, h[k]);
   }
 }
 
@@ -1132,14 +1109,14 @@ int launch_point_fix (const FusedParams &p, const PointFix &pf, const double *sr
   if (p.fp16)
   {
     if (pair)
-      point_fix_kernel<__half, true><<<1, 128, 0, s>>> (p, pf, src, stride);
+      point_fix_kernel<__half, true><<<1, 512, 0, s>>> (p, pf, src, stride);
     else
-      point_fix_kernel<__half, false><<<1, 128, 0, s>>> (p, pf, src, stride);
+      point_fix_kernel<__half, false><<<1, 512, 0, s>>> (p, pf, src, stride);
   }
   else if (pair)
-    point_fix_kernel<float, true><<<1, 128, 0, s>>> (p, pf, src, stride);
+    point_fix_kernel<float, true><<<1, 512, 0, s>>> (p, pf, src, stride);
   else
-    point_fix_kernel<float, false><<<1, 128, 0, s>>> (p, pf, src, stride);
+    point_fix_kernel<float, false><<<1, 512, 0, s>>> (p, pf, src, stride);
   return 1;
 }
 

@@ -101,14 +101,15 @@ struct CurrentFix
   int pos[3];
   int mask_e, mask_h;          // bit c: a current on component c of the family
   float scale_e, scale_h;      // I dx -> curl units (eta0 for E, 1 for H)
+  int ps_pos[3], ps_mask;      // hard point source: its components are left as they are
 };
 int launch_current_fix (const FusedParams &p, const CurrentFix &cf, const double *src, cudaStream_t s);
 
 // Hard point source of a one-sweep step (or of a pair of steps): the sweep
-// updates every cell without it, and the fields take the linear response of
-// the change the source makes at its cell (launch_point_fix in fused3d.cu).
-// Used when the cells the response reaches are outside the PML, not Drude
-// cells, and for a pair outside the TF/SF band.
+// updates every cell without it, and the cells the source's value reaches are
+// worked out again with it (launch_point_fix in fused3d.cu).  Used when every
+// cell that takes part is outside the PML and the TF/SF band, and no Drude
+// cell.
 struct PointFix
 {
   int pos[3];
