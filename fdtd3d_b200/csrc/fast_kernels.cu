@@ -230,8 +230,13 @@ __device__ __forceinline__ void fast_component (const FastHalf &p, int ci, int *
   st (F, id, f);
 }
 
-template <typename T>
-__global__ void __launch_bounds__ (256) fast_half_kernel (FastHalf p, int *err)
+// BLOCKS: CTAs an SM is to hold.  The kernel waits for memory, so large grids
+// take six (40 registers, 44 B of spills) and grids that four hold at once
+// four (59 registers, none).  us per step, left to the compiler (56 registers
+// in FP16 storage, 48 in FP32) / now: H_CENTERED 200^3 FP16 617 / 506, FP32 504 /
+// 489, 61^3 31.4 / 28.1, 30.3 / 27.4; 2-D with a DFT 2048^2 FP16 176 / 158.
+template <typename T, int BLOCKS>
+__global__ void __launch_bounds__ (256, BLOCKS) fast_half_kernel (FastHalf p, int *err)
 {
   // interior cells: 1 .. n - 2 on every axis a mode keeps, 0 on a dropped one
   const int ix = (p.g.drop & 1) ? 1 : p.g.n[0] - 2;
@@ -498,10 +503,10 @@ int launch_fast_half (const FastHalf &p, int *err, int sm_count, cudaStream_t s)
     blocks = cap;
   if (blocks < 1)
     blocks = 1;
-  if (p.fp16)
-    fast_half_kernel<__half><<<(unsigned) blocks, 256, 0, s>>> (p, err);
-  else
-    fast_half_kernel<float><<<(unsigned) blocks, 256, 0, s>>> (p, err);
+  const bool few = blocks <= 4 * (int64_t) sm_count;
+  auto kern = p.fp16 ? (few ? fast_half_kernel<__half, 4> : fast_half_kernel<__half, 6>)
+                     : (few ? fast_half_kernel<float, 4> : fast_half_kernel<float, 6>);
+  kern<<<(unsigned) blocks, 256, 0, s>>> (p, err);
   return 1;
 }
 

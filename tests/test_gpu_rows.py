@@ -52,3 +52,30 @@ def test_padded_rows_match_fp64(fdtd, nz, prec, tol):
         assert _family(out[prec], out[0], fam) <= tol, (nz, fam, _family(out[prec], out[0], fam))
     assert np.linalg.norm(spectrum[prec] - spectrum[0]) <= tol * np.linalg.norm(spectrum[0])
     assert abs(energy[prec] / energy[0] - 1) <= tol
+
+
+# a mu map takes the per-cell kernels: rows of nz cells and padded ones, grids
+# that four CTAs an SM hold at once (up to 151 552 updated cells on 148) and
+# larger ones
+@pytest.mark.parametrize("shape", [(18, 15, 31), (18, 15, 36), (18, 15, 37), (18, 15, 40), (18, 15, 63), (66, 39, 66),
+                                   (66, 40, 66), (61, 62, 63)])
+@pytest.mark.parametrize("prec,tol", [(1, 1e-5), (2, 2e-2)])
+def test_per_cell_kernels_on_either_row(fdtd, shape, prec, tol):
+    nz = shape[2]
+    rng = np.random.default_rng(nz)
+    fields = {c: np.zeros(shape) for c in COMPS}
+    for c in COMPS:
+        fields[c][1:-1, 1:-1, 1:-1] = rng.standard_normal(tuple(n - 2 for n in shape)) / (1 if c[0] == "E" else ETA0)
+    maps = {m: 1 + np.kron(rng.uniform(0, 3, [n // 5 + 1 for n in shape]), np.ones((5, 5, 5))) for m in ("eps", "mu")}
+    maps = {m: v[:shape[0], :shape[1], :nz] for m, v in maps.items()}
+    maps = {m: v.astype(np.float32).astype(np.float64) for m, v in maps.items()}
+    out = {}
+    for p in (0, prec):
+        with fdtd.Simulation(materials=maps, precision=p, mode=3, size=shape, use_pml=True, pml=3) as sim:
+            for c, v in fields.items():
+                sim.set_field(c, v)
+            sim.step(12, t_start=30)
+            out[p] = {c: sim.field(c) for c in COMPS}
+            assert not p or sim.step_kernel == "per_cell", sim.step_kernel
+    for fam in "EH":
+        assert _family(out[prec], out[0], fam) <= tol, (nz, fam, _family(out[prec], out[0], fam))
