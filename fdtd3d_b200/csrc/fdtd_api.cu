@@ -1663,6 +1663,34 @@ bool tile2d_ready (const fdtd_ctx *ctx)
   return true;
 }
 
+// Whether a single step of a 2-D mode (a call of one step, the rest of a longer
+// one) takes the per-cell kernels: a tile computes its halo of seven cells
+// whatever the number of steps, which one step does not earn back on a large
+// grid where the arithmetic (FP64) or the border terms weigh.  us per step in
+// calls of one step, cells / tiles, PML, n^2 cells:
+//  FP64: 256 16 / 15, 384 21 / 24, 2048 270 / 302, 8192 2370 / 4540; with
+//   TF/SF 30 / 36, 299 / 405, 2530 / 6050; no PML 2048 210 / 177, 3000 294 /
+//   368, 8192 1220 / 2670;
+//  FP32, TF/SF: 192 23 / 15 (small tiles, all at once), 256 23 / 32, 512 32 /
+//   31, 4096 521 / 645; without TF/SF 512 21 / 15, 8192 1820 / 1300;
+//  FP16 storage as FP32, but with an eps map 4096 536 / 532, 8192 1833 / 2095
+//   (without 1662 / 1440).
+// (Two steps in FP64 are two launches of one; three steps and more are faster
+// in tiles at every size.)
+bool step2d_by_cells (const fdtd_ctx *ctx)
+{
+  const Geometry &g = ctx->g;
+  if (ctx->kind == 0)
+    return g.cells >= (g.cfg.use_pml || g.cfg.use_tfsf ? 100000 : 6000000);
+  if (g.cfg.use_tfsf)
+  {
+    const int ua = g.drop == 1 ? 1 : 0, va = g.drop == 4 ? 1 : 2;
+    const int own = 32 - 2 * kTileSteps;
+    return (int64_t) ((g.n[ua] + own - 1) / own) * ((g.n[va] + own - 1) / own) > ctx->sm_count;
+  }
+  return ctx->kind == 2 && g.cells >= 32000000 && (ctx->mat32[0] || ctx->mat32[1] || g.dmp);
+}
+
 // Steps i .. i + steps - 1 of the call in one launch (t > 0).
 int tile2d_run (fdtd_ctx *ctx, uint32_t i, int steps)
 {
@@ -1858,11 +1886,14 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
       int steps = (int) std::min<uint32_t> (kTileSteps, n - i);
       if (ctx->kind == 0 && steps % 2 == 0)
         --steps;
-      if ((r = tile2d_run (ctx, i, steps)) != FDTD_OK)
-        return r;
-      ctx->prev_src = 0;
-      i += steps - 1;
-      continue;
+      if (steps > 1 || !step2d_by_cells (ctx))
+      {
+        if ((r = tile2d_run (ctx, i, steps)) != FDTD_OK)
+          return r;
+        ctx->prev_src = 0;
+        i += steps - 1;
+        continue;
+      }
     }
     if (fused && t > 0)
     {

@@ -89,3 +89,44 @@ def test_fast_forms_match_fp64(fdtd, mode, size, source, prec, tol):
             g = np.concatenate([got[c].ravel() for c in got if c[0] == fam])
             w = np.concatenate([want[c].ravel() for c in want if c[0] == fam])
             assert np.linalg.norm(g - w) <= tol * np.linalg.norm(w), (layout, fam)
+
+
+# one step of a call by the per-cell kernels (two launches or more) or by tiles
+# (one), on either side of the lines; 8 steps of FP64 are 7 and 1
+@pytest.mark.parametrize("prec,size,kw,cells", [
+    (0, (316, 316), dict(use_pml=True, pml=8), False),
+    (0, (320, 316), dict(use_pml=True, pml=8), True),
+    (0, (320, 316), dict(), False),
+    (1, (216, 216), "tfsf", False),
+    (1, (217, 216), "tfsf", True),
+    (2, (217, 216), "tfsf", True),
+    (1, (420, 380), dict(use_pml=True, pml=8), False),
+    (2, (420, 380), dict(use_pml=True, pml=8), False),
+])
+def test_single_steps_by_cells_or_by_tiles(fdtd, prec, size, kw, cells):
+    if kw == "tfsf":
+        kw = dict(use_pml=True, pml=8, use_tfsf=True, tfsf_left=14, tfsf_right=14, teta=90, phi=25, psi=90)
+    rng = np.random.default_rng(8)
+    fields = {c: np.zeros(size) for c in ("Ez", "Hx", "Hy")}
+    for c, v in fields.items():
+        v[1:-1, 1:-1] = rng.standard_normal([n - 2 for n in size]) / (1 if c[0] == "E" else 376.73)
+    eps = {"eps": 1 + np.kron(rng.integers(0, 4, [n // 8 + 1 for n in size]), np.ones((8, 8)))[: size[0], : size[1]]}
+    got = []
+    for calls in ([1] * 9, [8, 1], [9]):
+        with fdtd.Simulation(mode=2, size=size, precision=prec, materials=eps, **kw) as sim:
+            for c, v in fields.items():
+                sim.set_field(c, v)
+            sim.t = 50
+            sim.step(3)
+            for n in calls:
+                before = sim.launch_count()
+                sim.step(n)
+                if n == 1:
+                    assert (sim.launch_count() - before > 1) == cells, sim.launch_count() - before
+            got.append({c: sim.field(c) for c in fields})
+    for g in got[1:]:
+        for c in fields:
+            if prec == 0:
+                assert np.array_equal(g[c].view(np.int64), got[0][c].view(np.int64)), c
+            else:   # (12 steps of FP32; FP16 storage rounds once per launch of tiles)
+                assert np.linalg.norm(g[c] - got[0][c]) <= (1e-6 if prec == 1 else 5e-3) * np.linalg.norm(got[0][c]), c
