@@ -421,8 +421,9 @@ class Simulation:
 
 
 class Batch:
-    """Many 2-D TMz simulations of different sizes advanced by one persistent
-    kernel launch per ``step`` call (captured in a CUDA graph), FP32.
+    """Many 2-D TMz simulations of different sizes advanced together, by one
+    persistent kernel launch per ``step`` call (captured in a CUDA graph) or, in
+    calls of up to three steps, by one launch per step; FP32.
 
     ``sizes`` is a list of (nx, ny); every instance has its point source at
     its centre and shares the physics given as keyword arguments."""

@@ -1,5 +1,6 @@
 // tmz_batch.cu - many 2-D TMz simulations of uneven sizes in one persistent
-// kernel launch (captured in a CUDA graph), FP32.
+// kernel launch (captured in a CUDA graph), FP32; calls of a few steps in a
+// launch per step.
 //
 // Every instance is an fdtd3d Dim2_TMz E_CENTERED run (Ez, Hx, Hy) with PML,
 // its own eps map and a point source at its centre; they share dx, Courant
@@ -14,7 +15,8 @@
 // memory, the halo recomputed), fields double buffered; a grid-wide barrier
 // separates rounds.  One step per round (a warp per 30-cell strip, fields
 // streamed from L2 / HBM) was bound by bytes in flight and the barrier: 20
-// instances, 6.08 M cells: 82 us per step, 49 us now.
+// instances, 6.08 M cells: 82 us per step, 49 us now.  Calls of up to three
+// steps go by cells instead, a launch per step (tmz_cells_kernel).
 // The barrier is a bounded spin on a global generation counter (globaltimer
 // timeout -> error flag, every CTA leaves); the kernel is launched
 // cooperatively so all CTAs are co-resident.
@@ -55,6 +57,14 @@ struct TileDev
 {
   int inst, u0, v0;                   // corner of the tile, halo included
 };
+
+// A CTA's part of a step by cells: kCellRows rows from u0, kCellCols columns
+// from v0.
+struct PatchDev
+{
+  int inst, u0, v0;
+};
+constexpr int kCellWarps = 8, kCellRun = 4, kCellRows = kCellWarps * kCellRun, kCellCols = 31;
 
 struct BatchParams
 {
@@ -174,6 +184,112 @@ __global__ void __launch_bounds__ (kTileThreads, 1) tmz_batch_kernel (BatchParam
   }
 }
 
+// The arenas of a step by cells: Ez, Hx, Hy and their auxiliaries, from one set
+// into the other.
+struct CellArrays
+{
+  const float *in[3], *xin[3];
+  float *out[3], *xout[3];
+  const float *eps, *tab;
+  float courant;
+  int use_pml;
+};
+
+// F after a curl of `cu` (m: 1 / eps or 1), and X where the cell has PML.
+__device__ __forceinline__ float cell_update (bool pml, float f, float cu, float m, float S, float ca1, float sq1,
+                                              float p5, float q5, float g4p, float g4m, const float *xo, float *xn,
+                                              int64_t id, bool store)
+{
+  if (!pml)
+    return f + S * m * cu;
+  const float o = xo[id], n = ca1 * o + sq1 * cu;
+  if (store)
+    xn[id] = n;
+  return p5 * f + (g4p * n - g4m * o) * q5 * m;
+}
+
+// One time step of every instance (update = 0: only the sources): a thread Ez of
+// four cells of a column and, again, of the one after them, then H of the four;
+// Ez of the next column by a shuffle (lane 31 has no cell of its own).  No
+// thread waits for another, and every value is read and written once.  The form
+// of calls of a few steps, whose tiles would be set up, read and written for
+// little.
+__global__ void __launch_bounds__ (32 * kCellWarps)
+    tmz_cells_kernel (const __grid_constant__ CellArrays p, const InstDev *inst, const PatchDev *patches,
+                      const double *src, int update)
+{
+  const PatchDev td = patches[blockIdx.x];
+  const InstDev &in = inst[td.inst];
+  const int nx = in.nx, ny = in.ny, v = td.v0 + threadIdx.x, u0 = td.u0 + kCellRun * threadIdx.y;
+  const int64_t base = in.off + (int64_t) u0 * ny + v;
+  const int su = in.ps && v == ny / 2 ? nx / 2 : -1;
+  if (!update)
+  {
+    if (threadIdx.x < kCellCols && su >= u0 && su < u0 + kCellRun)
+      const_cast<float *> (p.in[0])[base + (int64_t) (su - u0) * ny] = (float) *src;
+    return;
+  }
+  if (u0 > nx - 2)
+    return;   // (the whole warp)
+  const float S = p.courant;
+  const bool pml = p.use_pml, column = v <= ny - 2, own = column && threadIdx.x < kCellCols;
+  // tables of the instance: Ez ca1, sq1 (x), p5, q5 (y); Hx g4p, g4m (x), ca1,
+  // sq1 (y); Hy p5, q5 (x), g4p, g4m (y)
+  const float *const T = p.tab + in.tab;
+  const int t1 = 2 * (nx + ny), t2 = 2 * t1;
+  float e[kCellRun + 1], hx[kCellRun + 1], hy[kCellRun + 2], left[kCellRun + 1], m[kCellRun + 1];
+  hy[0] = column ? p.in[2][base - ny] : 0.f;
+#pragma unroll
+  for (int r = 0; r <= kCellRun; ++r)
+  {
+    const int64_t id = base + (int64_t) r * ny;
+    const bool there = v <= ny - 1 && u0 + r <= nx - 1, on = column && u0 + r <= nx - 2;
+    e[r] = there ? p.in[0][id] : 0.f;
+    hx[r] = on ? p.in[1][id] : 0.f;
+    left[r] = on ? p.in[1][id - 1] : 0.f;
+    hy[r + 1] = on ? p.in[2][id] : 0.f;
+    m[r] = on ? p.eps[id] : 1.f;
+  }
+  {
+    const bool yin = v >= in.ilo[0][1] && v < in.ihi[0][1];
+    const int lo = in.ilo[0][0], hi = in.ihi[0][0];
+#pragma unroll
+    for (int r = 0; r <= kCellRun; ++r)
+    {
+      const int u = u0 + r;
+      if (!column || u > nx - 2)
+        continue;
+      const int64_t id = base + (int64_t) r * ny;
+      const bool pm = pml && !(yin && u >= lo && u < hi), store = own && r < kCellRun;
+      e[r] = cell_update (pm, e[r], (hy[r + 1] - hy[r]) - (hx[r] - left[r]), 1.f / m[r], S, pm ? T[u] : 1.f,
+                          pm ? T[nx + u] : S, pm ? T[2 * nx + v] : 1.f, pm ? T[2 * nx + ny + v] : 1.f, 1.f, 1.f,
+                          p.xin[0], p.xout[0], id, store);
+      if (u == su)
+        e[r] = (float) *src;
+      if (store)
+        p.out[0][id] = e[r];
+    }
+  }
+  const bool yx = v >= in.ilo[1][1] && v < in.ihi[1][1], yy = v >= in.ilo[2][1] && v < in.ihi[2][1];
+  const int xlo = in.ilo[1][0], xhi = in.ihi[1][0], ylo = in.ilo[2][0], yhi = in.ihi[2][0];
+#pragma unroll
+  for (int r = 0; r < kCellRun; ++r)
+  {
+    const int u = u0 + r;
+    const float up = __shfl_down_sync (0xffffffffu, e[r], 1);
+    if (!own || u > nx - 2)
+      continue;
+    const int64_t id = base + (int64_t) r * ny;
+    const bool px = pml && !(yx && u >= xlo && u < xhi), py = pml && !(yy && u >= ylo && u < yhi);
+    p.out[1][id] = cell_update (px, hx[r], e[r] - up, 1.f, S, px ? T[t1 + 2 * nx + v] : 1.f,
+                                px ? T[t1 + 2 * nx + ny + v] : S, 1.f, 1.f, px ? T[t1 + u] : 1.f,
+                                px ? T[t1 + nx + u] : 1.f, p.xin[1], p.xout[1], id, true);
+    p.out[2][id] = cell_update (py, hy[r + 1], e[r + 1] - e[r], 1.f, S, 1.f, S, py ? T[t2 + u] : 1.f,
+                                py ? T[t2 + nx + u] : 1.f, py ? T[t2 + 2 * nx + v] : 1.f,
+                                py ? T[t2 + 2 * nx + ny + v] : 1.f, p.xin[2], p.xout[2], id, true);
+  }
+}
+
 }  // namespace
 
 }  // namespace fdtdb
@@ -197,6 +313,9 @@ struct fdtd_batch
   size_t stage_cells = 0;
   fdtdb::TileDev *d_tiles = nullptr;
   int ntiles = 0;
+  fdtdb::PatchDev *d_patches = nullptr;
+  fdtdb::InstDev *d_geo = nullptr;
+  int npatches = 0;
   float *d_tab = nullptr;
   float *ez[2] = {}, *hx[2] = {}, *hy[2] = {}, *aez[2] = {}, *ahx[2] = {}, *ahy[2] = {};
   float *eps = nullptr;
@@ -206,8 +325,9 @@ struct fdtd_batch
   unsigned *d_generation = nullptr;
   int *d_err = nullptr;
   int cur = 0;
-  // launch shape (autotuned): tile height in x (64: 64 x 64 cells, 32: 32 x
+  // launch shape of the tiles (autotuned): tile height in x (64: 64 x 64 cells, 32: 32 x
   // 32, halo included), CTAs per SM
+  bool tuning = false;                // every call in tiles
   int x_chunk = 64;
   int ctas_per_sm = 1;
   // graph of (source upload, counter reset, persistent kernel)
@@ -354,10 +474,42 @@ int max_ctas (int tile)
   return per_sm;
 }
 
-// Enqueues one launch (source upload, counter reset, cooperative kernel).
+// Whether a call of n steps takes them by cells (tmz_cells_kernel).  us per
+// call of 1, 2, 3, 4, 5 steps, PML, cells / tiles: one instance of 512^2 25 / 38,
+// 34 / 40, 44 / 42, 52 / 45, 64 / 48; 20 of 100 .. 1000 a side (4.5 M cells) 69 /
+// 206, 120 / 220, 173 / 235, 223 / 251, 277 / 265; two of 2048^2 87 / 312, 157 /
+// 332, 230 / 351, 299 / 372, 373 / 392.
+bool by_cells (const fdtd_batch *b, uint32_t n)
+{
+  return n <= 3 && !b->tuning;
+}
+
+// Enqueues one call (source upload, then counter reset and cooperative kernel,
+// or the steps by cells).
 int enqueue (fdtd_batch *b, uint32_t t_start, uint32_t n)
 {
   BCK (cudaMemcpyAsync (b->d_src + 1, b->h_src, (size_t) n * sizeof (double), cudaMemcpyHostToDevice, b->stream));
+  if (by_cells (b, n))
+  {
+    int cur = b->cur;
+    for (uint32_t s = 0; s < n; ++s)
+    {
+      const int o = cur, w = 1 - cur, update = t_start + s > 0;
+      const fdtdb::CellArrays p = {{b->ez[o], b->hx[o], b->hy[o]},
+                                   {b->aez[o], b->ahx[o], b->ahy[o]},
+                                   {b->ez[w], b->hx[w], b->hy[w]},
+                                   {b->aez[w], b->ahx[w], b->ahy[w]},
+                                   b->eps,
+                                   b->d_tab,
+                                   b->tab_host[1],
+                                   b->base.use_pml};
+      fdtdb::tmz_cells_kernel<<<b->npatches, dim3 (32, fdtdb::kCellWarps), 0, b->stream>>> (
+          p, b->d_geo, b->d_patches, b->d_src + 1 + s, update);
+      cur ^= update;
+    }
+    BCK (cudaGetLastError ());
+    return FDTD_OK;
+  }
   BCK (cudaMemsetAsync (b->d_counters, 0, 3 * sizeof (unsigned), b->stream));
   BatchParams p = params (b, t_start, n);
   void *args[] = {&p};
@@ -384,11 +536,11 @@ int enqueue (fdtd_batch *b, uint32_t t_start, uint32_t n)
 // Cells of the read-out's staging buffer at most (64 MB; no row is longer).
 constexpr size_t kStageCells = (size_t) 1 << 23;
 
-// Rounds of a launch: the buffer set changes with each.
-uint32_t batch_rounds (uint32_t t_start, uint32_t n)
+// Rounds of a call (by cells: its steps): the buffer set changes with each.
+uint32_t batch_rounds (const fdtd_batch *b, uint32_t t_start, uint32_t n)
 {
   const uint32_t steps = n - (t_start == 0 ? 1 : 0);
-  return (steps + fdtdb::kTileSteps - 1) / fdtdb::kTileSteps;
+  return by_cells (b, n) ? steps : (steps + fdtdb::kTileSteps - 1) / fdtdb::kTileSteps;
 }
 
 }  // namespace
@@ -580,6 +732,18 @@ int create_batch (fdtd_batch *b, const fdtd_config *base, int count, const int *
                           b->stream));
     BCK (cudaStreamSynchronize (b->stream));
   }
+  std::vector<PatchDev> patches;
+  for (int i = 0; i < count; ++i)
+    for (int u = 1; u <= b->inst[i].nx - 2; u += kCellRows)
+      for (int v = 1; v <= b->inst[i].ny - 2; v += kCellCols)
+        patches.push_back ({i, u, v});
+  b->npatches = (int) patches.size ();
+  BALLOC (b->d_geo, b->inst.size () * sizeof (InstDev));
+  BCK (cudaMemcpyAsync (b->d_geo, b->inst.data (), b->inst.size () * sizeof (InstDev), cudaMemcpyHostToDevice,
+                        b->stream));
+  BALLOC (b->d_patches, patches.size () * sizeof (PatchDev));
+  BCK (cudaMemcpyAsync (b->d_patches, patches.data (), patches.size () * sizeof (PatchDev), cudaMemcpyHostToDevice,
+                        b->stream));
   BALLOC (b->d_counters, 4 * sizeof (unsigned));
   BALLOC (b->d_generation, sizeof (unsigned));
   BALLOC (b->d_err, sizeof (int));
@@ -675,7 +839,7 @@ int step_batch (fdtd_batch *b, uint32_t t_start, uint32_t n, bool allow_graph)
       return r;
   }
   BCK (cudaEventRecord (b->ev1, b->stream));
-  if (batch_rounds (t_start, n) & 1u)
+  if (batch_rounds (b, t_start, n) & 1u)
     b->cur ^= 1;
   return FDTD_OK;
 }
@@ -817,7 +981,9 @@ int fdtd_batch_tune (fdtd_batch *b, int steps, int *choice)
       if (s > max_ctas (c))
         continue;
       b->ctas_per_sm = s;
+      b->tuning = true;
       r = step_batch (b, 1, (uint32_t) steps, false);
+      b->tuning = false;
       if (r != FDTD_OK)
         return r;
       BCK (cudaStreamSynchronize (b->stream));
