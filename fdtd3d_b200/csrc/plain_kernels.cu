@@ -651,7 +651,7 @@ int launch_plain_march (const PlainHalf &p, const PlainTabs &t, const IncidentJo
   // its planes and the start of a column (about three planes' time)
   int chunk = 4;
   double best = 1e300;
-  for (int c : {2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
+  for (int c : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
   {
     const int m = (planes + c - 1) / c, even = (planes + m - 1) / m;
     const double waves = std::max (1.0, (double) col_blocks * m / ((double) sm_count * per_sm));

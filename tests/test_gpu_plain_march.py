@@ -11,6 +11,12 @@ pytestmark = pytest.mark.gpu
 COMPS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
 
 
+@pytest.fixture(autouse=True)
+def _columns_at_every_size(monkeypatch):
+    """The columns' edges are at small sizes, which take the per-cell kernel by default."""
+    monkeypatch.setenv("FDTDB_MARCH", "1")
+
+
 def _maps(shape, seed):
     rng = np.random.default_rng(seed)
     blocks = rng.uniform(1.0, 4.0, tuple(n // 4 + 1 for n in shape))
@@ -104,3 +110,26 @@ def test_material_of_minus_one(fdtd, where, pml, which):
             got, want = sim.field(c), o.field(c)
             assert np.array_equal(got.view(np.int64), want.view(np.int64)), (c, np.max(np.abs(got - want)))
     o.close()
+
+
+# 40000 cells: the default route on either side of the line, with its incident
+# grid, against the other one
+@pytest.mark.parametrize("shape", [(33, 34, 35), (33, 34, 36), (40, 40, 25)])
+def test_columns_or_cells_by_size(fdtd, monkeypatch, shape):
+    kw = dict(mode=3, size=shape, use_pml=True, pml=4, use_tfsf=True, tfsf_left=7, tfsf_right=7, teta=35, phi=50, psi=20)
+    out, launches = [], []
+    for march in (None, "0", "1"):
+        monkeypatch.delenv("FDTDB_MARCH", raising=False)
+        if march:
+            monkeypatch.setenv("FDTDB_MARCH", march)
+        with fdtd.Simulation(materials={"eps": _maps(shape, 1)}, **kw) as sim:
+            sim.step(20)
+            before = sim.launch_count()
+            sim.step(5)
+            launches.append(sim.launch_count() - before)
+            out.append({c: sim.field(c) for c in COMPS})
+    # (by cells the incident grid's two updates are launches of their own)
+    assert launches[1] == 2 * launches[2] and launches[0] == launches[2 if np.prod(shape) >= 40000 else 1], launches
+    for got in out[1:]:
+        for c in COMPS:
+            assert np.array_equal(got[c].view(np.int64), out[0][c].view(np.int64)), c
