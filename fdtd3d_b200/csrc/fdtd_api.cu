@@ -206,6 +206,9 @@ struct fdtd_ctx
   // each, and a context holds 30 to 90 arrays
   char *slab = nullptr;
   size_t slab_left = 0;
+  // 2-D FP32 / FP16: the buffer sets' allocations; the set the fields are not
+  // in only serves the several-step launches and is given up for want of memory
+  void *set_slab[2] = {nullptr, nullptr};
 
   // field-kernel timing
   bool profiling = false;
@@ -236,13 +239,39 @@ constexpr size_t slab_size (size_t bytes)
   return (bytes + 255) & ~(size_t) 255;
 }
 
+// Gives up the spare buffer set of a 2-D run (its steps go by cells from then
+// on); false if there is none.
+bool drop_spare_set (fdtd_ctx *ctx)
+{
+  const int spare = 1 - ctx->fcur;
+  if (!ctx->set_slab[0] || !ctx->set_slab[1] || cudaStreamSynchronize (ctx->stream) != cudaSuccess)
+    return false;
+  ctx->allocs.erase (std::find (ctx->allocs.begin (), ctx->allocs.end (), ctx->set_slab[spare]));
+  cudaFree (ctx->set_slab[spare]);
+  ctx->set_slab[spare] = nullptr;
+  for (int k = 0; k < 6; ++k)
+  {
+    ctx->ffb[spare][k] = nullptr;
+    ctx->auxb[spare][k] = nullptr;
+  }
+  return true;
+}
+
+cudaError_t device_malloc_or_spare (fdtd_ctx *ctx, void **p, size_t bytes)
+{
+  cudaError_t e = device_malloc (p, bytes);
+  if (e == cudaErrorMemoryAllocation && drop_spare_set (ctx))
+    e = device_malloc (p, bytes);
+  return e;
+}
+
 // Takes `bytes` (zeroed) from the device in one allocation for the DALLOCs
 // that follow; what does not fit is allocated by itself.
 int slab_reserve (fdtd_ctx *ctx, size_t bytes)
 {
   ctx->slab_left = 0;
   void *p = nullptr;
-  cudaError_t e = device_malloc (&p, bytes);
+  cudaError_t e = device_malloc_or_spare (ctx, &p, bytes);
   if (e != cudaSuccess)
     return fail (ctx, FDTD_ERR_NOMEM, std::string ("cudaMalloc: ") + cudaGetErrorString (e));
   ctx->allocs.push_back (p);
@@ -271,7 +300,7 @@ int dalloc (fdtd_ctx *ctx, void **p, size_t bytes, bool zero = true)
     ctx->slab_left -= need;
     return FDTD_OK;
   }
-  cudaError_t e = device_malloc (p, bytes ? bytes : 16);
+  cudaError_t e = device_malloc_or_spare (ctx, p, bytes ? bytes : 16);
   if (e != cudaSuccess)
   {
     *p = nullptr;
@@ -627,13 +656,21 @@ int alloc_fast (fdtd_ctx *ctx)
   // E_CENTERED stencil on cell-centred materials; H_CENTERED, double material
   // precision and the 2-D / 1-D modes run the per-cell kernels on one buffer set
   ctx->has_second = g.drop == 0 && g.cfg.layout == 0 && !g.dmp;
-  // (the 2-D modes' several-step launches write a second set as well)
+  // (the 2-D modes' several-step launches write a second set as well; a grid
+  // that leaves no room for it steps by cells)
   size_t comps = 0;
   for (int k = 0; k < 6; ++k)
     comps += g.comp[k].exists ? 1 : 0;
   for (int b = 0; b < (ctx->has_second || tile2d_mode (g) ? 2 : 1); ++b)
   {
-    SLAB (comps * (slab_size (n * elem_size (ctx->kind)) + (g.cfg.use_pml ? slab_size (n * sizeof (float)) : 0)));
+    const int r = slab_reserve (
+        ctx, comps * (slab_size (n * elem_size (ctx->kind)) + (g.cfg.use_pml ? slab_size (n * sizeof (float)) : 0)));
+    if (r == FDTD_ERR_NOMEM && b == 1 && !ctx->has_second)
+      break;
+    if (r != FDTD_OK)
+      return r;
+    if (tile2d_mode (g))
+      ctx->set_slab[b] = ctx->allocs.back ();
     for (int k = 0; k < 6; ++k)
     {
       if (!g.comp[k].exists)
@@ -1363,7 +1400,7 @@ int plan_sweep (fdtd_ctx *ctx)
   return FDTD_OK;
 }
 
-int create_impl (const fdtd_config *cfg, int device, fdtd_ctx *ctx)
+int create_impl (const fdtd_config *cfg, int device, fdtd_ctx *ctx, bool pad)
 {
   std::string err = build_geometry (*cfg, ctx->g);
   if (!err.empty ())
@@ -1394,7 +1431,7 @@ int create_impl (const fdtd_config *cfg, int device, fdtd_ctx *ctx)
         ctx->cs_mask[k / 3] |= 1 << (k % 3);
   }
   ctx->kind = kind_of (cfg->precision);
-  ctx->pz = row_pitch (ctx->g, ctx->kind);
+  ctx->pz = pad ? row_pitch (ctx->g, ctx->kind) : ctx->g.n[2];
   ctx->scells = (size_t) ctx->g.n[0] * ctx->g.n[1] * ctx->pz;
   ctx->eta0 = ctx->kind == 0 ? 1.0 : kEta0;
   CK (cudaSetDevice (device));
@@ -1665,11 +1702,13 @@ IncidentJob incident_h_job (fdtd_ctx *ctx)
 
 // Whether this call's steps may take the 2-D several-step launches: nothing
 // reads the fields between the steps (DFT, kept levels), no J / M current,
-// and a point source on an updated cell.
+// a point source on an updated cell, and a second buffer set.
 bool tile2d_ready (const fdtd_ctx *ctx)
 {
   const Geometry &g = ctx->g;
   if (!tile2d_mode (g) || ctx->cs_mask[0] || ctx->cs_mask[1] || ctx->dft_comp >= 0 || (ctx->kind && ctx->keep_prev))
+    return false;
+  if (ctx->kind && !ctx->set_slab[1 - ctx->fcur])
     return false;
   if (g.cfg.point_source_mask)
     for (int a = 0; a < 3; ++a)
@@ -2199,22 +2238,34 @@ int fdtd_create (const fdtd_config *cfg, int device, fdtd_ctx **out)
     return FDTD_ERR_ARG;
   }
   *out = nullptr;
-  fdtd_ctx *ctx = new (std::nothrow) fdtd_ctx ();
-  if (!ctx)
+  // a grid that fits the device, with the staging grid and an eps map, only
+  // without padded rows goes without them
+  for (bool pad : {true, false})
   {
-    g_last_error = "host allocation failed";
-    return FDTD_ERR_NOMEM;
-  }
-  int r = create_impl (cfg, device, ctx);
-  if (r != FDTD_OK)
-  {
+    fdtd_ctx *ctx = new (std::nothrow) fdtd_ctx ();
+    if (!ctx)
+    {
+      g_last_error = "host allocation failed";
+      return FDTD_ERR_NOMEM;
+    }
+    int r = create_impl (cfg, device, ctx, pad);
+    size_t left = 0, all = 0;
+    if (r == FDTD_OK && ctx->pz > ctx->g.n[2] && cudaMemGetInfo (&left, &all) == cudaSuccess &&
+        left < (size_t) ctx->g.cells * 12)
+      r = FDTD_ERR_NOMEM;
+    if (r == FDTD_OK)
+    {
+      *out = ctx;
+      return FDTD_OK;
+    }
+    const bool padded = ctx->pz > ctx->g.n[2];
     std::string keep = g_last_error;
     release (ctx);
     g_last_error = keep;
-    return r;
+    if (r != FDTD_ERR_NOMEM || !padded)
+      return r;
   }
-  *out = ctx;
-  return FDTD_OK;
+  return FDTD_ERR_NOMEM;
 }
 
 int fdtd_upload_material (fdtd_ctx *ctx, int which, const double *host)
@@ -2626,6 +2677,8 @@ int adjoint_entry (fdtd_ctx *ctx, const fdtd_adjoint_cfg *cfg, double *objective
   const void *eps = ctx->kind == 0 ? (const void *) ctx->mat64[0] : (const void *) ctx->mat32[0];
   CK (cudaStreamSynchronize (ctx->stream));
   std::string why = adjoint_run (g, eps, ctx->kind == 0, run, objective, grad, ctx->sm_count, ctx->stream);
+  if (why.find ("allocation") != std::string::npos && drop_spare_set (ctx))
+    why = adjoint_run (g, eps, ctx->kind == 0, run, objective, grad, ctx->sm_count, ctx->stream);
   if (!why.empty ())
     return fail (ctx,
                  why.find ("timed out") != std::string::npos
@@ -2946,7 +2999,10 @@ cudaError_t fdtdb::device_malloc (void **p, size_t bytes)
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
-  return cudaMalloc (p, bytes);
+  const cudaError_t e = cudaMalloc (p, bytes);
+  if (e != cudaSuccess)
+    cudaGetLastError ();   // (reported by the return value: a caller may go on without the memory)
+  return e;
 }
 
 cudaError_t fdtdb::pinned_malloc (void **p, size_t bytes)
