@@ -79,13 +79,17 @@ struct Launch
   uint32_t fk0, fk1;
   R *F[2];                     // two sets of Ez, Hx, Hy, Xz, Xx, Xy (N values each); a launch starts in set 0
   const R *load;               // state to start from (6 N values) instead of set 0, or null
-  R *ck;                       // state before step k stored at ck + (k / every) 6 N when k % every == 0, or null
+  // state before step k stored at ck + (k / every - 1) 6 N when k % every == 0, or
+  // null (not before step 0, which is 0, nor before keep0, from where the
+  // per-step data are kept)
+  R *ck;
   uint32_t every;
   R *dedm;                     // dEz/dim of step k at dedm + (k - keep0) N for k >= keep0, or null
   double *keep;                // probe Ez of step k at keep + (k - keep0) npr
   uint32_t keep0;
-  double *jpart;               // sum of Ez^2 over the probe cells of step k and probe tile q at k nprt + q, or null
-  int prt_u0, prt_v0, prt_nv, nprt;   // tiles that hold probe cells
+  double *jpart;               // sum of Ez^2 over the probe cells of probe tile q and all steps: a pair (sum, compensation)
+                               // at 2 q, or null
+  int prt_u0, prt_v0, prt_nv;  // tiles that hold probe cells
   // reverse group
   uint32_t rk0, rk1;
   R *A[2];                     // two sets of aE, aXz, aHx, aHy, aXx, aXy, acz (N values each)
@@ -319,6 +323,14 @@ __device__ __forceinline__ void adj_update (const R *T, int c, const AdjCells<R,
   }
 }
 
+// (s, c) += v, the rounding error of the sum kept in c.
+__device__ __forceinline__ void adj_add (double &s, double &c, double v)
+{
+  const double t = s + v, z = t - s;
+  c += (s - (t - z)) + (v - z);
+  s = t;
+}
+
 // Steps k0 .. k0 + steps - 1 of one tile, from `in` to `out`.
 template <typename R, int RU, int RV>
 __device__ void forward_tile (const Launch<R> &L, const R *in, R *out, int tu, int tv, uint32_t k0, int steps, R *S,
@@ -345,9 +357,9 @@ __device__ void forward_tile (const Launch<R> &L, const R *in, R *out, int tu, i
     im[r] = (c.upd >> r) & 1u ? p.im[id] : R (0);
   }
   adj_tables<R, RU, RV> (p, T, u0, v0);
-  if (L.ck && k0 % L.every == 0)
+  if (L.ck && k0 % L.every == 0 && k0 > 0 && k0 < L.keep0)
   {
-    R *const save = L.ck + (size_t) (k0 / L.every) * 6 * N;
+    R *const save = L.ck + (size_t) (k0 / L.every - 1) * 6 * N;
 #pragma unroll
     for (int r = 0; r < G::C; ++r)
       if ((c.own >> r) & 1u)
@@ -360,6 +372,11 @@ __device__ void forward_tile (const Launch<R> &L, const R *in, R *out, int tu, i
   }
   const bool probe = u0 + kRound < p.pr_hi[0] && u0 + kRound + G::OU > p.pr_lo[0] && v0 + kRound < p.pr_hi[1] &&
                      v0 + kRound + G::OV > p.pr_lo[1];
+  // the tile's sum so far, thread 0's (the same CTA takes a tile in every round,
+  // and the steps are added one by one: how they fall into rounds changes nothing)
+  auto j_at = [&] { return L.jpart + 2 * ((size_t) (tu - L.prt_u0) * L.prt_nv + (tv - L.prt_v0)); };
+  if (probe && L.jpart && threadIdx.x < 2)
+    s_sum[kThreads / 32 + threadIdx.x] = j_at ()[threadIdx.x];
   // Ez reads Hy one row lower, Hy reads Ez one row higher
   adj_publish<R, RU, RV, -1> (f[2], HRow, c.w, c.lane);
   __syncthreads ();
@@ -457,8 +474,13 @@ __device__ void forward_tile (const Launch<R> &L, const R *in, R *out, int tu, i
       double tot = 0.0;
       for (int q = 0; q < kThreads / 32; ++q)
         tot += s_sum[q];
-      L.jpart[(size_t) k * L.nprt + (tu - L.prt_u0) * L.prt_nv + (tv - L.prt_v0)] = tot;
+      adj_add (s_sum[kThreads / 32], s_sum[kThreads / 32 + 1], tot);
     }
+  }
+  if (probe && L.jpart && threadIdx.x == 0)
+  {
+    j_at ()[0] = s_sum[kThreads / 32];
+    j_at ()[1] = s_sum[kThreads / 32 + 1];
   }
 #pragma unroll
   for (int r = 0; r < G::C; ++r)
@@ -681,7 +703,7 @@ template <typename R, int RU, int RV>
 __global__ void __launch_bounds__ (kThreads, 1) adjoint_kernel (const __grid_constant__ Launch<R> L)
 {
   extern __shared__ __align__ (16) unsigned char adj_smem[];
-  __shared__ double s_sum[kThreads / 32];
+  __shared__ double s_sum[kThreads / 32 + 2];
   R *const S = reinterpret_cast<R *> (adj_smem);
   if ((int) blockIdx.x < L.fwd_ctas)
     forward_part<R, RU, RV> (L, blockIdx.x, L.fwd_ctas, S, s_sum);
@@ -689,18 +711,16 @@ __global__ void __launch_bounds__ (kThreads, 1) adjoint_kernel (const __grid_con
     reverse_part<R, RU, RV> (L, blockIdx.x - L.fwd_ctas, gridDim.x - L.fwd_ctas, S);
 }
 
-// Compensated sum of n doubles (one block of 256).
+// Compensated sum of n (sum, compensation) pairs (one block of 256).
 __global__ void adj_sum_kernel (const double *v, size_t n, double *acc)
 {
   __shared__ double ss[256], sc[256];
-  auto add = [] (double &s, double &c, double y) {
-    const double t = s + y, z = t - s;
-    c += (s - (t - z)) + (y - z);
-    s = t;
-  };
   double s = 0.0, c = 0.0;
   for (size_t i = threadIdx.x; i < n; i += 256)
-    add (s, c, v[i]);
+  {
+    adj_add (s, c, v[2 * i]);
+    c += v[2 * i + 1];
+  }
   ss[threadIdx.x] = s;
   sc[threadIdx.x] = c;
   __syncthreads ();
@@ -708,7 +728,7 @@ __global__ void adj_sum_kernel (const double *v, size_t n, double *acc)
   {
     if ((int) threadIdx.x < o)
     {
-      add (ss[threadIdx.x], sc[threadIdx.x], ss[threadIdx.x + o]);
+      adj_add (ss[threadIdx.x], sc[threadIdx.x], ss[threadIdx.x + o]);
       sc[threadIdx.x] += sc[threadIdx.x + o];
     }
     __syncthreads ();
@@ -770,7 +790,8 @@ __global__ void invm_kernel (const E *eps, int nx, int ny, int nmat, int m1x, in
       md = 0.25 * ((double) at (0, 0) + (double) at (m1x, m1y) + (double) at (m2x, m2y) + (double) at (m3x, m3y));
     }
     im[t] = R (1) / m;
-    imd[t] = 1.0 / md;
+    if (imd)
+      imd[t] = 1.0 / md;
   }
 }
 
@@ -987,21 +1008,23 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
     i_tab.push_back (ar.reserve<R> (v.size ()));
   const int i_src = ar.reserve<R> (src.size ());
   const int i_state = ar.reserve<R> (12 * N);
-  // probe tiles, and a sum per step and probe tile
+  // probe tiles, and a sum per probe tile
   const int pt_u0 = run.probe_lo[0] / ou, pt_u1 = (run.probe_hi[0] - 1) / ou;
   const int pt_v0 = run.probe_lo[1] / ov, pt_v1 = (run.probe_hi[1] - 1) / ov;
-  const int nprt = (pt_u1 - pt_u0 + 1) * (pt_v1 - pt_v0 + 1);
-  const int i_jpart = ar.reserve<double> ((size_t) run.steps * nprt);
+  const size_t nprt = (size_t) (pt_u1 - pt_u0 + 1) * (pt_v1 - pt_v0 + 1);
+  const int i_jpart = ar.reserve<double> (2 * nprt);
   const int i_im = ar.reserve<R> (N);
-  const int i_imd = ar.reserve<double> (N);
+  const int i_imd = ar.reserve<double> (grad ? N : 0);
   const int i_acc = ar.reserve<double> (2);
   const int i_bar = ar.reserve<unsigned> (2 * kBarStride);
   const int i_err = ar.reserve<int> (1);
   int i_ck = -1, i_dedm[2] = {-1, -1}, i_probe[2] = {-1, -1}, i_adj = -1, i_gim = -1, i_gout = -1;
   if (grad)
   {
-    i_ck = ar.reserve<R> ((size_t) nck * 6 * N);
-    for (int b = 0; b < 2; ++b)
+    // (the double buffers take 11 N values more than single ones would; the
+    // checkpoints of the first and the last segment are not stored for that)
+    i_ck = ar.reserve<R> ((size_t) (nck > 2 ? nck - 2 : 0) * 6 * N);
+    for (int b = 0; b < (nck > 1 ? 2 : 1); ++b)
     {
       i_dedm[b] = ar.reserve<R> ((size_t) K * N);
       i_probe[b] = ar.reserve<double> ((size_t) K * npr);
@@ -1031,12 +1054,13 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   int *err = ar.at<int> (i_err);
   if (cudaMemsetAsync (state, 0, 12 * N * sizeof (R), s) != cudaSuccess ||
       cudaMemsetAsync (acc, 0, 2 * sizeof (double), s) != cudaSuccess ||
+      cudaMemsetAsync (ar.at<double> (i_jpart), 0, 2 * nprt * sizeof (double), s) != cudaSuccess ||
       cudaMemsetAsync (bar, 0, 2 * kBarStride * sizeof (unsigned), s) != cudaSuccess ||
       cudaMemsetAsync (err, 0, sizeof (int), s) != cudaSuccess)
     return "device initialisation failed";
   const CompLayout &LE = g.comp[EZ];
   const int blocks = (int) std::min<size_t> ((N + 255) / 256, (size_t) sm_count * 8);
-  double *imd = ar.at<double> (i_imd);
+  double *imd = grad ? ar.at<double> (i_imd) : nullptr;
   if (eps_is_double)
     invm_kernel<R, double><<<blocks, 256, 0, s>>> ((const double *) eps_dev, nx, ny, LE.nmat, LE.m[1][0], LE.m[1][1],
                                                    LE.m[2][0], LE.m[2][1], LE.m[3][0], LE.m[3][1], imw, imd);
@@ -1058,7 +1082,6 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   L.prt_u0 = pt_u0;
   L.prt_v0 = pt_v0;
   L.prt_nv = pt_v1 - pt_v0 + 1;
-  L.nprt = nprt;
 
   // forward run: checkpoints, and the per-step data of the last segment
   const uint32_t last0 = (nck - 1) * K;
@@ -1069,14 +1092,14 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
   L.every = K;
   if (grad)
   {
-    L.ck = ar.at<R> (i_ck);
+    L.ck = nck > 2 ? ar.at<R> (i_ck) : nullptr;
     L.dedm = ar.at<R> (i_dedm[0]);
     L.keep = ar.at<double> (i_probe[0]);
     L.keep0 = last0;
   }
   if (launch (L, kern, smem, ctas, s) != cudaSuccess)
     return std::string ("adjoint forward launch failed: ") + cudaGetErrorString (cudaGetLastError ());
-  adj_sum_kernel<<<1, 256, 0, s>>> (L.jpart, (size_t) run.steps * nprt, acc);
+  adj_sum_kernel<<<1, 256, 0, s>>> (L.jpart, nprt, acc);
   double hacc[2];
   int herr = 0;
   if (cudaMemcpyAsync (hacc, acc, sizeof (hacc), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -1117,7 +1140,10 @@ std::string run_t (const Geometry &g, const void *eps_dev, bool eps_is_double, c
       L.fwd_ctas = fwd_split;
       L.fk0 = (j - 1) * K;
       L.fk1 = j * K;
-      L.load = ck + (size_t) (j - 1) * 6 * N;
+      L.load = j > 1 ? ck + (size_t) (j - 2) * 6 * N : nullptr;
+      // (the first segment starts from 0, in set 0)
+      if (j == 1 && cudaMemsetAsync (state, 0, 6 * N * sizeof (R), s) != cudaSuccess)
+        return "device initialisation failed";
       L.dedm = ar.at<R> (i_dedm[1 - b]);
       L.keep = ar.at<double> (i_probe[1 - b]);
       L.keep0 = L.fk0;

@@ -47,3 +47,41 @@ def test_gradient_matches_central_differences(fdtd, size):
         em[x, y] -= h
         fd = (objective(ep) - objective(em)) / (2 * h)
         assert abs(fd - g[x, y]) <= 2e-6 * np.max(np.abs(g)), ((x, y), fd, g[x, y])
+
+
+@pytest.mark.parametrize("every", [200, 100, 67, 30, 7, 1])
+@pytest.mark.parametrize("whole", [False, True])
+def test_memory_of_a_run(fdtd, every, whole):
+    """Device memory of a backward run, against the run with single buffers: state 6 N, adjoint 9 N, checkpoints 6 N
+    each, two segments' per-step data (K N values, and the K probe fields in FP64), im in both precisions, the
+    gradient twice.  With a probe of a few cells, and one that covers the grid."""
+    import torch
+
+    size, steps = (1200, 1100), 200
+    cells = size[0] * size[1]
+    probe = ((1, 1), (size[0] - 1, size[1] - 1)) if whole else ((700, 600), (704, 603))
+    npr = (probe[1][0] - probe[0][0]) * (probe[1][1] - probe[0][1])
+    kw = dict(mode=2, size=size, use_pml=True, pml=8, teta=90, phi=0, psi=90, point_source=(500, 500, 0),
+              point_source_mask=4, precision=1)
+    segments = -(-steps // every)
+    single = cells * (4 * (6 + 9 + 6 * segments + 2 * every + 1) + 8 * 3) + 16 * every * npr
+    with fdtd.Simulation(**kw) as sim:
+        sim.step(1)
+        sim.sync()
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info(0)[0]
+        sim.backward(steps, every, *probe, 1)
+        used = before - torch.cuda.mem_get_info(0)[0]
+    assert used <= single + (8 << 20), (used / single)
+
+
+@pytest.mark.parametrize("every", [44, 22, 21, 15, 7, 1])
+def test_segments_agree_whatever_their_number(fdtd, every):
+    """One segment, two (neither is stored as a checkpoint), three and more: the same gradient, bit for bit, from the
+    same forward run, with a probe over several tiles."""
+    kw, eps, _, _ = _grid((90, 111))
+    with fdtd.Simulation(materials={"eps": eps}, precision=1, **kw) as sim:
+        j, g = sim.backward(44, 1000, (20, 30), (70, 90), 0)
+        j1, g1 = sim.backward(44, every, (20, 30), (70, 90), 0)
+        assert sim.objective(44, (20, 30), (70, 90), 0) == j
+    assert j > 0 and j1 == j and np.array_equal(g1, g)
