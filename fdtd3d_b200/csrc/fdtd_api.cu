@@ -1345,7 +1345,9 @@ int plan_sweep (fdtd_ctx *ctx)
     bool tb2 = exact_pairs || (int64_t) g.cells >= line;
     if (const char *v = std::getenv ("FDTDB_TB2"))
       tb2 = std::atoi (v) != 0;
-    if (!tb2)
+    if (g.cfg.use_metamaterials)
+      ctx->tb2_why = "metamaterials";   // (before the shell's buffer set is allocated)
+    else if (!tb2)
       ctx->tb2_why = "single steps are faster on a grid this small, or FDTDB_TB2=0";
     else
     {
