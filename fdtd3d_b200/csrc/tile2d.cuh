@@ -397,7 +397,8 @@ __device__ __forceinline__ void tile2d_steps (const Tile2D &p, int u0, int v0, u
   // other family looks down (u - 1), the first where it looks up
   auto publish = [&] (auto j_c) __attribute__ ((always_inline)) {
     constexpr int j = decltype (j_c)::value;
-    constexpr int r = M::low (M::is_h (j) ? (M::TE ? 0 : 0) : (M::TE ? 2 : 1)) == -1 ? RU - 1 : 0;
+    // (a component of the other family: E is the first one, H the last)
+    constexpr int r = M::low (M::is_h (j) ? 0 : 2) == -1 ? RU - 1 : 0;
     sts_row<RV> (Row + (j * kTileWarps + w) * TV + col0, f[j][r]);
   };
   publish (std::integral_constant<int, 0>{});
