@@ -65,7 +65,11 @@ typedef struct fdtd_ctx fdtd_ctx;
 /* arithmetic forms */
 #define FDTD_PREC_FP64_PLAIN 0   /* reference formulation, FP64, bit-faithful */
 #define FDTD_PREC_FP32 1         /* fused step, FP32 storage and compute */
-#define FDTD_PREC_FP16S 2        /* fused step, FP16 field storage, FP32 compute */
+/* FP16 field storage, FP32 compute.  Fields are rounded to FP16 once per pass
+ * over them: after a step, after a pair of steps (3-D) or after a launch of up
+ * to seven (2-D), so runs that split the same steps into other calls differ by
+ * that rounding (seven calls of one step and one call of seven, for instance). */
+#define FDTD_PREC_FP16S 2
 
 /* field components (fdtd3d GridType order) */
 #define FDTD_EX 0
@@ -270,7 +274,9 @@ int fdtd_keep_previous_level (fdtd_ctx *ctx, int on);
  * (two steps per pass: the last call ended on a pair), "sweep3d_tma"
  * (TMA-pipelined one-sweep 3-D kernel), "fused3d_regblock" (register-blocked
  * one-sweep 3-D kernel), "per_cell" (the per-cell kernels, one launch per
- * half-step, or in the 2-D modes up to seven steps), or "not_stepped" before the first update.  Null for a null context. */
+ * half-step, or in the 2-D modes up to seven steps), or "not_stepped" before
+ * the first update.  "plain_fp64" and "per_cell" do not tell the launch forms
+ * of a route apart; fdtd_launch_count does.  Null for a null context. */
 const char *fdtd_step_kernel (const fdtd_ctx *ctx);
 
 /* The cudaStream_t (as void *) every launch of this context goes to, so a
@@ -325,8 +331,8 @@ int fdtd_backward (fdtd_ctx *ctx, const fdtd_adjoint_cfg *cfg, double *objective
 /*
  * Batched 2-D TMz (no counterpart in the reference, whose runs are one grid
  * per process): many Dim2_TMz simulations of different sizes advanced
- * together by one persistent kernel launch per fdtd_batch_step call,
- * captured in a CUDA graph.  `base` gives the shared physics (dx,
+ * together by one persistent kernel launch per fdtd_batch_step call (a launch
+ * per step in calls of up to three), captured in a CUDA graph.  `base` gives the shared physics (dx,
  * wavelength, Courant factor, PML width, point-source kind/bandwidth and the
  * Ez bit of point_source_mask); precision must be FDTD_PREC_FP32 and TF/SF
  * and metamaterials are not provided.  `sizes` holds count (nx, ny) pairs;
