@@ -1731,8 +1731,7 @@ bool tile2d_ready (const fdtd_ctx *ctx)
 //   31, 4096 521 / 645; without TF/SF 512 21 / 15, 8192 1820 / 1300;
 //  FP16 storage as FP32, but with an eps map 4096 536 / 532, 8192 1833 / 2095
 //   (without 1662 / 1440).
-// (Two steps in FP64 are two launches of one; three steps and more are faster
-// in tiles at every size.)
+// (Launches of three steps and more are faster in tiles at every size.)
 bool step2d_by_cells (const fdtd_ctx *ctx)
 {
   const Geometry &g = ctx->g;
@@ -1938,9 +1937,12 @@ int step_impl (fdtd_ctx *ctx, uint32_t t_start, uint32_t n)
     uint32_t t = t_start + i;
     if (tiles && t > 0)
     {
-      // an odd number of steps in FP64 (tile2d.cuh says why)
-      int steps = (int) std::min<uint32_t> (kTileSteps, n - i);
-      if (ctx->kind == 0 && steps % 2 == 0)
+      // FP64 keeps the level before the current one (a step at t = 0 goes back
+      // to it), so a call's last step is a launch of its own; and an odd number
+      // of steps each (tile2d.cuh says why)
+      const bool levels = ctx->kind == 0;
+      int steps = (int) std::min<uint32_t> (kTileSteps, n - i - (levels && n - i > 1 ? 1 : 0));
+      if (levels && steps % 2 == 0)
         --steps;
       if (steps > 1 || !step2d_by_cells (ctx))
       {

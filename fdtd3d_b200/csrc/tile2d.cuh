@@ -19,7 +19,9 @@
 // FP64 keeps two levels of every field whose face cells are never updated: a
 // step leaves the other level's face cells current, so a tile alternates the
 // two values, and an odd number of steps per launch ends on the level that
-// is written.
+// is written.  The level before the current one is the state a launch began
+// with; the last launch of a call takes one step, so that after a call it is
+// the step before, as the per-cell kernels leave it.
 #pragma once
 
 #include <cuda_fp16.h>

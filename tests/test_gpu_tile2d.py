@@ -130,3 +130,27 @@ def test_single_steps_by_cells_or_by_tiles(fdtd, prec, size, kw, cells):
                 assert np.array_equal(g[c].view(np.int64), got[0][c].view(np.int64)), c
             else:   # (12 steps of FP32; FP16 storage rounds once per launch of tiles)
                 assert np.linalg.norm(g[c] - got[0][c]) <= (1e-6 if prec == 1 else 5e-3) * np.linalg.norm(got[0][c]), c
+
+
+# a step at t = 0 updates nothing but moves on a level: in FP64 the fields are
+# then those of the step before the call's last, whatever its launches were
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 7, 8, 9, 14, 15, 22])
+@pytest.mark.parametrize("size", [(60, 45), (330, 340)])
+@pytest.mark.parametrize("source", ["tfsf", "point"])
+def test_fp64_step_at_zero_after_a_call(fdtd, n, size, source):
+    kw, mats, fields = _setup(fdtd, 2, size, source, 11)
+    out = []
+    for calls in ([n], [1] * n):
+        with fdtd.Simulation(materials=mats, precision=0, **kw) as sim:
+            for c, v in fields.items():
+                sim.set_field(c, v)
+            sim.t = 20
+            for k in calls:
+                sim.step(k)
+            sim.step(1, t_start=0)
+            got = {c: sim.field(c) for c in fields}
+            sim.step(5, t_start=40)
+            got.update({c + "5": sim.field(c) for c in fields})
+            out.append(got)
+    for c in out[0]:
+        assert np.array_equal(out[0][c].view(np.int64), out[1][c].view(np.int64)), c
