@@ -76,6 +76,7 @@ __device__ __forceinline__ void sts_row (C *p, const C v[N])
 
 // The incident grid on [c0, c0 + n) in shared memory: E, then H step.  Cells
 // whose neighbour lies outside the window turn invalid from its ends inwards.
+// (Rounded operations: the same bits in every form.)
 __device__ __forceinline__ void inc_e_step (double *e, const double *h, int c0, int n, const Tile2D &p, double src)
 {
   const int q = threadIdx.x + 32 * threadIdx.y, i = c0 + q;
@@ -84,14 +85,14 @@ __device__ __forceinline__ void inc_e_step (double *e, const double *h, int c0, 
     if (i == 0)
       e[q] = src;
     else if (q > 0)
-      e[q] = e[q] + (h[q - 1] - h[q]) * p.mod_e;
+      e[q] = __dadd_rn (e[q], __dmul_rn (__dsub_rn (h[q - 1], h[q]), p.mod_e));
   }
 }
 __device__ __forceinline__ void inc_h_step (double *h, const double *e, int c0, int n, const Tile2D &p)
 {
   const int q = threadIdx.x + 32 * threadIdx.y, i = c0 + q;
   if (q + 1 < n && i < p.inc_len - 1)
-    h[q] = h[q] + (e[q] - e[q + 1]) * p.mod_h;
+    h[q] = __dadd_rn (h[q], __dmul_rn (__dsub_rn (e[q], e[q + 1]), p.mod_h));
 }
 
 // One border term of a cell, resolved once per launch: the two incident cells

@@ -154,3 +154,19 @@ def test_fp64_step_at_zero_after_a_call(fdtd, n, size, source):
             out.append(got)
     for c in out[0]:
         assert np.array_equal(out[0][c].view(np.int64), out[1][c].view(np.int64)), c
+
+
+@pytest.mark.parametrize("calls", [[1] * 30, [30], [8, 22]])
+@pytest.mark.parametrize("mode", [2, 5])
+def test_incident_grid_has_the_same_bits_in_every_form(fdtd, calls, mode):
+    kw = dict(mode=mode, size=(64, 59), use_pml=True, pml=5, use_tfsf=True, tfsf_left=9, tfsf_right=9, teta=40, phi=25,
+              psi=20)
+    got = []
+    for prec in (0, 1, 2):
+        with fdtd.Simulation(precision=prec, **kw) as sim:
+            for n in calls:
+                sim.step(n)
+            got.append((sim.incident("E"), sim.incident("H")))
+    assert np.any(got[0][0] != 0)
+    for g in got[1:]:
+        assert np.array_equal(g[0], got[0][0]) and np.array_equal(g[1], got[0][1])
