@@ -1011,8 +1011,8 @@ int launch_current_fix (const FusedParams &p, const CurrentFix &cf, const double
 
 namespace {
 
-// The cells a point source's value reaches, one thread per cell of an 8^3 box
-// with the source at (4, 4, 4): worked out again from the old set with the
+// The cells a point source's value reaches, one thread per cell of a box with
+// the source in its upper middle (4^3 for a step, 8^3 for a pair): worked out again from the old set with the
 // source in place, in the sweep's arithmetic and in FP32 between the half-steps
 // (adding the change the source makes to the sweep's result instead rounds H
 // twice, and FP16 storage has rounded E before the change is formed).  The
@@ -1022,12 +1022,14 @@ namespace {
 // are not stored.
 // Inside the sweep a source cost its items the general class, 116 of 165 us of
 // a 256 x 224 x 240 step with one CTA at work, and kept the run from pairs;
-// this kernel is one CTA's latency, about 4 us a step or pair.
+// this kernel is one CTA's latency, about 4 us a step, 5 us a pair.
+constexpr int point_box (bool pair) { return pair ? 8 : 4; }
+
 template <typename T, bool PAIR>
-__global__ void __launch_bounds__ (512) point_fix_kernel (const __grid_constant__ FusedParams p, PointFix pf,
-                                                          const double *src, int stride)
+__global__ void __launch_bounds__ (point_box (PAIR) * point_box (PAIR) * point_box (PAIR))
+    point_fix_kernel (const __grid_constant__ FusedParams p, PointFix pf, const double *src, int stride)
 {
-  constexpr int W = 8, SRC = 4;
+  constexpr int W = point_box (PAIR), SRC = W / 2;
   __shared__ float sE[3][W * W * W], sH[3][W * W * W];
   const int q = threadIdx.x;
   const int l[3] = {q / (W * W), q / W % W, q % W};
@@ -1111,12 +1113,12 @@ int launch_point_fix (const FusedParams &p, const PointFix &pf, const double *sr
     if (pair)
       point_fix_kernel<__half, true><<<1, 512, 0, s>>> (p, pf, src, stride);
     else
-      point_fix_kernel<__half, false><<<1, 512, 0, s>>> (p, pf, src, stride);
+      point_fix_kernel<__half, false><<<1, 64, 0, s>>> (p, pf, src, stride);
   }
   else if (pair)
     point_fix_kernel<float, true><<<1, 512, 0, s>>> (p, pf, src, stride);
   else
-    point_fix_kernel<float, false><<<1, 512, 0, s>>> (p, pf, src, stride);
+    point_fix_kernel<float, false><<<1, 64, 0, s>>> (p, pf, src, stride);
   return 1;
 }
 
