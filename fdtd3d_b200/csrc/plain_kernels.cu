@@ -314,8 +314,9 @@ constexpr int kMarchMax = 64;   // largest x chunk (per-plane TF/SF masks in sha
 //  * the x neighbours are the previous plane's values.
 // Columns are numbered flat over y and z, so no lane idles on odd sizes; the
 // next plane's material and coefficients are worked out after the stores,
-// where few values are live (96 registers, 20 warps per SM).  What is left is
-// memory latency (3.9 TB/s of DRAM, 30 % issue active).
+// where few values are live (96 registers, 16 to 20 warps per SM).  What is left
+// is memory latency (256^3: 11 to 13 of 16 warps wait for loads, 25 % issue
+// active, 4.1 to 4.4 TB/s of DRAM; 512^3: 5.0 TB/s).
 // 203 x 181 x 165, PML 12, TF/SF: 370 -> 210 us per half-step (a step 735 ->
 // 429 us); a step at 80^3, PML 10: 82 -> 55 us.
 // IS_H: the family, which orders the two differences of a curl.  LO: the lower
