@@ -1082,6 +1082,11 @@ __device__ __forceinline__ bool band_cell (const BandBox &b, int first, int &x, 
 // only its own cell; the E corrections of the +x / +y / +z neighbours are
 // recomputed from the box's neighbour masks, never read, so there are no
 // races.
+// FP16 storage: what the sweep stored is rounded already, so adding to it would
+// round twice, and H would miss the correction of an E that was rounded.  The
+// band's values are worked out again from the old set instead, in FP32 and in
+// the order of a sweep with the corrections inside it (same bits; a plane wave's
+// first 20 steps 4.54e-4 -> 4.13e-4 off FP64).
 template <typename T>
 __global__ void __launch_bounds__ (256) tfsf_post_kernel (const __grid_constant__ FusedParams p, const BandBox *boxes,
                                                           const int2 *blk, int *err)
@@ -1116,6 +1121,49 @@ __global__ void __launch_bounds__ (256) tfsf_post_kernel (const __grid_constant_
   };
   auto em = [] (unsigned mask, int k) { return (mask >> (4 * k)) & 15u; };
   const size_t id = (size_t) x * sx + (size_t) y * pz + z;
+  const bool at_src = x == p.ps[0] && y == p.ps[1] && z == p.ps[2];
+  if constexpr (std::is_same<T, __half>::value)
+  {
+    const size_t st[3] = {sx, (size_t) pz, 1};
+    auto at = [] (const void *f, size_t i) { return __half2float (static_cast<const __half *> (f)[i]); };
+    // E component k after the step, one cell up along `up` (-1: here)
+    auto e_new = [&] (int k, unsigned m, int up) -> float {
+      const int cx = x + (up == 0), cy = y + (up == 1), cz = z + (up == 2);
+      const size_t c = up < 0 ? id : id + st[up];
+      const float o = at (p.e_old[k], c);
+      if (cx > nx - 2 || cy > ny - 2 || cz > nz - 2)
+        return o;
+      if (((p.ps_mask >> k) & 1) && cx == p.ps[0] && cy == p.ps[1] && cz == p.ps[2])
+        return (float) p.src[p.src_index];
+      const int b1 = (k + 1) % 3, b2 = (k + 2) % 3;
+      float cu = (at (p.h_old[b2], c) - at (p.h_old[b2], c - st[b1])) - (at (p.h_old[b1], c) - at (p.h_old[b1], c - st[b2]));
+      if (m)
+        cu += tfsf_terms (p, k, m, p.inc_h, err, cx, cy, cz);
+      const float im = p.eps ? __fdividef (2.f, p.eps[c] + p.eps[c + st[k]]) : 1.f;
+      return o + (S * im) * cu;
+    };
+    float e[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+      e[k] = e_new (k, em (b.mask, k), -1);
+      if (em (b.mask, k))
+        static_cast<__half *> (p.e_new[k])[id] = __float2half_rn (e[k]);
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+    {
+      const int b1 = (m + 1) % 3, b2 = (m + 2) % 3;
+      const unsigned m1 = em (b.nmask[b2], b1), m2 = em (b.nmask[b1], b2), mh = em (b.mask, 3 + m);
+      if (!(m1 | m2 | mh | em (b.mask, b1) | em (b.mask, b2)) || (at_src && ((p.ps_mask >> (3 + m)) & 1)))
+        continue;
+      float cu = (e_new (b1, m1, b2) - e[b1]) - (e_new (b2, m2, b1) - e[b2]);
+      if (mh)
+        cu += tfsf_terms (p, 3 + m, mh, p.inc_e, err, x, y, z);
+      static_cast<__half *> (p.h_new[m])[id] = __float2half_rn (at (p.h_old[m], id) + S * cu);
+    }
+    return;
+  }
   const float d0 = de (0, em (b.mask, 0), x, y, z), d1 = de (1, em (b.mask, 1), x, y, z),
               d2 = de (2, em (b.mask, 2), x, y, z);
   const float dd[3] = {d0, d1, d2};
@@ -1134,7 +1182,6 @@ __global__ void __launch_bounds__ (256) tfsf_post_kernel (const __grid_constant_
           (hm[1] ? tfsf_terms (p, 4, hm[1], p.inc_e, err, x, y, z) : 0.f),
       (de (0, em (b.nmask[1], 0), x, y + 1, z) - d0) - (de (1, em (b.nmask[0], 1), x + 1, y, z) - d1) +
           (hm[2] ? tfsf_terms (p, 5, hm[2], p.inc_e, err, x, y, z) : 0.f)};
-  const bool at_src = x == p.ps[0] && y == p.ps[1] && z == p.ps[2];
 #pragma unroll
   for (int m = 0; m < 3; ++m)
     if (a[m] != 0.f && !(at_src && ((p.ps_mask >> (3 + m)) & 1)))
