@@ -79,3 +79,22 @@ def test_per_cell_kernels_on_either_row(fdtd, shape, prec, tol):
             assert not p or sim.step_kernel == "per_cell", sim.step_kernel
     for fam in "EH":
         assert _family(out[prec], out[0], fam) <= tol, (nz, fam, _family(out[prec], out[0], fam))
+
+
+# fields to the device and back: rows of nz cells below and above the line of
+# the four-cell form (8 M cells; the last one not a multiple of four), padded rows
+@pytest.mark.parametrize("shape", [(20, 21, 40), (200, 200, 200), (201, 199, 200), (250, 181, 177), (21, 20, 33), (251, 252, 129)])
+@pytest.mark.parametrize("prec", [1, 2])
+def test_fields_come_back_as_they_went(fdtd, shape, prec):
+    import torch
+
+    rng = np.random.default_rng(1)
+    v = rng.integers(-1000, 1001, shape) / 8.0   # (values that 11 bits hold)
+    with fdtd.Simulation(mode=3, size=shape, precision=prec) as sim:
+        sim.set_field("Ey", v)
+        assert np.array_equal(sim.field("Ey"), v)
+        out = torch.empty(v.size + 1, dtype=torch.float64, device="cuda")
+        sim.field_device("Ey", out.data_ptr() + 8)   # off the 16-byte boundary
+        sim.sync()
+        assert np.array_equal(out[1:].cpu().numpy().reshape(shape), v)
+        assert not np.any(sim.field("Ex"))
